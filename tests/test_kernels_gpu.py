@@ -93,6 +93,25 @@ def test_gemm_rows_do_not_depend_on_the_batch():
         assert torch.equal(one[0], whole[r])
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 1, 4), (3, 7, 20), (4, 256, 128), (5, 9, 132), (8, 33, 64), (9, 17, 68),
+                                   (16, 65, 260), (17, 31, 36), (33, 65, 68), (65, 130, 100), (129, 1157, 20),
+                                   (200, 333, 1000), (385, 2600, 132), (1300, 3000, 36)])
+def test_float32_products_of_every_size_keep_the_order_of_the_sum(m, n, k):
+    """The kernels for aligned float32 operands (few rows, three tiles) give the bits of the general one,
+    which rows off 16 bytes go to: the same additions in the same order."""
+    from minfer_b200.kernels import api as K
+    g = torch.Generator().manual_seed(m * 1000 + n)
+    a, w = torch.randn(m, k, generator=g).cuda(), torch.randn(n, k, generator=g).cuda()
+    bias, old = torch.randn(n, generator=g).cuda(), torch.randn(m, n + 3, generator=g).cuda()
+    a_off = torch.zeros(m, k + 1, device="cuda")[:, 1:]
+    a_off.copy_(a)
+    for b, accumulate in ((None, False), (bias, False), (bias, True)):
+        got, want = old.clone(), old.clone()
+        K.gemm_simt(a, w, b, got[:, 1:n + 1], accumulate=accumulate)
+        K.gemm_simt(a_off, w, b, want[:, 1:n + 1], accumulate=accumulate)
+        assert torch.equal(got, want)
+
+
 def rope_reference(x, pos, inv_freq, rotary_dim, style):
     """x [T, H, hd] float64."""
     out = x.clone()
