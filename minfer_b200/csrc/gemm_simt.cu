@@ -102,14 +102,23 @@ __device__ __forceinline__ void fma_f32x2(unsigned long long& acc, unsigned long
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
+// An operand's 16 bytes, never moved above the wait for the kernel before: a load through a const
+// __restrict__ pointer counts as invariant, and the compiler did move the first tile's there.
+__device__ __forceinline__ float4 load16(const float* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
 template <int ROWS, int THREADS, int BKT>
-__device__ __forceinline__ void f32_tile_fetch(const float* __restrict__ src, long long ld, int row0, int rows,
+__device__ __forceinline__ void f32_tile_fetch(const float* src, long long ld, int row0, int rows,
                                                int k0, int K, float4* held) {
 #pragma unroll
     for (int e = 0; e < ROWS * (BKT / 4) / THREADS; ++e) {
         const int idx = (int)threadIdx.x + e * THREADS;
         const int r = row0 + idx / (BKT / 4), k = k0 + (idx % (BKT / 4)) * 4;
-        held[e] = (r < rows && k < K) ? *reinterpret_cast<const float4*>(src + (size_t)r * ld + k)
+        held[e] = (r < rows && k < K) ? load16(src + (size_t)r * ld + k)
                                       : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
@@ -136,8 +145,8 @@ struct F32Tile {
 template <int BM_, int BN_, int TM, int TN, int BKT>
 __global__ void __launch_bounds__(F32Tile<BM_, BN_, TM, TN>::THREADS,
                                   512 / F32Tile<BM_, BN_, TM, TN>::THREADS)
-gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                     float* __restrict__ C, int M, int N, int K, long long lda, long long ldw,
+gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ bias, float* C,
+                     int M, int N, int K, long long lda, long long ldw,
                      long long ldc, int accumulate) {
     constexpr int THREADS = F32Tile<BM_, BN_, TM, TN>::THREADS;
     constexpr int WARPS_N = F32Tile<BM_, BN_, TM, TN>::WARPS_N;

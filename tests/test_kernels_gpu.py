@@ -112,6 +112,27 @@ def test_float32_products_of_every_size_keep_the_order_of_the_sum(m, n, k):
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("m", [3, 12, 40, 385, 1500])
+def test_float32_product_waits_for_the_kernel_that_writes_its_input(m):
+    """Launched while a norm still writes the rows it reads (programmatic dependent launch), the product
+    gives the bits it gives when launched after the norm has ended."""
+    from minfer_b200.kernels import api as K
+    g = torch.Generator().manual_seed(m)
+    h, w = torch.randn(m, 896, generator=g).cuda(), torch.randn(1152, 896, generator=g).cuda()
+    scale = torch.rand(896, generator=g).cuda()
+    x, out = torch.empty(m, 896, device="cuda"), torch.empty(m, 1152, device="cuda")
+    K.rmsnorm(h, scale, 1e-5, x)
+    torch.cuda.synchronize()
+    K.gemm_simt(x, w, None, out)
+    torch.cuda.synchronize()
+    want = out.clone()
+    for _ in range(20):
+        x.fill_(float("nan"))
+        K.rmsnorm(h, scale, 1e-5, x)
+        K.gemm_simt(x, w, None, out)
+        assert torch.equal(out, want)
+
+
 def rope_reference(x, pos, inv_freq, rotary_dim, style):
     """x [T, H, hd] float64."""
     out = x.clone()
