@@ -685,7 +685,7 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k,
             }
             for (int i = 0; i < cnt; ++i) {
                 const int pg = __shfl_sync(0xffffffffu, page, i);
-                if (lane == 0 && ok) {
+                if (elect_one() && ok) {
                     const int n = base + i, s = n % STAGES;
                     const uint32_t ph = (uint32_t)(n / STAGES) & 1u;
                     // a page that ends below the row's position holds no key of this step
@@ -709,8 +709,10 @@ attention_decode_ring_kernel(const __grid_constant__ CUtensorMap map_k,
                 }
             }
         }
-        if (lane == 0 && !waited) pdl_wait();
-        if (lane == 0 && !ok && a.status) atomicOr(a.status, MF_STATUS_WAIT_TIMEOUT);
+        if (elect_one()) {
+            if (!waited) pdl_wait();
+            if (!ok && a.status) atomicOr(a.status, MF_STATUS_WAIT_TIMEOUT);
+        }
         return;
     }
     pdl_wait();

@@ -326,7 +326,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // row of scores each, take it.
     if (warp < 4) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-      if (warp == 0 && lane == 0) {
+      if (warp == 0 && elect_one()) {
         // ---- TMA producer ---------------------------------------------------------------
         fa_expect_tx(fa_smem(q_full), has1 ? 2 * T_BYTES : T_BYTES);
         for (int t = 0; t < (has1 ? 2 : 1); ++t)
@@ -375,7 +375,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 fa_tma(fa_smem(v_s + st * T_BYTES + c * BLOCK), &map_v, hk * HD + 64 * c, key0,
                        fa_smem(&v_full[st]));
         }
-      } else if (warp == 1 && lane == 0) {
+      } else if (warp == 1 && elect_one()) {
         // ---- MMA issuer -------------------------------------------------------------------
         // S: M = 128 queries, N = 128 keys, both operands K-major
         constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(FA_KEYS >> 3) << 17) |

@@ -416,7 +416,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---- TMA producer ------------------------------------------------------------
         // The weights are constant over the step: their first tiles are requested before the
         // kernel waits for the one before it, so that they stream in while that one finishes.
@@ -451,7 +451,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
     // the tokens' 1 / rms, by the two warps that have nothing to do while the weights stream
     if (a.row_ssq != nullptr && warp >= 2) row_scales(a, m0, NT, scale_s, tid - 64, 64);
-    if (warp == 1 && lane == 0) {
+    if (warp == 1 && elect_one()) {
         // ---- MMA issuer --------------------------------------------------------------
         constexpr uint32_t idesc = umma_idesc(NT);
         bool ok = true;
@@ -594,7 +594,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---- TMA producer (weights first: they are constant over the step) --------------------
         const int pre = n_iter < STAGES ? n_iter : STAGES;
         for (int i = 0; i < pre; ++i) {
@@ -624,7 +624,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         pdl_wait();
     }
     if (a.row_ssq != nullptr && warp >= 2) row_scales(a, m0, NT, scale_s, tid - 64, 64);
-    if (warp == 1 && lane == 0) {
+    if (warp == 1 && elect_one()) {
         // ---- MMA issuer ---------------------------------------------------------------------
         constexpr uint32_t idesc = umma_idesc(NT);
         bool ok = true;
@@ -1049,7 +1049,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---- TMA producer ------------------------------------------------------------
         int it = 0;
         bool ok = true;
@@ -1074,7 +1074,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                                      m0 + NT + (int)rank * (NT / 2), leader_full);
             }
         }
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+    } else if (warp == 1 && rank == 0 && elect_one()) {
         // ---- MMA issuer (leader) -------------------------------------------------------
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) |
                                    ((uint32_t)(256 >> 4) << 24);
