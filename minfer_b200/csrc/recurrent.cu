@@ -225,18 +225,24 @@ __device__ __forceinline__ void rc_cp_async16(float* dst, const float* src) {
 #define RC_TU 4
 
 // TU consecutive tokens of a chunk, from token `tt` on: S <- da S + dt x B, y = S . C + D x for
-// each in turn (S carries over), the TU sums reduced over a column's NS threads together.
-template <int NREG, bool VEC, int TU, int NS>
-__device__ __forceinline__ void rc_walk(float (&S)[NREG], const float* xs, const float* Bs, const float* Cs,
+// each in turn (S carries over), the TU sums reduced over a column's NS threads together.  A thread
+// has CPT columns, RC_PB apart: what it reads of B and C from shared memory serves them all.
+template <int NREG, bool VEC, int TU, int NS, int CPT>
+__device__ __forceinline__ void rc_walk(float (&S)[CPT][NREG], const float* xs, const float* Bs, const float* Cs,
                                         const float* dts, const float* das, int tt, int N, int s, int pl,
-                                        bool p_ok, float dsk, float* y_col, int inner) {
-    float xv[TU], da[TU], dtx[TU], acc[TU];
+                                        int n_p, float dsk, float* y_col, int inner) {
+    constexpr int PB = RC_PB * CPT;
+    float xv[CPT][TU], da[TU], dtx[CPT][TU], acc[CPT][TU];
 #pragma unroll
     for (int u = 0; u < TU; ++u) {
-        xv[u] = p_ok ? xs[(tt + u) * RC_PB + pl] : 0.0f;
         da[u] = das[tt + u];
-        dtx[u] = dts[tt + u] * xv[u];
-        acc[u] = 0.0f;
+        const float dt = dts[tt + u];
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+            xv[c][u] = pl + RC_PB * c < n_p ? xs[(tt + u) * PB + pl + RC_PB * c] : 0.0f;
+            dtx[c][u] = dt * xv[c][u];
+            acc[c][u] = 0.0f;
+        }
     }
     if (VEC) {
 #pragma unroll
@@ -247,12 +253,15 @@ __device__ __forceinline__ void rc_walk(float (&S)[NREG], const float* xs, const
                 for (int u = 0; u < TU; ++u) {
                     const float4 bv = *reinterpret_cast<const float4*>(Bs + (tt + u) * N + n);
                     const float4 cv = *reinterpret_cast<const float4*>(Cs + (tt + u) * N + n);
-                    S[4 * j] = fmaf(da[u], S[4 * j], dtx[u] * bv.x);
-                    S[4 * j + 1] = fmaf(da[u], S[4 * j + 1], dtx[u] * bv.y);
-                    S[4 * j + 2] = fmaf(da[u], S[4 * j + 2], dtx[u] * bv.z);
-                    S[4 * j + 3] = fmaf(da[u], S[4 * j + 3], dtx[u] * bv.w);
-                    acc[u] += fmaf(S[4 * j + 3], cv.w,
-                                   fmaf(S[4 * j + 2], cv.z, fmaf(S[4 * j + 1], cv.y, S[4 * j] * cv.x)));
+#pragma unroll
+                    for (int c = 0; c < CPT; ++c) {
+                        S[c][4 * j] = fmaf(da[u], S[c][4 * j], dtx[c][u] * bv.x);
+                        S[c][4 * j + 1] = fmaf(da[u], S[c][4 * j + 1], dtx[c][u] * bv.y);
+                        S[c][4 * j + 2] = fmaf(da[u], S[c][4 * j + 2], dtx[c][u] * bv.z);
+                        S[c][4 * j + 3] = fmaf(da[u], S[c][4 * j + 3], dtx[c][u] * bv.w);
+                        acc[c][u] += fmaf(S[c][4 * j + 3], cv.w,
+                                          fmaf(S[c][4 * j + 2], cv.z, fmaf(S[c][4 * j + 1], cv.y, S[c][4 * j] * cv.x)));
+                    }
                 }
             }
         }
@@ -263,8 +272,11 @@ __device__ __forceinline__ void rc_walk(float (&S)[NREG], const float* xs, const
             if (n < N) {
 #pragma unroll
                 for (int u = 0; u < TU; ++u) {
-                    S[r] = fmaf(da[u], S[r], dtx[u] * Bs[(tt + u) * N + n]);
-                    acc[u] = fmaf(S[r], Cs[(tt + u) * N + n], acc[u]);
+#pragma unroll
+                    for (int c = 0; c < CPT; ++c) {
+                        S[c][r] = fmaf(da[u], S[c][r], dtx[c][u] * Bs[(tt + u) * N + n]);
+                        acc[c][u] = fmaf(S[c][r], Cs[(tt + u) * N + n], acc[c][u]);
+                    }
                 }
             }
         }
@@ -272,30 +284,37 @@ __device__ __forceinline__ void rc_walk(float (&S)[NREG], const float* xs, const
 #pragma unroll
     for (int o = 1; o < NS; o <<= 1) {
 #pragma unroll
-        for (int u = 0; u < TU; ++u) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
-    }
-    if (s == 0 && p_ok) {
+        for (int u = 0; u < TU; ++u)
 #pragma unroll
-        for (int u = 0; u < TU; ++u) y_col[(size_t)(tt + u) * inner] = fmaf(dsk, xv[u], acc[u]);
+            for (int c = 0; c < CPT; ++c) acc[c][u] += __shfl_xor_sync(0xffffffffu, acc[c][u], o);
+    }
+    if (s == 0) {
+#pragma unroll
+        for (int c = 0; c < CPT; ++c)
+            if (pl + RC_PB * c < n_p) {
+#pragma unroll
+                for (int u = 0; u < TU; ++u)
+                    y_col[(size_t)(tt + u) * inner + RC_PB * c] = fmaf(dsk, xv[c][u], acc[c][u]);
+            }
     }
 }
 
-template <int NREG, bool VEC, int NS>
+template <int NREG, bool VEC, int NS, int CPT>
 __global__ void __launch_bounds__(RC_PB * NS) ssm_scan_kernel(ScanArgs a) {
     // (the kernel behind this one is let in only after the walk, further down: a block here runs
     // for as long as its row is, and blocks of the next kernel that wait beside it on the same SM
     // slowed it down: a prompt of 2,048 tokens through six layer runs 3.54 ms against 2.89 ms
     // without early launches)
+    constexpr int PB = RC_PB * CPT;               // columns of a block
     extern __shared__ __align__(16) float rc_smem[];
-    const int b = blockIdx.x, h = blockIdx.y, p0 = blockIdx.z * RC_PB;
+    const int b = blockIdx.x, h = blockIdx.y, p0 = blockIdx.z * PB;
     const int tid = threadIdx.x, s = tid & (NS - 1), pl = tid / NS;
     const int p = p0 + pl;
-    const int n_p = min(RC_PB, a.P - p0);
-    const bool p_ok = pl < n_p;
+    const int n_p = min(PB, a.P - p0);
     const int N = a.N, P = a.P;
     // two buffers of a chunk's x, B and C (the next chunk travels while this one is walked),
     // then the chunks' step sizes and decays
-    const int buf_floats = RC_TC * (RC_PB + 2 * N);
+    const int buf_floats = RC_TC * (PB + 2 * N);
     float* dts = rc_smem + 2 * buf_floats;        // [2][TC]
     float* das = dts + 2 * RC_TC;                 // [2][TC]
     const int g = h / (a.heads / a.groups);
@@ -314,19 +333,19 @@ __global__ void __launch_bounds__(RC_PB * NS) ssm_scan_kernel(ScanArgs a) {
     auto fetch = [&](int c0, int buf) {
         const int nc = min(RC_TC, n_b - c0);
         float* xs = rc_smem + buf * buf_floats;
-        float* Bs = xs + RC_TC * RC_PB;
+        float* Bs = xs + RC_TC * PB;
         float* Cs = Bs + RC_TC * N;
         const float* base = a.u + (size_t)(t0 + c0) * a.channels;
         if (x16) {
             const int q = n_p >> 2;
             for (int i = tid; i < nc * q; i += blockDim.x) {
                 const int tt = i / q, pp = (i - tt * q) << 2;
-                rc_cp_async16(xs + tt * RC_PB + pp, base + (size_t)tt * a.channels + h * P + p0 + pp);
+                rc_cp_async16(xs + tt * PB + pp, base + (size_t)tt * a.channels + h * P + p0 + pp);
             }
         } else {
             for (int i = tid; i < nc * n_p; i += blockDim.x) {
                 const int tt = i / n_p, pp = i - tt * n_p;
-                rc_cp_async4(xs + tt * RC_PB + pp, base + (size_t)tt * a.channels + h * P + p0 + pp);
+                rc_cp_async4(xs + tt * PB + pp, base + (size_t)tt * a.channels + h * P + p0 + pp);
             }
         }
         if (VEC && (a.channels & 3) == 0 && ((inner + g * N) & 3) == 0) {
@@ -353,19 +372,24 @@ __global__ void __launch_bounds__(RC_PB * NS) ssm_scan_kernel(ScanArgs a) {
         }
     };
     if (n_b > 0) fetch(0, 0);
-    float* st = a.state + (((size_t)slot * a.heads + h) * P + (p_ok ? p : p0)) * N;
-    float S[NREG];
-    if (VEC) {
+    float* st[CPT];                               // (a column that is not there: its neighbour's, unused)
+    float S[CPT][NREG];
 #pragma unroll
-        for (int j = 0; j < NREG / 4; ++j) {
-            const int n = 4 * (s + NS * j);
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (p_ok && n < N) v = *reinterpret_cast<const float4*>(st + n);
-            S[4 * j] = v.x; S[4 * j + 1] = v.y; S[4 * j + 2] = v.z; S[4 * j + 3] = v.w;
+    for (int c = 0; c < CPT; ++c) {
+        const bool p_ok = pl + RC_PB * c < n_p;
+        st[c] = a.state + (((size_t)slot * a.heads + h) * P + (p_ok ? p + RC_PB * c : p0)) * N;
+        if (VEC) {
+#pragma unroll
+            for (int j = 0; j < NREG / 4; ++j) {
+                const int n = 4 * (s + NS * j);
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (p_ok && n < N) v = *reinterpret_cast<const float4*>(st[c] + n);
+                S[c][4 * j] = v.x; S[c][4 * j + 1] = v.y; S[c][4 * j + 2] = v.z; S[c][4 * j + 3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < NREG; ++r) S[c][r] = (p_ok && n_of(r) < N) ? st[c][n_of(r)] : 0.0f;
         }
-    } else {
-#pragma unroll
-        for (int r = 0; r < NREG; ++r) S[r] = (p_ok && n_of(r) < N) ? st[n_of(r)] : 0.0f;
     }
     int buf = 0;
     for (int c0 = 0; c0 < n_b; c0 += RC_TC, buf ^= 1) {
@@ -378,34 +402,36 @@ __global__ void __launch_bounds__(RC_PB * NS) ssm_scan_kernel(ScanArgs a) {
         }
         __syncthreads();
         const float* xs = rc_smem + buf * buf_floats;
-        const float* Bs = xs + RC_TC * RC_PB;
+        const float* Bs = xs + RC_TC * PB;
         const float* Cs = Bs + RC_TC * N;
         // RC_TU tokens an iteration: a token's chain (products, the column's threads' sums by
         // shuffles, the store) is long and the next token only waits for S, so the chains of
         // RC_TU tokens are issued side by side; the tokens left over go one by one
         int tt = 0;
         for (; tt + RC_TU <= nc; tt += RC_TU)
-            rc_walk<NREG, VEC, RC_TU, NS>(S, xs, Bs, Cs, dts + buf * RC_TC, das + buf * RC_TC, tt, N, s, pl, p_ok,
+            rc_walk<NREG, VEC, RC_TU, NS, CPT>(S, xs, Bs, Cs, dts + buf * RC_TC, das + buf * RC_TC, tt, N, s, pl, n_p,
                                       dsk, a.y + (size_t)(t0 + c0) * inner + h * P + p, inner);
         for (; tt < nc; ++tt)
-            rc_walk<NREG, VEC, 1, NS>(S, xs, Bs, Cs, dts + buf * RC_TC, das + buf * RC_TC, tt, N, s, pl, p_ok,
+            rc_walk<NREG, VEC, 1, NS, CPT>(S, xs, Bs, Cs, dts + buf * RC_TC, das + buf * RC_TC, tt, N, s, pl, n_p,
                                   dsk, a.y + (size_t)(t0 + c0) * inner + h * P + p, inner);
         __syncthreads();                          // the buffer may be refilled now
     }
     pdl_launch_dependents();
-    if (p_ok) {
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) {
+        if (pl + RC_PB * c >= n_p) continue;
         if (VEC) {
 #pragma unroll
             for (int j = 0; j < NREG / 4; ++j) {
                 const int n = 4 * (s + NS * j);
                 if (n < N)
-                    *reinterpret_cast<float4*>(st + n) =
-                        make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
+                    *reinterpret_cast<float4*>(st[c] + n) =
+                        make_float4(S[c][4 * j], S[c][4 * j + 1], S[c][4 * j + 2], S[c][4 * j + 3]);
             }
         } else {
 #pragma unroll
             for (int r = 0; r < NREG; ++r)
-                if (n_of(r) < N) st[n_of(r)] = S[r];
+                if (n_of(r) < N) st[c][n_of(r)] = S[c][r];
         }
     }
 }
@@ -439,41 +465,54 @@ extern "C" int mf_ssm_scan(const float* u, const float* proj, long long in_width
     const long long n_blocks = (long long)n_rows * heads * ((P + RC_PB - 1) / RC_PB);
     int ns = (vec && N >= 128 && (long long)n_tokens >= 64LL * n_rows && n_blocks <= mf_sm_count()) ? 16 : RC_NS;
     if (vec && N >= 64 && (forced == 8 || forced == 16)) ns = forced;
-    dim3 grid(n_rows, heads, (P + RC_PB - 1) / RC_PB), block(((pb * ns + 31) / 32) * 32);
-    size_t smem = (size_t)(2 * RC_TC * (RC_PB + 2 * N + 2)) * sizeof(float);
+    // Columns of a thread: two for prompts.  With one, a thread reads 8 float4 of B and C from shared
+    // memory for 48 multiply-adds and the shared memory is what the kernel waits for; with two the same
+    // reads serve 96.  Not where that leaves SMs without a block, nor for a step of few tokens, which is
+    // bound by the state it reads and writes.  Eight prompts of 601 to 1,300 tokens, 64 heads of 64
+    // columns, state 128, one column a thread -> two: 1.43 -> 1.06 ms.
+    const bool two = vec && ns == RC_NS && P > RC_PB && (long long)n_tokens >= 16LL * n_rows &&
+                     (long long)n_rows * heads * ((P + 2 * RC_PB - 1) / (2 * RC_PB)) >= mf_sm_count();
+    const int cols = two ? 2 * RC_PB : RC_PB;
+    dim3 grid(n_rows, heads, (P + cols - 1) / cols), block(((pb * ns + 31) / 32) * 32);
+    size_t smem = (size_t)(2 * RC_TC * (cols + 2 * N + 2)) * sizeof(float);
     // A block runs for as long as its row is, so the blocks must lie evenly over the SMs.  Launched
     // early (programmatic dependent launch), they are placed while the kernel before still holds
     // most SMs, and several land on one SM although others will be free in a moment (a prompt of
     // 2,048 tokens through six layer runs: 3.5 ms against 2.9 ms without early launches).  So a
     // block asks for so much shared memory that no SM takes more than its even share.
     {
-        const long long blocks = (long long)n_rows * heads * ((P + RC_PB - 1) / RC_PB);
+        const long long blocks = (long long)grid.x * grid.y * grid.z;
         const long long share = (blocks + mf_sm_count() - 1) / mf_sm_count();       // blocks an SM, evenly
         const size_t most = 227 * 1024;                // shared memory of an SM that blocks can have
         const size_t pad = most / (size_t)(share + 1) + 1024;
         if (pad > smem && pad <= most - 1024) smem = pad;
     }
     const int nreg = vec ? 4 * ((N / 4 + ns - 1) / ns) : (N + ns - 1) / ns;
-#define MF_SCAN(NR, V, S_) \
+#define MF_SCAN(NR, V, S_, C_) \
     do { \
         if (smem > 48 * 1024) \
-            cudaFuncSetAttribute(ssm_scan_kernel<NR, V, S_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        mf_launch(ssm_scan_kernel<NR, V, S_>, grid, block, smem, stream, a); \
+            cudaFuncSetAttribute(ssm_scan_kernel<NR, V, S_, C_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        mf_launch(ssm_scan_kernel<NR, V, S_, C_>, grid, block, smem, stream, a); \
     } while (0)
     if (vec && ns == 16) {
-        if (nreg <= 8) MF_SCAN(8, true, 16);
-        else MF_SCAN(16, true, 16);
+        if (nreg <= 8) MF_SCAN(8, true, 16, 1);
+        else MF_SCAN(16, true, 16, 1);
+    } else if (two) {
+        if (nreg <= 4) MF_SCAN(4, true, 8, 2);
+        else if (nreg <= 8) MF_SCAN(8, true, 8, 2);
+        else if (nreg <= 16) MF_SCAN(16, true, 8, 2);
+        else MF_SCAN(32, true, 8, 2);
     } else if (vec) {
-        if (nreg <= 4) MF_SCAN(4, true, 8);
-        else if (nreg <= 8) MF_SCAN(8, true, 8);
-        else if (nreg <= 16) MF_SCAN(16, true, 8);
-        else MF_SCAN(32, true, 8);
+        if (nreg <= 4) MF_SCAN(4, true, 8, 1);
+        else if (nreg <= 8) MF_SCAN(8, true, 8, 1);
+        else if (nreg <= 16) MF_SCAN(16, true, 8, 1);
+        else MF_SCAN(32, true, 8, 1);
     } else {
-        if (nreg <= 2) MF_SCAN(2, false, 8);
-        else if (nreg <= 4) MF_SCAN(4, false, 8);
-        else if (nreg <= 8) MF_SCAN(8, false, 8);
-        else if (nreg <= 16) MF_SCAN(16, false, 8);
-        else MF_SCAN(32, false, 8);
+        if (nreg <= 2) MF_SCAN(2, false, 8, 1);
+        else if (nreg <= 4) MF_SCAN(4, false, 8, 1);
+        else if (nreg <= 8) MF_SCAN(8, false, 8, 1);
+        else if (nreg <= 16) MF_SCAN(16, false, 8, 1);
+        else MF_SCAN(32, false, 8, 1);
     }
 #undef MF_SCAN
     return MF_LAUNCH_CHECK();
