@@ -1786,3 +1786,38 @@ extern "C" int mf_norm_terms(const NormTermsArgs* args, int n_rows, int out_dtyp
 #undef MF_NT2
     return MF_LAUNCH_CHECK();
 }
+
+// ---- the copies around a decode step, each group of calls in one -------------------------------------
+// A decode step of a small model is bound by the host that launches it; what these hold together were
+// three to five calls through the framework's Python layer each.  Events are the caller's.
+
+// A step's integers from pinned host memory, `done` recorded behind the copy (the host buffer is free
+// again then), and, if `tokens` is not null, the token ids that a kernel left on the device over the
+// first of them.
+extern "C" int mf_step_inputs(void* dev, const void* host, long long bytes, const void* tokens,
+                              long long token_bytes, cudaEvent_t done, cudaStream_t stream) {
+    if (dev == nullptr || host == nullptr || bytes <= 0 || token_bytes > bytes) return MF_ERR_ARGUMENT;
+    cudaError_t e = cudaMemcpyAsync(dev, host, (size_t)bytes, cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess) e = cudaEventRecord(done, stream);
+    if (e == cudaSuccess && tokens != nullptr && token_bytes > 0)
+        e = cudaMemcpyAsync(dev, tokens, (size_t)token_bytes, cudaMemcpyDeviceToDevice, stream);
+    return (int)e;
+}
+
+// Device memory to pinned host memory, `done` recorded behind the copy; on `side`, if that is not null,
+// behind what `stream` holds so far (`ready` is recorded there), so that later work on `stream` is not
+// waited for.
+extern "C" int mf_copy_back(void* host, const void* dev, long long bytes, cudaEvent_t ready, cudaEvent_t done,
+                            cudaStream_t side, cudaStream_t stream) {
+    if (dev == nullptr || host == nullptr || bytes <= 0) return MF_ERR_ARGUMENT;
+    cudaStream_t on = stream;
+    cudaError_t e = cudaSuccess;
+    if (side != nullptr) {
+        on = side;
+        e = cudaEventRecord(ready, stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(side, ready, 0);
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(host, dev, (size_t)bytes, cudaMemcpyDeviceToHost, on);
+    if (e == cudaSuccess) e = cudaEventRecord(done, on);
+    return (int)e;
+}

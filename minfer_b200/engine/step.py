@@ -141,7 +141,7 @@ class Engine:
         # raises if a copy that has arrived shows a bit
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._status_host = torch.zeros(1, dtype=torch.int32).pin_memory()
-        self._status_event = torch.cuda.Event()
+        self._status_event = K.made_event()
         self._status_in_flight = False
         self._graphs: Dict[tuple, dict] = {}
         self._seen_shapes: set = set()
@@ -436,11 +436,8 @@ class Engine:
         host, event = ring[slot_i]
         event.synchronize()                         # the copy that last used this buffer is done
         host.numpy()[:] = flat
-        entry["dev"].copy_(host, non_blocking=True)
-        event.record()
+        K.step_inputs(entry["dev"], host, device_tokens, event)
         self.h2d_bytes += host.numel() * 4
-        if device_tokens is not None:
-            entry["dev"][:n_live].copy_(device_tokens)
         entry["graph"].replay()
         K.launches += entry["kernels"]
         return entry["logits"][:n_live]
@@ -465,7 +462,7 @@ class Engine:
         ring = []
         for _ in range(4):
             host = torch.empty(total, dtype=torch.int32).pin_memory()
-            ring.append((host, torch.cuda.Event()))
+            ring.append((host, K.made_event()))
         entry = {"graph": graph, "dev": dev, "logits": logits, "ring": ring, "next": 0,
                  "kernels": captured}
         self._graphs[key] = entry
@@ -594,8 +591,7 @@ class Engine:
         """Sends the status word on its way to the host behind the step just launched."""
         if self._status_in_flight and not self._status_event.query():
             return                                   # the last copy is still under way
-        self._status_host.copy_(self.status, non_blocking=True)
-        self._status_event.record()
+        K.copy_back(self._status_host, self.status, self._status_event)
         self._status_in_flight = True
 
     def _raise_if_flagged(self) -> None:

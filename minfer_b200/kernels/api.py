@@ -132,6 +132,44 @@ def _sig_ops(lib: ctypes.CDLL) -> None:
     lib.mf_scaled_add.argtypes = ([c_void_p] + [c_void_p, c_void_p, c_int, c_void_p] * 2 +
                                   [c_int, c_int, c_void_p, c_float, c_void_p, c_int, c_void_p])
     lib.mf_norm_terms.argtypes = [c_void_p, c_int, c_int, c_void_p]
+    lib.mf_step_inputs.argtypes = [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p]
+    lib.mf_copy_back.argtypes = [c_void_p, c_void_p, c_longlong] + [c_void_p] * 4
+
+
+def made_event() -> torch.cuda.Event:
+    """An event whose handle exists (torch creates it at the first record)."""
+    event = torch.cuda.Event()
+    event.record()
+    return event
+
+
+def step_inputs(dev: torch.Tensor, host: torch.Tensor, tokens: Optional[torch.Tensor],
+                done: torch.cuda.Event) -> None:
+    """Copies pinned ``host`` (int32) to ``dev`` on the current stream, records ``done`` behind that, and
+    copies ``tokens`` (int32 on the device, or None) over the first of them."""
+    if (dev.dtype != torch.int32 or host.dtype != torch.int32 or dev.numel() != host.numel()
+            or not host.is_contiguous()):
+        raise KernelError("step_inputs: int32 buffers of one size")
+    n = 0
+    if tokens is not None:
+        n = tokens.numel()
+        if n > dev.numel():
+            raise KernelError("step_inputs: more tokens than the buffer takes")
+        if not tokens.is_contiguous():
+            tokens = tokens.contiguous()
+    _check(_lib("ops").mf_step_inputs(_ptr(dev, "dev"), host.data_ptr(), host.numel() * 4,
+                                      _i32(tokens, "tokens"), n * 4, done.cuda_event, _stream()), "step_inputs", 0)
+
+
+def copy_back(host: torch.Tensor, dev: torch.Tensor, done: torch.cuda.Event,
+              ready: Optional[torch.cuda.Event] = None, side: Optional[torch.cuda.Stream] = None) -> None:
+    """Copies int32 ``dev`` to pinned ``host`` behind what the current stream holds, on stream ``side`` if
+    one is given (``ready`` is recorded on the current one then), and records ``done`` behind the copy."""
+    if host.dtype != torch.int32 or host.numel() != dev.numel() or not host.is_contiguous():
+        raise KernelError("copy_back: int32 buffers of one size")
+    _check(_lib("ops").mf_copy_back(
+        host.data_ptr(), _i32(dev, "dev"), host.numel() * 4, ready.cuda_event if ready is not None else None,
+        done.cuda_event, side.cuda_stream if side is not None else None, _stream()), "copy_back", 0)
 
 
 def _sig_gemm_simt(lib: ctypes.CDLL) -> None:

@@ -36,6 +36,7 @@ class DeviceSampler:
         self._meta_host = None
         self._copy_stream = torch.cuda.Stream(device=self.device)
         self._pinned: list = []
+        self._events: list = []
         self._next_pinned = 0
 
     def begin(self, slots: Sequence[int], prompts: Sequence[Sequence[int]]) -> None:
@@ -85,9 +86,10 @@ class DeviceSampler:
         if not self._pinned or self._pinned[0].numel() < n:
             self._pinned = [torch.empty(max(n, 64), dtype=torch.int32).pin_memory()
                             for _ in range(self.RING)]
-        host = self._pinned[self._next_pinned % self.RING][:n]
+            self._events = [(K.made_event(), K.made_event()) for _ in range(self.RING)]
+        at = self._next_pinned % self.RING
         self._next_pinned += 1
-        return TokenFetch(tokens, self._copy_stream, host)
+        return TokenFetch(tokens, self._copy_stream, self._pinned[at][:n], *self._events[at])
 
     def sample(self, logits: torch.Tensor, slots: Sequence[int],
                streams: Sequence[int]) -> List[int]:
@@ -98,15 +100,10 @@ class DeviceSampler:
 class TokenFetch:
     """A device-to-host copy of a few token ids that does not wait for later work."""
 
-    def __init__(self, tokens: torch.Tensor, copy_stream: torch.cuda.Stream, host: torch.Tensor):
-        self.host = host
-        self.done = torch.cuda.Event()
-        ready = torch.cuda.Event()
-        ready.record()                                  # after the sampling kernel
-        with torch.cuda.stream(copy_stream):
-            copy_stream.wait_event(ready)
-            self.host.copy_(tokens, non_blocking=True)
-            self.done.record()
+    def __init__(self, tokens: torch.Tensor, copy_stream: torch.cuda.Stream, host: torch.Tensor,
+                 ready: torch.cuda.Event, done: torch.cuda.Event):
+        self.host, self.done = host, done
+        K.copy_back(host, tokens, done, ready, copy_stream)     # behind the sampling kernel
         self._keep = tokens                             # not freed before the copy has run
 
     def get(self) -> List[int]:
