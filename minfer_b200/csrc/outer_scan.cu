@@ -17,7 +17,7 @@
 // The scan: a block owns (row, head, a tile of columns).  Four warps walk the tokens: LD neighbouring
 // lanes share a pair of columns and hold its state elements d = 4 (l + LD i) .. + 3 in registers, so
 // that what a lane reads of q, k and the decays from shared memory (16 bytes at a time) serves two
-// columns.  The sums of eight tokens (16 numbers a lane) are formed side by side and added over the
+// columns (gla over long prompts: four, two pairs).  The sums of eight tokens (16 numbers a lane) are formed side by side and added over the
 // lanes by halving: each step sends what the partner keeps, 8 + 4 + 2 + 1 shuffles for all of them.  A
 // sum's tree does not depend on how the tokens are grouped.  Four more warps do what is not the
 // chain: they keep a ring of four chunks of tokens filled by cp.async, two chunks ahead, and prepare
@@ -147,12 +147,13 @@ __device__ __forceinline__ void os_token(float4 (&S0)[ND4], float4 (&S1)[ND4], c
 __device__ __forceinline__ float os_soft_cap(float z, float cap) { return cap * tanhf(z / cap); }
 
 // LD: lanes that share a pair of columns; ND4: float4 groups of a column a lane holds (D <= 4 LD ND4);
-// tc: tokens of a chunk
-template <int LD, int ND4, int MODE>
+// tc: tokens of a chunk; PAIRS: pairs of columns a lane has (2 c and 2 c + 1, then the same TV / PAIRS on):
+// what it reads of r, k and the decays serves them all
+template <int LD, int ND4, int MODE, int PAIRS>
 __global__ void __launch_bounds__(OS_THREADS + 32 * OS_FEED) outer_scan_kernel(OuterScanArgs a, int tc) {
     pdl_launch_dependents();
     constexpr int DP = 4 * LD * ND4;                   // padded key size
-    constexpr int TV = 2 * (OS_THREADS / LD);          // columns of a block
+    constexpr int TP = 2 * (OS_THREADS / LD), TV = PAIRS * TP;          // columns of one pair a lane, of the block
     constexpr bool DECAYS = OuterTraits<MODE>::DECAYS, BONUS = OuterTraits<MODE>::BONUS, GATES = OuterTraits<MODE>::GATES;
     constexpr int NVEC = DECAYS ? 3 : 2;               // vectors staged per token: r, k (and decays)
     extern __shared__ __align__(16) float os_smem[];
@@ -335,11 +336,10 @@ __global__ void __launch_bounds__(OS_THREADS + 32 * OS_FEED) outer_scan_kernel(O
 
     // ---- the four warps that walk the tokens ---------------------------------------------------------
     const int l = tid % LD, c = tid / LD;              // lane of the pair's group; pair of columns
-    const bool live0 = 2 * c < n_cols, live1 = 2 * c + 1 < n_cols;
+    auto column = [&](int pair, int which) { return pair * TP + 2 * c + which; };       // of the block's tile
     pdl_wait();
-    float* st0 = a.state + (((size_t)slot * a.heads + h) * cols + j0 + (live0 ? 2 * c : 0)) * D;
-    float* st1 = live1 ? st0 + D : st0;
-    float4 S0[ND4], S1[ND4];
+    float* st = a.state + (((size_t)slot * a.heads + h) * cols + j0) * D;               // the tile's columns
+    float4 S0[PAIRS][ND4], S1[PAIRS][ND4];
     const bool vec_state = (D & 3) == 0;
     auto get = [&](const float* p, int d, bool ok) {
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -356,9 +356,13 @@ __global__ void __launch_bounds__(OS_THREADS + 32 * OS_FEED) outer_scan_kernel(O
         return x;
     };
 #pragma unroll
-    for (int i = 0; i < ND4; ++i) {
-        S0[i] = get(st0, 4 * (l + LD * i), live0);
-        S1[i] = get(st1, 4 * (l + LD * i), live1);
+    for (int p = 0; p < PAIRS; ++p) {
+        const int c0 = column(p, 0), c1 = column(p, 1);
+#pragma unroll
+        for (int i = 0; i < ND4; ++i) {
+            S0[p][i] = get(st + (size_t)min(c0, n_cols - 1) * D, 4 * (l + LD * i), c0 < n_cols);
+            S1[p][i] = get(st + (size_t)min(c1, n_cols - 1) * D, 4 * (l + LD * i), c1 < n_cols);
+        }
     }
     const size_t out_row = (size_t)a.heads * Dv;
     float* out0 = a.out + (size_t)t0 * out_row + (size_t)h * Dv + j0;
@@ -383,45 +387,58 @@ __global__ void __launch_bounds__(OS_THREADS + 32 * OS_FEED) outer_scan_kernel(O
         const int token = t0 + chunk * tc;
         int tt = 0;
         for (; tt + OS_TU <= nc; tt += OS_TU) {
-            float acc[2 * OS_TU];
+            float acc[PAIRS][2 * OS_TU];
 #pragma unroll
             for (int u = 0; u < OS_TU; ++u) {
                 const int t = tt + u;
-                float2 vv = *reinterpret_cast<const float2*>(v_s + t * TV + 2 * c);
-                float keep = 0.f;
+                float keep = 0.f, factor = 1.f;
                 if (GATES) {
                     const float2 f = *reinterpret_cast<const float2*>(f_s + 2 * t);
-                    keep = f.x; vv.x *= f.y; vv.y *= f.y;
+                    keep = f.x; factor = f.y;
                 }
-                os_token<ND4, MODE>(S0, S1, r4 + t * (DP / 4), k4 + t * (DP / 4), w4 + t * (DP / 4), keep, vv.x, vv.y, LD,
-                                   acc[2 * u], acc[2 * u + 1]);
+#pragma unroll
+                for (int p = 0; p < PAIRS; ++p) {
+                    float2 vv = *reinterpret_cast<const float2*>(v_s + t * TV + column(p, 0));
+                    if (GATES) { vv.x *= factor; vv.y *= factor; }
+                    os_token<ND4, MODE>(S0[p], S1[p], r4 + t * (DP / 4), k4 + t * (DP / 4), w4 + t * (DP / 4), keep,
+                                        vv.x, vv.y, LD, acc[p][2 * u], acc[p][2 * u + 1]);
+                }
             }
-            os_reduce16<LD>(acc, l);
-            if (LD == 8) {
-                emit(acc[0], o, v_s, f_s, tt + l, 2 * c, token);
-                emit(acc[1], o, v_s, f_s, tt + l, 2 * c + 1, token);
-            } else if (LD == 16) {
-                emit(acc[0], o, v_s, f_s, tt + (l >> 1), 2 * c + (l & 1), token);
-            } else if ((l & 1) == 0) {
-                emit(acc[0], o, v_s, f_s, tt + (l >> 2), 2 * c + ((l >> 1) & 1), token);
+#pragma unroll
+            for (int p = 0; p < PAIRS; ++p) {
+                os_reduce16<LD>(acc[p], l);
+                if (LD == 8) {
+                    emit(acc[p][0], o, v_s, f_s, tt + l, column(p, 0), token);
+                    emit(acc[p][1], o, v_s, f_s, tt + l, column(p, 1), token);
+                } else if (LD == 16) {
+                    emit(acc[p][0], o, v_s, f_s, tt + (l >> 1), column(p, l & 1), token);
+                } else if ((l & 1) == 0) {
+                    emit(acc[p][0], o, v_s, f_s, tt + (l >> 2), column(p, (l >> 1) & 1), token);
+                }
             }
         }
         for (; tt < nc; ++tt) {
-            float2 vv = *reinterpret_cast<const float2*>(v_s + tt * TV + 2 * c);
-            float keep = 0.f, a0, a1;
+            float keep = 0.f, factor = 1.f;
             if (GATES) {
                 const float2 f = *reinterpret_cast<const float2*>(f_s + 2 * tt);
-                keep = f.x; vv.x *= f.y; vv.y *= f.y;
+                keep = f.x; factor = f.y;
             }
-            os_token<ND4, MODE>(S0, S1, r4 + tt * (DP / 4), k4 + tt * (DP / 4), w4 + tt * (DP / 4), keep, vv.x, vv.y, LD, a0, a1);
 #pragma unroll
-            for (int o2 = LD / 2; o2 > 0; o2 >>= 1) {
-                a0 += __shfl_xor_sync(0xffffffffu, a0, o2);
-                a1 += __shfl_xor_sync(0xffffffffu, a1, o2);
-            }
-            if (l == 0) {
-                emit(a0, o, v_s, f_s, tt, 2 * c, token);
-                emit(a1, o, v_s, f_s, tt, 2 * c + 1, token);
+            for (int p = 0; p < PAIRS; ++p) {
+                float2 vv = *reinterpret_cast<const float2*>(v_s + tt * TV + column(p, 0));
+                if (GATES) { vv.x *= factor; vv.y *= factor; }
+                float a0, a1;
+                os_token<ND4, MODE>(S0[p], S1[p], r4 + tt * (DP / 4), k4 + tt * (DP / 4), w4 + tt * (DP / 4), keep,
+                                    vv.x, vv.y, LD, a0, a1);
+#pragma unroll
+                for (int o2 = LD / 2; o2 > 0; o2 >>= 1) {
+                    a0 += __shfl_xor_sync(0xffffffffu, a0, o2);
+                    a1 += __shfl_xor_sync(0xffffffffu, a1, o2);
+                }
+                if (l == 0) {
+                    emit(a0, o, v_s, f_s, tt, column(p, 0), token);
+                    emit(a1, o, v_s, f_s, tt, column(p, 1), token);
+                }
             }
         }
         // (only a stage that will be filled again is handed back: nobody waits for the others)
@@ -438,15 +455,19 @@ __global__ void __launch_bounds__(OS_THREADS + 32 * OS_FEED) outer_scan_kernel(O
         }
     };
 #pragma unroll
-    for (int i = 0; i < ND4; ++i) {
-        if (live0) put(st0, 4 * (l + LD * i), S0[i]);
-        if (live1) put(st1, 4 * (l + LD * i), S1[i]);
+    for (int p = 0; p < PAIRS; ++p) {
+        const int c0 = column(p, 0), c1 = column(p, 1);
+#pragma unroll
+        for (int i = 0; i < ND4; ++i) {
+            if (c0 < n_cols) put(st + (size_t)c0 * D, 4 * (l + LD * i), S0[p][i]);
+            if (c1 < n_cols) put(st + (size_t)c1 * D, 4 * (l + LD * i), S1[p][i]);
+        }
     }
 }
 
-template <int LD, int ND4, int MODE>
+template <int LD, int ND4, int MODE, int PAIRS = 1>
 static int os_launch(const OuterScanArgs& a, int max_tokens, cudaStream_t stream) {
-    constexpr int DP = 4 * LD * ND4, TV = 2 * (OS_THREADS / LD), NVEC = OuterTraits<MODE>::DECAYS ? 3 : 2;
+    constexpr int DP = 4 * LD * ND4, TV = PAIRS * 2 * (OS_THREADS / LD), NVEC = OuterTraits<MODE>::DECAYS ? 3 : 2;
     // (short rows take shorter chunks, so that more blocks fit an SM: single tokens most of all)
     const int tc = max_tokens < 1 ? OS_TC : max_tokens < OS_TC ? max_tokens : OS_TC;
     auto bytes = [&](int t) { return (size_t)OS_STAGES * (t * (NVEC * DP + TV) + 4 * ((3 * t + 3) / 4)) * sizeof(float); };
@@ -454,14 +475,14 @@ static int os_launch(const OuterScanArgs& a, int max_tokens, cudaStream_t stream
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MF_ERR_UNSUPPORTED;
     if (!configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(outer_scan_kernel<LD, ND4, MODE>,
+        cudaError_t e = cudaFuncSetAttribute(outer_scan_kernel<LD, ND4, MODE, PAIRS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(OS_TC));
         if (e != cudaSuccess) return (int)e;
         configured[dev] = true;
     }
     const int cols = OuterTraits<MODE>::GATES ? a.Dv + 1 : a.Dv;
     const int tiles = (cols + TV - 1) / TV;
-    mf_launch(outer_scan_kernel<LD, ND4, MODE>, dim3(a.heads * tiles, a.n_rows), dim3(OS_THREADS + 32 * OS_FEED), bytes(tc),
+    mf_launch(outer_scan_kernel<LD, ND4, MODE, PAIRS>, dim3(a.heads * tiles, a.n_rows), dim3(OS_THREADS + 32 * OS_FEED), bytes(tc),
               stream, a, tc);
     return MF_LAUNCH_CHECK();
 }
@@ -471,6 +492,16 @@ static int os_choose(const OuterScanArgs& a, int max_tokens, cudaStream_t stream
     if (a.n_rows <= 0) return 0;
     if (a.D < 1 || a.D > OS_MAX_D || a.Dv < 1 || a.heads < 1 || a.n_rows > 65535) return MF_ERR_UNSUPPORTED;
     if (((uintptr_t)a.state & 15) != 0) return MF_ERR_UNSUPPORTED;
+    // Prompts that give every SM the two blocks it has room for also with four columns a lane take them:
+    // a lane then reads 3 float4 from shared memory for 48 multiply-adds instead of 24.  GLA_MEASURED
+    // Prompts that fill the GPU's room (two blocks an SM) also with four columns a lane take them: a lane then
+    // reads 3 float4 from shared memory for 48 multiply-adds instead of 24.  Eight prompts of 601 to 1,300
+    // tokens, 8 heads of 128 x 256: 603 -> 452 us.  (The other recurrences: not measured, left as they are.)
+    if constexpr (MODE == OS_GLA) {
+        if (a.D > 32 && a.D <= 128 && max_tokens >= 4 * OS_TC &&
+            (long long)a.n_rows * a.heads * ((a.Dv + 31) / 32) >= 2LL * mf_sm_count())
+            return a.D <= 64 ? os_launch<16, 1, MODE, 2>(a, max_tokens, stream) : os_launch<16, 2, MODE, 2>(a, max_tokens, stream);
+    }
     if (a.D <= 32) return os_launch<8, 1, MODE>(a, max_tokens, stream);
     if (a.D <= 64) return os_launch<16, 1, MODE>(a, max_tokens, stream);
     if (a.D <= 128) return os_launch<16, 2, MODE>(a, max_tokens, stream);

@@ -88,6 +88,29 @@ def test_gla_scan_over_cuts_and_slots(H, D, Dv, known, off):
     assert torch.equal(state[[1, 3, 5]], stale)
 
 
+@pytest.mark.parametrize("D,Dv", [(33, 33), (64, 64), (100, 65), (128, 250), (128, 256), (36, 40)])
+def test_gla_scan_of_long_rows_gives_the_bits_of_short_pieces(D, Dv):
+    """Long rows on a grid that fills the GPU give a lane four columns, pieces two; a column's operations
+    are the same in both, so outputs and states are too."""
+    from minfer_b200.kernels import api as K
+    H, lens, slots = 60, [131, 64, 40], [4, 0, 2]
+    n, width = sum(lens), H * (2 * D + Dv)
+    g = torch.Generator().manual_seed(D * 1000 + Dv)
+    proj = torch.randn(n, width, generator=g).to(DEV)
+    d = (torch.sigmoid(torch.randn(n, H * D, generator=g) * 3 + 2) ** 0.25).to(DEV)
+    whole = torch.randn(6, H, Dv, D, generator=g).to(DEV)
+    pieces, out, want = whole.clone(), torch.empty(n, H * Dv, device=DEV), torch.empty(n, H * Dv, device=DEV)
+    K.gla_scan(proj, 0, H * D, 2 * H * D, d, D ** -0.5, whole, _i32(_cu(lens)), _i32(slots), out, 3, max(lens))
+    for b, lo in enumerate(_cu(lens)[:-1]):
+        for at in range(lo, lo + lens[b], 24):
+            c = min(24, lo + lens[b] - at)
+            part = torch.empty(c, H * Dv, device=DEV)
+            K.gla_scan(proj[at:at + c].contiguous(), 0, H * D, 2 * H * D, d[at:at + c].contiguous(), D ** -0.5, pieces,
+                       _i32([0, c]), _i32([slots[b]]), part, 1, c)
+            want[at:at + c] = part
+    assert torch.equal(out, want) and torch.equal(whole, pieces)
+
+
 @pytest.mark.parametrize("n,rank,channels", [(1, 5, 36), (7, 64, 300), (65, 16, 128), (130, 1, 33), (200, 160, 256)])
 @pytest.mark.parametrize("tau", [1.0, 16.5])
 def test_sigmoid_decay(n, rank, channels, tau):
