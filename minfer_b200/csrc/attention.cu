@@ -175,6 +175,194 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_generic_kernel(AttnA
     }
 }
 
+// ---- float32, whole prompts ------------------------------------------------------------------
+// The generic kernel's arithmetic, in its order (the same bits), with the keys read once for 32 queries:
+// a CTA takes 32 consecutive rows of one head and walks tiles of 32 keys that it stages in shared memory
+// (two buffers, cp.async).  A warp owns eight of the rows: for the scores a lane is a key (one key read
+// serves eight rows), for the weighted sum a lane is an output dimension (one value read serves eight).
+// The generic kernel reads every key's row from L1 for every query.  130 + 255 tokens, 14 heads of 64:
+// 150 -> 50 us; four of 400: 579 -> 121.
+#define PF_ROWS 32
+#define PF_R 8
+#define PF_KEYS 32
+
+__device__ __forceinline__ void pf_copy16(float* dst, const float* src, bool real) {
+    const int bytes = real ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                 ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+static int pf_smem(int hd) {
+    return (PF_ROWS * hd + 2 * PF_KEYS * (hd + 4) + 2 * PF_KEYS * hd + PF_ROWS * PF_KEYS) * (int)sizeof(float);
+}
+
+// NI: output dimensions a lane holds (hd <= 32 NI)
+template <int NI>
+__global__ void __launch_bounds__(128) attention_packed_f32_kernel(AttnArgs a) {
+    pdl_prologue();
+    extern __shared__ __align__(16) float pf_smem_raw[];
+    __shared__ int seq_s[PF_ROWS], pos_s[PF_ROWS];
+    const int hd = a.hd, kp = hd + 4;
+    float* q_s = pf_smem_raw;                         // [PF_ROWS][hd], scaled
+    float* k_s = q_s + PF_ROWS * hd;                  // [2][PF_KEYS][hd + 4]
+    float* v_s = k_s + 2 * PF_KEYS * kp;              // [2][PF_KEYS][hd]
+    float* p_s = v_s + 2 * PF_KEYS * hd;              // [PF_ROWS][PF_KEYS]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int head = blockIdx.y, hk = head / (a.n_heads / a.n_kv);
+    const int r0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * PF_ROWS;   // late rows see more keys: first
+    const int n_rows = min(PF_ROWS, a.rows - r0);
+    if (tid < n_rows) { seq_s[tid] = a.row_seq[r0 + tid]; pos_s[tid] = a.row_pos[r0 + tid]; }
+    const float* q = (const float*)a.q;
+    const int per = hd >> 2;
+    for (int i = tid; i < PF_ROWS * per; i += 128) {
+        const int r = i / per, d = (i - r * per) * 4;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < n_rows) x = *reinterpret_cast<const float4*>(q + ((size_t)(r0 + r) * a.n_heads + head) * hd + d);
+        *reinterpret_cast<float4*>(q_s + r * hd + d) = make_float4(x.x * a.scale, x.y * a.scale, x.z * a.scale, x.w * a.scale);
+    }
+    __syncthreads();
+    const float* kbase = (const float*)a.k;
+    const float* vbase = (const float*)a.v;
+    // the rows of one sequence after another (mostly there is one)
+    for (int first = 0, next; first < n_rows; first = next) {
+        const int b = seq_s[first];
+        int top = 0;                                  // one past the last key any of them sees
+        for (next = first; next < n_rows && seq_s[next] == b; ++next) top = max(top, pos_s[next] + 1);
+        const long long packed0 = a.cu_seqlens[b];
+        auto fetch = [&](int tile) {
+            const int buf = tile & 1;
+            for (int i = tid; i < PF_KEYS * per; i += 128) {
+                const int r = i / per, d = (i - r * per) * 4, j = tile * PF_KEYS + r;
+                const long long off = ((packed0 + (j < top ? j : 0)) * a.n_kv + hk) * hd + d;
+                pf_copy16(k_s + (buf * PF_KEYS + r) * kp + d, kbase + off, j < top);
+                pf_copy16(v_s + (buf * PF_KEYS + r) * hd + d, vbase + off, j < top);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        int hi[PF_R];                                 // keys row r of this warp sees (0: not in this run of rows)
+        float m[PF_R], l[PF_R], acc[PF_R][NI];
+        int warp_top = 0;
+#pragma unroll
+        for (int r = 0; r < PF_R; ++r) {
+            const int row = warp * PF_R + r;
+            hi[r] = row >= first && row < next ? pos_s[row] + 1 : 0;
+            warp_top = max(warp_top, hi[r]);
+            m[r] = -INFINITY;
+            l[r] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < NI; ++i) acc[r][i] = 0.0f;
+        }
+        const int tiles = (top + PF_KEYS - 1) / PF_KEYS;
+        fetch(0);
+        for (int t = 0; t < tiles; ++t) {
+            if (t + 1 < tiles) {
+                fetch(t + 1);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncthreads();
+            const int j0 = t * PF_KEYS;
+            if (j0 < warp_top) {
+                const float* kt = k_s + ((t & 1) * PF_KEYS + lane) * kp;
+                const float* vt = v_s + (t & 1) * PF_KEYS * hd;
+                const float* qw = q_s + warp * PF_R * hd;
+                float dot[PF_R];
+#pragma unroll
+                for (int r = 0; r < PF_R; ++r) dot[r] = 0.0f;
+#pragma unroll 4
+                for (int d = 0; d < hd; d += 4) {
+                    const float4 kv = *reinterpret_cast<const float4*>(kt + d);
+#pragma unroll
+                    for (int r = 0; r < PF_R; ++r) {
+                        const float4 x = *reinterpret_cast<const float4*>(qw + r * hd + d);
+                        dot[r] = fmaf(x.x, kv.x, dot[r]);
+                        dot[r] = fmaf(x.y, kv.y, dot[r]);
+                        dot[r] = fmaf(x.z, kv.z, dot[r]);
+                        dot[r] = fmaf(x.w, kv.w, dot[r]);
+                    }
+                }
+                bool whole = true;                    // every row sees all keys of the tile
+#pragma unroll
+                for (int r = 0; r < PF_R; ++r) {
+                    whole &= hi[r] >= j0 + PF_KEYS;
+                    if (hi[r] <= j0) continue;        // (uniform over the warp)
+                    const bool valid = j0 + lane < hi[r];
+                    const float sc = valid ? dot[r] : -INFINITY;
+                    const float m_new = fmaxf(m[r], warp_max(sc));
+                    const float corr = expf(m[r] - m_new);
+                    const float p = valid ? expf(sc - m_new) : 0.0f;
+                    l[r] = l[r] * corr + warp_sum(p);
+                    m[r] = m_new;
+#pragma unroll
+                    for (int i = 0; i < NI; ++i) acc[r][i] *= corr;
+                    p_s[(warp * PF_R + r) * PF_KEYS + lane] = p;
+                }
+                __syncwarp();
+                const float* pw = p_s + warp * PF_R * PF_KEYS;
+                if (whole) {
+#pragma unroll 2
+                    for (int jj = 0; jj < PF_KEYS; jj += 4) {
+                        float v[4][NI];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+#pragma unroll
+                            for (int i = 0; i < NI; ++i)
+                                v[e][i] = lane + 32 * i < hd ? vt[(jj + e) * hd + lane + 32 * i] : 0.0f;
+#pragma unroll
+                        for (int r = 0; r < PF_R; ++r) {
+                            const float4 p = *reinterpret_cast<const float4*>(pw + r * PF_KEYS + jj);
+#pragma unroll
+                            for (int i = 0; i < NI; ++i) {
+                                acc[r][i] = fmaf(p.x, v[0][i], acc[r][i]);
+                                acc[r][i] = fmaf(p.y, v[1][i], acc[r][i]);
+                                acc[r][i] = fmaf(p.z, v[2][i], acc[r][i]);
+                                acc[r][i] = fmaf(p.w, v[3][i], acc[r][i]);
+                            }
+                        }
+                    }
+                } else {
+                    // (a key a row does not see takes no part in its sum, whatever its values are)
+                    for (int jj = 0; jj < PF_KEYS; ++jj) {
+                        float v[NI];
+#pragma unroll
+                        for (int i = 0; i < NI; ++i) v[i] = lane + 32 * i < hd ? vt[jj * hd + lane + 32 * i] : 0.0f;
+#pragma unroll
+                        for (int r = 0; r < PF_R; ++r) {
+                            if (j0 + jj >= hi[r]) continue;
+                            const float p = pw[r * PF_KEYS + jj];
+#pragma unroll
+                            for (int i = 0; i < NI; ++i) acc[r][i] = fmaf(p, v[i], acc[r][i]);
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            __syncthreads();                          // the buffer may be refilled now
+        }
+#pragma unroll
+        for (int r = 0; r < PF_R; ++r) {
+            if (hi[r] == 0) continue;
+            float* o = (float*)a.out + ((size_t)(r0 + warp * PF_R + r) * a.n_heads + head) * hd;
+            const float inv = 1.0f / l[r];
+#pragma unroll
+            for (int i = 0; i < NI; ++i)
+                if (lane + 32 * i < hd) o[lane + 32 * i] = acc[r][i] * inv;
+        }
+    }
+}
+
+template <int NI>
+static int launch_packed_f32(const AttnArgs& a, cudaStream_t stream) {
+    const int smem = pf_smem(a.hd);
+    cudaError_t e = cudaFuncSetAttribute(attention_packed_f32_kernel<NI>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, pf_smem(32 * NI));
+    if (e != cudaSuccess) return (int)e;
+    mf_launch(attention_packed_f32_kernel<NI>, dim3((a.rows + PF_ROWS - 1) / PF_ROWS, a.n_heads), dim3(128),
+              (size_t)smem, stream, a);
+    return MF_LAUNCH_CHECK();
+}
+
 // merges the chunks of one (row, head) in chunk order.  The chunks' maxima and sums are
 // fetched once (a load per thread), the factors exp(m_c - m) computed once per chunk; then
 // every thread sums its output dimension over the chunks with loads that do not wait for one
@@ -999,6 +1187,12 @@ extern "C" int mf_attention_packed(const void* q, const void* k, const void* v, 
     a.chunk = 0; a.n_chunks = 1; a.scale = scale;
     const long long items = (long long)rows * n_heads;
     const unsigned blocks = (unsigned)((items + ATT_WARPS - 1) / ATT_WARPS);
+    // float32 over all earlier keys (a window's tiles would start at another key for every row), from
+    // where 32 rows share their keys; 16 bytes at a time
+    if (dtype == MF_DTYPE_F32 && window == 0 && rows >= 16 && hd <= 128 && n_heads <= 65535 &&
+        (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0)
+        return hd <= 32 ? launch_packed_f32<1>(a, stream) : hd <= 64 ? launch_packed_f32<2>(a, stream)
+                                                                     : launch_packed_f32<4>(a, stream);
     if (dtype == MF_DTYPE_F32)
         mf_launch(attention_generic_kernel<float, false>, dim3(blocks), dim3(ATT_WARPS * 32), 0, stream, a);
     else if (dtype == MF_DTYPE_BF16)
