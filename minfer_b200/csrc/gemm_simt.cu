@@ -90,9 +90,11 @@ gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const float
 // issue).  Tiles lie in shared memory by k (a warp reads 4 rows x 8 column groups), the columns of a
 // k swizzled by its quarter so that the transposing stores do not conflict; the next tile's loads are
 // in flight in registers while this one is multiplied.
-// Measured (us, the 64 x 64 x 16 kernel above in brackets): 385 x 9,728 x 896 195 [387],
-// 385 x 896 x 4,864 204 [480], 385 x 151,936 x 896 2,640 [5,617], 1,600 x 8,448 x 2,048 1,192
-// [2,505] = 46 TFLOP/s of the pipe's 74.  Plain multiply-adds instead of packed ones: 2 to 7 % slower.
+// Measured (us, the 64 x 64 x 16 kernel above in brackets): 385 x 9,728 x 896 194 [387],
+// 385 x 896 x 4,864 228 [480], 64 x 896 x 4,864 95 [469], 385 x 151,936 x 896 2,630 [5,617],
+// 1,600 x 8,448 x 2,048 1,080 [2,505] = 51 TFLOP/s of the pipe's 74.  Plain multiply-adds instead of
+// packed ones: 2 to 7 % slower.  AHEAD 2 (loads two tiles ahead) for the smallest tile, whose product of
+// a tile is shorter than a trip to memory: 64 x 896 x 4,864 129 -> 95; for 64 x 64 it lost (240 -> 280).
 __device__ __forceinline__ unsigned long long f32x2(float lo, float hi) {
     unsigned long long r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -142,9 +144,9 @@ struct F32Tile {
     static constexpr int THREADS = 32 * WARPS_N * (BM_ / (4 * TM));
 };
 
-template <int BM_, int BN_, int TM, int TN, int BKT>
+template <int BM_, int BN_, int TM, int TN, int BKT, int AHEAD>
 __global__ void __launch_bounds__(F32Tile<BM_, BN_, TM, TN>::THREADS,
-                                  512 / F32Tile<BM_, BN_, TM, TN>::THREADS)
+                                  (AHEAD == 1 ? 512 : 384) / F32Tile<BM_, BN_, TM, TN>::THREADS)
 gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ bias, float* C,
                      int M, int N, int K, long long lda, long long ldw,
                      long long ldc, int accumulate) {
@@ -165,19 +167,16 @@ gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ b
         for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
 
     pdl_prologue();
-    float4 ha[FA], hw[FW];
-    f32_tile_fetch<BM_, THREADS, BKT>(A, lda, m0, M, 0, K, ha);
-    f32_tile_fetch<BN_, THREADS, BKT>(W, ldw, n0, N, 0, K, hw);
-    f32_tile_put<BM_, THREADS, BKT>(As[0], ha);
-    f32_tile_put<BN_, THREADS, BKT>(Ws[0], hw);
-    __syncthreads();
-    const int tiles = (K + BKT - 1) / BKT;
-    for (int t = 0; t < tiles; ++t) {
-        const bool more = t + 1 < tiles;
-        if (more) {
-            f32_tile_fetch<BM_, THREADS, BKT>(A, lda, m0, M, (t + 1) * BKT, K, ha);
-            f32_tile_fetch<BN_, THREADS, BKT>(W, ldw, n0, N, (t + 1) * BKT, K, hw);
-        }
+    float4 ha[AHEAD][FA], hw[AHEAD][FW];              // the next AHEAD tiles, on their way
+    auto fetch = [&](int t, int set) {
+        f32_tile_fetch<BM_, THREADS, BKT>(A, lda, m0, M, t * BKT, K, ha[set]);
+        f32_tile_fetch<BN_, THREADS, BKT>(W, ldw, n0, N, t * BKT, K, hw[set]);
+    };
+    auto put = [&](int t, int set) {
+        f32_tile_put<BM_, THREADS, BKT>(As[t & 1], ha[set]);
+        f32_tile_put<BN_, THREADS, BKT>(Ws[t & 1], hw[set]);
+    };
+    auto multiply = [&](int t) {
         const float (*at)[BM_] = As[t & 1];
         const float (*wt)[BN_] = Ws[t & 1];
 #pragma unroll
@@ -202,11 +201,22 @@ gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ b
                 }
             }
         }
-        if (more) {
-            f32_tile_put<BM_, THREADS, BKT>(As[(t + 1) & 1], ha);
-            f32_tile_put<BN_, THREADS, BKT>(Ws[(t + 1) & 1], hw);
+    };
+    // tiles beyond the last are fetched as zeros (no load) and never multiplied
+    const int tiles = (K + BKT - 1) / BKT;
+    fetch(0, 0);
+    put(0, 0);
+    if (AHEAD == 2) fetch(1, 1);
+    __syncthreads();
+    for (int t = 0; t < tiles; t += AHEAD) {
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            if (t + u >= tiles) break;
+            fetch(t + u + AHEAD, u);                  // (set u was put into shared memory a tile ago)
+            multiply(t + u);
+            put(t + u + 1, (u + 1) % AHEAD);
+            __syncthreads();
         }
-        __syncthreads();
     }
 #pragma unroll
     for (int h = 0; h < TN / 4; ++h) {
@@ -332,10 +342,10 @@ gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, co
     }
 }
 
-template <int BM_, int BN_, int TM, int TN, int BKT>
+template <int BM_, int BN_, int TM, int TN, int BKT, int AHEAD>
 static void launch_f32_tile(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
                             long long lda, long long ldw, long long ldc, int accumulate, cudaStream_t stream) {
-    mf_launch(gemm_f32_tile_kernel<BM_, BN_, TM, TN, BKT>, dim3((M + BM_ - 1) / BM_, (N + BN_ - 1) / BN_),
+    mf_launch(gemm_f32_tile_kernel<BM_, BN_, TM, TN, BKT, AHEAD>, dim3((M + BM_ - 1) / BM_, (N + BN_ - 1) / BN_),
               dim3(F32Tile<BM_, BN_, TM, TN>::THREADS), 0, stream, A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate);
 }
 
@@ -354,9 +364,11 @@ static bool launch_f32(const float* A, const float* W, const float* bias, float*
 #undef MF_FEW
         return true;
     }
-    // The tile whose fullest SM has the least to multiply.  A smaller tile loads more per
-    // multiply-add, which its rate stands for (measured with every SM full: 46, 44 and 36 TFLOP/s).
-    static const struct { int bm, bn; double rate; } tiles[] = {{128, 128, 1.0}, {64, 64, 0.95}, {32, 64, 0.78}};
+    // The tile whose fullest SM is done first.  A CTA alone on its SM waits for its own loads and barriers
+    // (`alone`); with others beside it, it takes its share of the pipe (`shared`).  Both measured, in units
+    // of the 64 x 64 tile's share: 28 us a thousand k.
+    static const struct { int bm, bn; double alone, shared; } tiles[] = {
+        {128, 128, 4.25, 3.83}, {64, 64, 1.79, 1.0}, {32, 64, 0.70, 0.61}};
     const int sms = mf_sm_count();
     int best = -1;
     double least = 0.0;
@@ -364,13 +376,14 @@ static bool launch_f32(const float* A, const float* W, const float* bias, float*
         const long long nt = ((long long)N + tiles[i].bn - 1) / tiles[i].bn;
         const long long mt = ((long long)M + tiles[i].bm - 1) / tiles[i].bm;
         if (nt > 65535) continue;                                    // the grid's second dimension
-        const double cost = (double)((nt * mt + sms - 1) / sms) * tiles[i].bm * tiles[i].bn / tiles[i].rate;
+        const double share = (double)((nt * mt + sms - 1) / sms) * tiles[i].shared;
+        const double cost = share > tiles[i].alone ? share : tiles[i].alone;
         if (best < 0 || cost < least) { best = i; least = cost; }
     }
     switch (best) {
-        case 0: launch_f32_tile<128, 128, 8, 8, 16>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;
-        case 1: launch_f32_tile<64, 64, 4, 8, 32>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;
-        case 2: launch_f32_tile<32, 64, 4, 4, 32>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;
+        case 0: launch_f32_tile<128, 128, 8, 8, 16, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;
+        case 1: launch_f32_tile<64, 64, 4, 8, 32, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;
+        case 2: launch_f32_tile<32, 64, 4, 4, 32, 2>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;
         default: return false;
     }
     return true;
