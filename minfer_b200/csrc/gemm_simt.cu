@@ -274,8 +274,7 @@ __device__ __forceinline__ void copy16_async(void* smem, const void* src, bool r
 
 template <int RT>
 __global__ void __launch_bounds__(F32Few<RT>::WARPS * 32)
-gemm_f32_few_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                    float* __restrict__ C, int M, int N, int K, long long lda, long long ldw,
+gemm_f32_few_kernel(const float* A, const float* W, const float* __restrict__ bias, float* C, int M, int N, int K, long long lda, long long ldw,
                     long long ldc, int accumulate) {
     typedef F32Few<RT> T;
     __shared__ __align__(16) float ring[T::WARPS][T::STAGES][T::ROWS][T::PITCH];
