@@ -140,8 +140,7 @@ class Engine:
         # every step it is copied to pinned host memory, and the next step (or check_status)
         # raises if a copy that has arrived shows a bit
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
-        self._status_host = torch.zeros(1, dtype=torch.int32).pin_memory()
-        self._status_event = K.made_event()
+        self._status_slot = K.PinnedSlot(1)
         self._status_in_flight = False
         self._graphs: Dict[tuple, dict] = {}
         self._seen_shapes: set = set()
@@ -433,11 +432,11 @@ class Engine:
         ring = entry["ring"]
         slot_i = entry["next"] % len(ring)
         entry["next"] += 1
-        host, event = ring[slot_i]
-        event.synchronize()                         # the copy that last used this buffer is done
-        host.numpy()[:] = flat
-        K.step_inputs(entry["dev"], host, device_tokens, event)
-        self.h2d_bytes += host.numel() * 4
+        slot = ring[slot_i]
+        slot.event.synchronize()                    # the copy that last used this buffer is done
+        slot.host.numpy()[:] = flat
+        K.step_inputs(entry["dev"], slot, device_tokens)
+        self.h2d_bytes += slot.host.numel() * 4
         entry["graph"].replay()
         K.launches += entry["kernels"]
         return entry["logits"][:n_live]
@@ -461,8 +460,7 @@ class Engine:
             self._graph_pool = graph.pool()
         ring = []
         for _ in range(4):
-            host = torch.empty(total, dtype=torch.int32).pin_memory()
-            ring.append((host, K.made_event()))
+            ring.append(K.PinnedSlot(total))
         entry = {"graph": graph, "dev": dev, "logits": logits, "ring": ring, "next": 0,
                  "kernels": captured}
         self._graphs[key] = entry
@@ -589,16 +587,16 @@ class Engine:
     # ---- the status word ----------------------------------------------------------------------
     def _post_status(self) -> None:
         """Sends the status word on its way to the host behind the step just launched."""
-        if self._status_in_flight and not self._status_event.query():
+        if self._status_in_flight and not self._status_slot.event.query():
             return                                   # the last copy is still under way
-        K.copy_back(self._status_host, self.status, self._status_event)
+        K.copy_back(self._status_slot, self.status)
         self._status_in_flight = True
 
     def _raise_if_flagged(self) -> None:
         """Raises if a copy of the status word that has arrived shows an error bit (no wait)."""
-        if self._status_in_flight and self._status_event.query():
+        if self._status_in_flight and self._status_slot.event.query():
             self._status_in_flight = False
-            if int(self._status_host[0]) != 0:
+            if int(self._status_slot.host[0]) != 0:
                 self.check_status()
 
     def check_status(self) -> None:

@@ -143,10 +143,26 @@ def made_event() -> torch.cuda.Event:
     return event
 
 
-def step_inputs(dev: torch.Tensor, host: torch.Tensor, tokens: Optional[torch.Tensor],
-                done: torch.cuda.Event) -> None:
-    """Copies pinned ``host`` (int32) to ``dev`` on the current stream, records ``done`` behind that, and
+class PinnedSlot:
+    """A pinned int32 buffer with the event behind the copy that last used it.  The copies below are not
+    known to torch's allocator of pinned memory, which would hand the buffer out again at once: a slot
+    that goes waits for its copy first."""
+
+    def __init__(self, n: int):
+        self.host = torch.zeros(n, dtype=torch.int32).pin_memory()
+        self.event = made_event()
+
+    def __del__(self):
+        try:
+            self.event.synchronize()
+        except Exception:       # (no event was made, or the context is gone)
+            pass
+
+
+def step_inputs(dev: torch.Tensor, slot: PinnedSlot, tokens: Optional[torch.Tensor]) -> None:
+    """Copies the slot's integers to ``dev`` on the current stream, records its event behind that, and
     copies ``tokens`` (int32 on the device, or None) over the first of them."""
+    host = slot.host
     if (dev.dtype != torch.int32 or host.dtype != torch.int32 or dev.numel() != host.numel()
             or not host.is_contiguous()):
         raise KernelError("step_inputs: int32 buffers of one size")
@@ -158,18 +174,21 @@ def step_inputs(dev: torch.Tensor, host: torch.Tensor, tokens: Optional[torch.Te
         if not tokens.is_contiguous():
             tokens = tokens.contiguous()
     _check(_lib("ops").mf_step_inputs(_ptr(dev, "dev"), host.data_ptr(), host.numel() * 4,
-                                      _i32(tokens, "tokens"), n * 4, done.cuda_event, _stream()), "step_inputs", 0)
+                                      _i32(tokens, "tokens"), n * 4, slot.event.cuda_event, _stream()),
+           "step_inputs", 0)
 
 
-def copy_back(host: torch.Tensor, dev: torch.Tensor, done: torch.cuda.Event,
-              ready: Optional[torch.cuda.Event] = None, side: Optional[torch.cuda.Stream] = None) -> None:
-    """Copies int32 ``dev`` to pinned ``host`` behind what the current stream holds, on stream ``side`` if
-    one is given (``ready`` is recorded on the current one then), and records ``done`` behind the copy."""
-    if host.dtype != torch.int32 or host.numel() != dev.numel() or not host.is_contiguous():
-        raise KernelError("copy_back: int32 buffers of one size")
+def copy_back(slot: PinnedSlot, dev: torch.Tensor, ready: Optional[torch.cuda.Event] = None,
+              side: Optional[torch.cuda.Stream] = None) -> None:
+    """Copies int32 ``dev`` to the first integers of the slot behind what the current stream holds, on
+    stream ``side`` if one is given (``ready`` is recorded on the current one then), and records the
+    slot's event behind the copy."""
+    n = dev.numel()
+    if n < 1 or n > slot.host.numel():
+        raise KernelError("copy_back: the buffer is too small")
     _check(_lib("ops").mf_copy_back(
-        host.data_ptr(), _i32(dev, "dev"), host.numel() * 4, ready.cuda_event if ready is not None else None,
-        done.cuda_event, side.cuda_stream if side is not None else None, _stream()), "copy_back", 0)
+        slot.host.data_ptr(), _i32(dev, "dev"), n * 4, ready.cuda_event if ready is not None else None,
+        slot.event.cuda_event, side.cuda_stream if side is not None else None, _stream()), "copy_back", 0)
 
 
 def _sig_gemm_simt(lib: ctypes.CDLL) -> None:

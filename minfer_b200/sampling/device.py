@@ -36,7 +36,6 @@ class DeviceSampler:
         self._meta_host = None
         self._copy_stream = torch.cuda.Stream(device=self.device)
         self._pinned: list = []
-        self._events: list = []
         self._next_pinned = 0
 
     def begin(self, slots: Sequence[int], prompts: Sequence[Sequence[int]]) -> None:
@@ -83,13 +82,11 @@ class DeviceSampler:
         # synchronises with the device); a buffer comes around again after RING fetches, long
         # after its tokens were read
         n = tokens.numel()
-        if not self._pinned or self._pinned[0].numel() < n:
-            self._pinned = [torch.empty(max(n, 64), dtype=torch.int32).pin_memory()
-                            for _ in range(self.RING)]
-            self._events = [(K.made_event(), K.made_event()) for _ in range(self.RING)]
-        at = self._next_pinned % self.RING
+        if not self._pinned or self._pinned[0][0].host.numel() < n:
+            self._pinned = [(K.PinnedSlot(max(n, 64)), K.made_event()) for _ in range(self.RING)]
+        slot, ready = self._pinned[self._next_pinned % self.RING]
         self._next_pinned += 1
-        return TokenFetch(tokens, self._copy_stream, self._pinned[at][:n], *self._events[at])
+        return TokenFetch(tokens, self._copy_stream, slot, ready)
 
     def sample(self, logits: torch.Tensor, slots: Sequence[int],
                streams: Sequence[int]) -> List[int]:
@@ -100,12 +97,12 @@ class DeviceSampler:
 class TokenFetch:
     """A device-to-host copy of a few token ids that does not wait for later work."""
 
-    def __init__(self, tokens: torch.Tensor, copy_stream: torch.cuda.Stream, host: torch.Tensor,
-                 ready: torch.cuda.Event, done: torch.cuda.Event):
-        self.host, self.done = host, done
-        K.copy_back(host, tokens, done, ready, copy_stream)     # behind the sampling kernel
+    def __init__(self, tokens: torch.Tensor, copy_stream: torch.cuda.Stream, slot: K.PinnedSlot,
+                 ready: torch.cuda.Event):
+        self.slot = slot
+        K.copy_back(slot, tokens, ready, copy_stream)   # behind the sampling kernel
         self._keep = tokens                             # not freed before the copy has run
 
     def get(self) -> List[int]:
-        self.done.synchronize()
-        return self.host.tolist()
+        self.slot.event.synchronize()
+        return self.slot.host[:self._keep.numel()].tolist()

@@ -96,3 +96,19 @@ def test_generation_stats_hold_device_times():
         # the device cannot have worked longer than the host waited for it
         assert st.prefill_device_seconds + st.decode_device_seconds <= \
             st.prefill_seconds + st.decode_seconds + 0.05
+
+
+def test_a_pinned_slot_waits_for_its_copy_before_its_memory_goes_back():
+    """The slot's memory may be handed out again as soon as it goes: by then the copy that uses it has ended."""
+    from minfer_b200.kernels import api as K
+    slot = K.PinnedSlot(8)
+    dev = torch.arange(8, dtype=torch.int32, device="cuda")
+    other = torch.cuda.Stream()
+    other.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(other):
+        torch.cuda._sleep(200_000_000)              # about a tenth of a second
+        K.copy_back(slot, dev)
+    event = slot.event
+    assert not event.query()
+    del slot
+    assert event.query()
