@@ -368,7 +368,7 @@ static int launch_packed_f32(const AttnArgs& a, cudaStream_t stream) {
 // every thread sums its output dimension over the chunks with loads that do not wait for one
 // another.  Dynamic shared memory: 2 * n_chunks floats.
 template <typename T>
-__global__ void attention_combine_kernel(const float* __restrict__ partial, T* __restrict__ out,
+__global__ void attention_combine_kernel(const float* partial, T* __restrict__ out,
                                          int n_chunks, int hd) {
     pdl_prologue();
     extern __shared__ float comb_s[];
@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32, MINB) attention_decode_mma_ker
         for (int nt = 0; nt < NT; ++nt) {
             const __nv_bfloat16* kr = kp + (size_t)(nt * 8 + g) * HD + 8 * t;
 #pragma unroll
-            for (int s = 0; s < HD / 32; ++s) kv[nt][s] = __ldg(reinterpret_cast<const uint4*>(kr + 32 * s));
+            for (int s = 0; s < HD / 32; ++s) kv[nt][s] = *reinterpret_cast<const uint4*>(kr + 32 * s);
         }
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) sacc[nt][0] = sacc[nt][1] = sacc[nt][2] = sacc[nt][3] = 0.0f;

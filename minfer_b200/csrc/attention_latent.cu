@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(LA_WARPS * 32) latent_decode_kernel(LatentArgs
 // formed once, then every output number is a sum of independent loads.
 #define LA_MAX_SPLITS 512
 __global__ void __launch_bounds__(256)
-latent_combine_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out, int n_splits, int vd,
+latent_combine_kernel(const float* partial, __nv_bfloat16* __restrict__ out, int n_splits, int vd,
                       int sink, const float* __restrict__ sink_logit, int n_heads) {
     pdl_prologue();
     __shared__ float f_s[LA_MAX_SPLITS];

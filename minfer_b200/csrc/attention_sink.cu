@@ -37,7 +37,7 @@
 // NI: 32-element groups of a head a lane may hold (sizes up to 32 * NI)
 template <typename T, int NI>
 __global__ void __launch_bounds__(SA_WARPS * 32)
-unit_norm_kvstore_kernel(const float* __restrict__ qkv, int n_partials, int n_tokens,
+unit_norm_kvstore_kernel(const float* qkv, int n_partials, int n_tokens,
                          const int* __restrict__ positions, const int* __restrict__ token_row,
                          const int* __restrict__ seq_end, T* __restrict__ q_out,
                          T* __restrict__ k_out, T* __restrict__ v_out, T* __restrict__ k_cache,
@@ -1062,7 +1062,7 @@ __global__ void __launch_bounds__(SD_WARPS * 32) sink_attention_decode_kernel(Si
 }
 
 // merges the splits of one (query, head) in split order and adds the sink
-__global__ void sink_decode_combine_kernel(const float* __restrict__ partial,
+__global__ void sink_decode_combine_kernel(const float* partial,
                                            __nv_bfloat16* __restrict__ out, int n_splits, int vd,
                                            int sink, const float* __restrict__ sink_logit,
                                            int n_heads) {

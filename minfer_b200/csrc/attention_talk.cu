@@ -323,8 +323,8 @@ extern "C" int mf_talk_attention(const TalkArgs* args, int paged, int dtype, cud
 // v <- (1 - lam) v + lam v_first over `width` columns of float32 rows (lam read on the device)
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-value_mix_kernel(float* __restrict__ v, long long v_width, int v_off,
-                 const float* __restrict__ first, long long first_width, int first_off,
+value_mix_kernel(float* v, long long v_width, int v_off,
+                 const float* first, long long first_width, int first_off,
                  const float* __restrict__ lam, long long total, int width) {
     pdl_launch_dependents();
     const float l = lam[0];

@@ -100,6 +100,9 @@ __device__ __forceinline__ bool elect_one() {
 // tiles, which no kernel of the step writes).  EVERY kernel executes the wait, needed or not,
 // so that completion stays transitive along the stream.  MINFER_B200_PDL=0 turns the launch
 // attribute off; the instructions are then no-ops.
+// What an earlier kernel of the step writes is never read through a const __restrict__ parameter (or
+// __ldg): such a load counts as invariant and may be moved above the wait.  __restrict__ is for weights,
+// the step's integers (copied to the device before its first kernel) and pure outputs.
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

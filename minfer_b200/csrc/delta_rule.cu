@@ -502,7 +502,7 @@ extern "C" int mf_delta_scan(const DeltaArgs* args, int max_row_tokens, int n_to
 // ------------------------------------------------------------------------------------------
 template <typename TO>
 __global__ void __launch_bounds__(256)
-head_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ gate,
+head_norm_gate_kernel(const float* o, const float* gate,
                       long long gate_width, int gate_off, const float* __restrict__ w,
                       TO* __restrict__ out, long long items, int heads, int Dv, float eps, int act) {
     pdl_prologue();

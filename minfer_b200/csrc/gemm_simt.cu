@@ -21,8 +21,8 @@
 // accumulate: 0  C = acc + bias        1  C = C + acc + bias  (C float32: residual stream)
 template <typename TA, typename TW, typename TC>
 __global__ void __launch_bounds__(256)
-gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const float* __restrict__ bias,
-                 TC* __restrict__ C, int M, int N, int K, long long lda, long long ldw,
+gemm_simt_kernel(const TA* A, const TW* __restrict__ W, const float* __restrict__ bias,
+                 TC* C, int M, int N, int K, long long lda, long long ldw,
                  long long ldc, int accumulate) {
     pdl_prologue();
     __shared__ float As[BK][BM + 4];

@@ -775,8 +775,8 @@ extern "C" int mf_wait_probe(unsigned* status, unsigned max_spin, unsigned long 
 
 // adds the K splits in order: out (+)= sum_s partial[s] + bias
 template <typename TO>
-__global__ void splitk_reduce_kernel(const float* __restrict__ partial, const float* __restrict__ bias,
-                                     TO* __restrict__ out, long long ldo, int M, int N, int splits,
+__global__ void splitk_reduce_kernel(const float* partial, const float* __restrict__ bias,
+                                     TO* out, long long ldo, int M, int N, int splits,
                                      int accumulate) {
     pdl_prologue();
     const long long total = (long long)M * N;

@@ -26,7 +26,7 @@
 #define MOE_MAX_TOP 16
 
 __global__ void __launch_bounds__(256)
-moe_route_kernel(const float* __restrict__ logits, int* __restrict__ idx, float* __restrict__ wts,
+moe_route_kernel(const float* logits, int* __restrict__ idx, float* __restrict__ wts,
                  int n_tokens, int experts, int top) {
     pdl_prologue();
     const int lane = threadIdx.x & 31;
@@ -78,7 +78,7 @@ extern "C" int mf_moe_route(const float* logits, int* idx, float* wts, int n_tok
 // block share the rows of W in L1.
 template <typename TX>
 __global__ void __launch_bounds__(256)
-router_logits_kernel(const TX* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+router_logits_kernel(const TX* x, const float* __restrict__ w, const float* __restrict__ bias,
                      float* __restrict__ logits, long long pairs, int outputs, int width) {
     pdl_prologue();
     const int lane = threadIdx.x & 31;
@@ -126,7 +126,7 @@ extern "C" int mf_router_logits(const void* x, int x_dtype, const float* w, cons
 // themselves (no correction, not renormalized).  `stride` floats separate the rows of `logits`
 // (a row may carry more columns than `experts`).  A warp per token.
 __global__ void __launch_bounds__(256)
-moe_route_scored_kernel(const float* __restrict__ logits, long long stride,
+moe_route_scored_kernel(const float* logits, long long stride,
                         const float* __restrict__ correction, int* __restrict__ idx,
                         float* __restrict__ wts, int n_tokens, int experts, int top) {
     pdl_prologue();
@@ -186,7 +186,7 @@ extern "C" int mf_moe_route_scored(const float* logits, long long stride, const 
 // first-ranked runs (groups 1: among all).  The `top` largest scores among them are chosen (ties anywhere: the
 // lower index), with weights score / (sum of the chosen scores + 1e-20) * scale.  A warp per token.
 __global__ void __launch_bounds__(256)
-moe_route_groups_kernel(const float* __restrict__ logits, long long stride, int* __restrict__ idx,
+moe_route_groups_kernel(const float* logits, long long stride, int* __restrict__ idx,
                         float* __restrict__ wts, int n_tokens, int experts, int top, int groups, int keep,
                         float scale) {
     pdl_prologue();
@@ -301,8 +301,8 @@ __device__ __forceinline__ float moe_dot(const __nv_bfloat16* w, const float* x,
 
 template <typename TX, typename TW>
 __global__ void __launch_bounds__(256)
-moe_up_kernel(const TX* __restrict__ x, const TW* __restrict__ wg, const TW* __restrict__ wu,
-              long long w_row, long long w_expert, const int* __restrict__ idx,
+moe_up_kernel(const TX* x, const TW* __restrict__ wg, const TW* __restrict__ wu,
+              long long w_row, long long w_expert, const int* idx,
               TX* __restrict__ hidden, int width, int ff, int top, int n_real, int act, float limit,
               float alpha) {
     pdl_launch_dependents();
@@ -338,9 +338,9 @@ moe_up_kernel(const TX* __restrict__ x, const TW* __restrict__ wg, const TW* __r
 
 template <typename TX, typename TW>
 __global__ void __launch_bounds__(256)
-moe_down_kernel(const TX* __restrict__ hidden, const TW* __restrict__ wd, const int* __restrict__ idx,
-                const float* __restrict__ wts, float* __restrict__ h, int width, int ff, int top,
-                int n_real, const TX* __restrict__ x, int store) {
+moe_down_kernel(const TX* hidden, const TW* __restrict__ wd, const int* idx,
+                const float* wts, float* h, int width, int ff, int top,
+                int n_real, const TX* x, int store) {
     pdl_launch_dependents();
     extern __shared__ float moe_hid[];             // [top][ff]
     const int t = blockIdx.x;                      // tokens along x, as the pairs above
@@ -396,7 +396,7 @@ extern "C" int mf_moe_experts(const void* x, int x_dtype, const void* wg, const 
 
 // ---- many tokens: grouping by expert --------------------------------------------------------
 // counts[e] = number of (token, choice) pairs that chose expert e (counts zeroed by the caller)
-__global__ void moe_counts_kernel(const int* __restrict__ idx, int* __restrict__ counts, int n_pairs) {
+__global__ void moe_counts_kernel(const int* idx, int* __restrict__ counts, int n_pairs) {
     pdl_prologue();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n_pairs) atomicAdd(&counts[idx[i]], 1);
@@ -409,7 +409,7 @@ extern "C" int mf_moe_counts(const int* idx, int* counts, int n_pairs, cudaStrea
 }
 
 // offsets[e] = counts[0] + .. + counts[e - 1], offsets[experts] = all pairs; one block
-__global__ void moe_offsets_kernel(const int* __restrict__ counts, int* __restrict__ offsets,
+__global__ void moe_offsets_kernel(const int* counts, int* __restrict__ offsets,
                                    int experts) {
     pdl_prologue();
     for (int e = threadIdx.x; e <= experts; e += blockDim.x) {
@@ -422,7 +422,7 @@ __global__ void moe_offsets_kernel(const int* __restrict__ counts, int* __restri
 // a block per expert walks all pairs in order: pair i of expert e gets row
 // where[i] = offsets[e] + (pairs of e before i), and order[where[i]] = i
 __global__ void __launch_bounds__(256)
-moe_place_kernel(const int* __restrict__ idx, const int* __restrict__ offsets,
+moe_place_kernel(const int* idx, const int* offsets,
                  int* __restrict__ order, int* __restrict__ where, int n_pairs) {
     pdl_prologue();
     __shared__ int warp_total[8];
@@ -461,7 +461,7 @@ extern "C" int mf_moe_place(const int* idx, const int* counts, int* offsets, int
 
 // rows of x (any type) picked by `pairs[i] / top` into a packed tensor of the same type
 template <typename T>
-__global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict__ pairs,
+__global__ void moe_gather_kernel(const T* x, const int* pairs,
                                   T* __restrict__ out, int width, int top) {
     pdl_prologue();
     const T* xr = x + (size_t)(pairs[blockIdx.x] / top) * width;
@@ -471,7 +471,7 @@ __global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict
 
 // the same 16 bytes a thread at a time, for rows that are whole numbers of them
 __global__ void __launch_bounds__(256)
-moe_gather_vec_kernel(const uint4* __restrict__ x, const int* __restrict__ pairs, uint4* __restrict__ out,
+moe_gather_vec_kernel(const uint4* x, const int* pairs, uint4* __restrict__ out,
                       int per_row, int top) {
     pdl_prologue();
     const uint4* xr = x + (size_t)(pairs[blockIdx.x] / top) * per_row;
@@ -483,7 +483,7 @@ moe_gather_vec_kernel(const uint4* __restrict__ x, const int* __restrict__ pairs
 // the pairs before it (experts in order, an expert's pairs in their order), which is its row, and
 // copies the token's input there; the first block also writes the experts' first rows.
 __global__ void __launch_bounds__(256)
-moe_group_few_kernel(const int* __restrict__ idx, int n_pairs, int experts, int top, const uint4* __restrict__ x,
+moe_group_few_kernel(const int* idx, int n_pairs, int experts, int top, const uint4* x,
                      uint4* __restrict__ out, int per_row, int* __restrict__ offsets, int* __restrict__ where) {
     pdl_prologue();
     extern __shared__ int mg_idx[];
@@ -539,8 +539,8 @@ extern "C" int mf_moe_gather(const void* x, int dtype, const int* pairs, void* o
 // h[t][:] += (store: =) sum over the token's choices k, in order, of wts[t][k] * y[where[t * top + k]][:],
 // `where` the row of pair (t, k) in the experts' packed output; one thread owns an element
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ where,
-                   const float* __restrict__ wts, float* __restrict__ h, int n_tokens, int width,
+moe_combine_kernel(const float* y, const int* where,
+                   const float* wts, float* h, int n_tokens, int width,
                    int top, int store) {
     pdl_prologue();
     const long long total = (long long)n_tokens * width;

@@ -17,7 +17,7 @@
 // unscaled (learned position vectors: row_idx = the tokens' positions); an index outside it sets
 // MF_STATUS_BAD_POSITION and adds nothing.
 template <typename T, typename TR>
-__global__ void embed_kernel(const T* __restrict__ table, const int* __restrict__ ids,
+__global__ void embed_kernel(const T* __restrict__ table, const int* ids,
                              float* __restrict__ out, int width, int vocab, float scale,
                              const TR* __restrict__ rows, const int* __restrict__ row_idx,
                              int n_rows_table, unsigned* __restrict__ status) {
@@ -83,7 +83,7 @@ extern "C" int mf_embed(const void* table, int table_dtype, const int* ids, floa
 // input row of output row r).  y = x * rsqrt(mean(x^2) + eps) * w
 // ------------------------------------------------------------------------------------
 template <typename TO>
-__global__ void rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void rmsnorm_kernel(const float* x, const float* __restrict__ w,
                                const int* __restrict__ rows, TO* __restrict__ y, int width,
                                float eps) {
     pdl_prologue();
@@ -122,7 +122,7 @@ template <> struct Pack4<__nv_bfloat16> {
 // widths that are multiples of 4 up to 16384
 template <typename TO>
 __global__ void __launch_bounds__(1024)
-rmsnorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w,
+rmsnorm_vec_kernel(const float* x, const float* __restrict__ w,
                    const int* __restrict__ rows, TO* __restrict__ y, int width, float eps) {
     // the norm's weights (and the row to take, an input of the step) are fetched while the
     // kernel before this one still runs
@@ -199,7 +199,7 @@ extern "C" int mf_rmsnorm(const float* x, const float* w, const int* rows, void*
 // separate reduction kernel and one round trip of h.
 // ------------------------------------------------------------------------------------
 template <typename TO>
-__global__ void add_rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ partial,
+__global__ void add_rmsnorm_kernel(float* h, const float* partial,
                                    int n_partials, const float* __restrict__ bias,
                                    const float* __restrict__ w, TO* __restrict__ y, int n_rows,
                                    int width, float eps) {
@@ -230,7 +230,7 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ h, const float* __restric
 #define ARN_MAXV 4
 template <typename TO, int MAXV>
 __global__ void __launch_bounds__(1024)
-add_rmsnorm_vec_kernel(float* __restrict__ h, const float* __restrict__ partial, int n_partials,
+add_rmsnorm_vec_kernel(float* h, const float* partial, int n_partials,
                        const float* __restrict__ bias, const float* __restrict__ w,
                        TO* __restrict__ y, int n_rows, int width, float eps) {
     // the norm's weights are fetched while the kernel before this one still runs
@@ -268,11 +268,15 @@ add_rmsnorm_vec_kernel(float* __restrict__ h, const float* __restrict__ partial,
             }
             if (MAXV != 1) v = hr[i];
             v.x += acc.x; v.y += acc.y; v.z += acc.z; v.w += acc.w;
-            hr[i] = v;
             row[j] = v;
             ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss);
             ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
         }
+    }
+#pragma unroll
+    for (int j = 0; j < MAXV; ++j) {                  // (behind all loads: none waits behind a store)
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < nv) hr[i] = row[j];
     }
     ss = block_sum(ss, scratch);
     const float scale = 1.0f / sqrtf(ss / (float)width + eps);
@@ -361,7 +365,7 @@ __device__ __forceinline__ float rotary_angle(int pos, double inv_freq) {
 }
 
 template <typename T>
-__global__ void rope_kvstore_kernel(const float* __restrict__ qkv, int n_partials, int n_tokens,
+__global__ void rope_kvstore_kernel(const float* qkv, int n_partials, int n_tokens,
                                     const float* __restrict__ bias,
                                     const int* __restrict__ positions,
                                     const int* __restrict__ token_row,
@@ -467,7 +471,7 @@ __global__ void rope_kvstore_kernel(const float* __restrict__ qkv, int n_partial
 // a long prompt share an SM and hide each other's loads.
 template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(128)
-rope_kvstore_vec_kernel(const float* __restrict__ qkv, int n_partials, int n_tokens,
+rope_kvstore_vec_kernel(const float* qkv, int n_partials, int n_tokens,
                         const float* __restrict__ bias, const int* __restrict__ positions,
                         const int* __restrict__ token_row, const int* __restrict__ seq_end,
                         const double* __restrict__ inv_freq, T* __restrict__ q_out,
@@ -665,7 +669,7 @@ __device__ __forceinline__ float gate_activation(float g, int act) {
 }
 
 template <typename TI, typename TO>
-__global__ void swiglu_kernel(const TI* __restrict__ gu, TO* __restrict__ out, int nf,
+__global__ void swiglu_kernel(const TI* gu, TO* __restrict__ out, int nf,
                               long long total, int interleaved, int act) {
     pdl_prologue();
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -701,7 +705,7 @@ extern "C" int mf_swiglu(const void* gu, int in_dtype, void* out, int out_dtype,
 // ------------------------------------------------------------------------------------
 // row gather of the float32 residual stream: out[r][:] = x[rows[r]][:]
 // ------------------------------------------------------------------------------------
-__global__ void gather_rows_kernel(const float* __restrict__ x, const int* __restrict__ rows,
+__global__ void gather_rows_kernel(const float* x, const int* __restrict__ rows,
                                    float* __restrict__ out, int width) {
     pdl_prologue();
     const float* xr = x + (size_t)rows[blockIdx.x] * width;
@@ -720,7 +724,7 @@ extern "C" int mf_gather_rows(const float* x, const int* rows, float* out, int n
 // cast between float32 and bfloat16 (round to nearest even)
 // ------------------------------------------------------------------------------------
 template <typename TI, typename TO>
-__global__ void cast_kernel(const TI* __restrict__ in, TO* __restrict__ out, long long n) {
+__global__ void cast_kernel(const TI* in, TO* __restrict__ out, long long n) {
     pdl_prologue();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x)
@@ -751,8 +755,8 @@ extern "C" int mf_cast(const void* in, int in_dtype, void* out, int out_dtype, l
 // status bit and adds nothing.
 // ------------------------------------------------------------------------------------
 template <typename T>
-__global__ void add_rows_kernel(float* __restrict__ h, const T* __restrict__ table,
-                                const int* __restrict__ idx, int width, int n_table,
+__global__ void add_rows_kernel(float* h, const T* __restrict__ table,
+                                const int* idx, int width, int n_table,
                                 unsigned* __restrict__ status) {
     pdl_launch_dependents();
     const int t = blockIdx.x;
@@ -800,13 +804,13 @@ extern "C" int mf_add_rows(float* h, const void* table, int table_dtype, const i
 // SPLITS: compiled with the addition of the K splits (kept out of the form for prompts, which
 // then needs few registers and shares an SM among several rows).
 template <typename TO, bool SPLITS>
-__global__ void norm_shift_kernel(float* x, const float* __restrict__ partial, int n_partials,
+__global__ void norm_shift_kernel(float* x, const float* partial, int n_partials,
                                   const float* __restrict__ bias, int n_tokens,
                                   const float* __restrict__ w, const float* __restrict__ shift,
                                   const int* __restrict__ positions,
                                   const int* __restrict__ token_row,
                                   const int* __restrict__ cu_seqlens,
-                                  const int* __restrict__ slots, float* __restrict__ state,
+                                  const int* __restrict__ slots, float* state,
                                   TO* __restrict__ y, int width, float eps) {
     pdl_launch_dependents();
     __shared__ float scratch[33];
@@ -888,10 +892,10 @@ __global__ void norm_shift_kernel(float* x, const float* __restrict__ partial, i
 // registers, one pass over memory; widths that are multiples of 4 up to 8 * blockDim
 template <typename TO>
 __global__ void __launch_bounds__(1024)
-norm_shift_vec_kernel(const float* __restrict__ x, const float* __restrict__ w,
+norm_shift_vec_kernel(const float* x, const float* __restrict__ w,
                       const float* __restrict__ shift, const int* __restrict__ positions,
                       const int* __restrict__ token_row, const int* __restrict__ cu_seqlens,
-                      const int* __restrict__ slots, float* __restrict__ state,
+                      const int* __restrict__ slots, float* state,
                       TO* __restrict__ y, int width, float eps) {
     pdl_launch_dependents();
     __shared__ float scratch[33];
@@ -959,9 +963,9 @@ norm_shift_vec_kernel(const float* __restrict__ x, const float* __restrict__ w,
     }
 }
 
-__global__ void norm_shift_save_kernel(const float* __restrict__ x, const float* __restrict__ w,
+__global__ void norm_shift_save_kernel(const float* x, const float* __restrict__ w,
                                        const int* __restrict__ cu_seqlens,
-                                       const int* __restrict__ slots, float* __restrict__ state,
+                                       const int* __restrict__ slots, float* state,
                                        int width, float eps) {
     pdl_launch_dependents();
     __shared__ float scratch[33];
@@ -1040,8 +1044,8 @@ __device__ __forceinline__ float xielu_f32(float z, float cp, float cn) {
 }
 
 template <typename TI, typename TO>
-__global__ void xielu_kernel(const TI* __restrict__ in, TO* __restrict__ out,
-                             const float* __restrict__ a, long long total) {
+__global__ void xielu_kernel(const TI* in, TO* __restrict__ out,
+                             const float* a, long long total) {
     pdl_launch_dependents();
     const float cp = softplus_f32(a[0]), cn = 0.5f + softplus_f32(a[1]);      // weights
     pdl_wait();
@@ -1070,7 +1074,7 @@ extern "C" int mf_xielu(const void* in, int in_dtype, void* out, int out_dtype, 
 // ------------------------------------------------------------------------------------
 // soft cap: x <- cap * tanh(x / cap), in place, float32 (logits)
 // ------------------------------------------------------------------------------------
-__global__ void tanh_cap_kernel(float* __restrict__ x, long long n, float cap, float inv_cap) {
+__global__ void tanh_cap_kernel(float* x, long long n, float cap, float inv_cap) {
     pdl_prologue();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x)
@@ -1092,7 +1096,7 @@ extern "C" int mf_tanh_cap(float* x, long long n, float cap, cudaStream_t stream
 // the residual stream before its first layer
 // ------------------------------------------------------------------------------------
 template <typename TV>
-__global__ void add_stream_kernel(float* __restrict__ h, const float* __restrict__ other,
+__global__ void add_stream_kernel(float* h, const float* other,
                                   const TV* __restrict__ vec, long long total, int width) {
     pdl_prologue();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -1128,7 +1132,7 @@ extern "C" int mf_add_stream(float* h, const float* other, const void* vec, int 
 // ------------------------------------------------------------------------------------
 template <typename TO>
 __global__ void __launch_bounds__(256)
-poly_norm_kernel(const float* __restrict__ z, const float* __restrict__ coef, TO* __restrict__ out,
+poly_norm_kernel(const float* z, const float* __restrict__ coef, TO* __restrict__ out,
                  int width, float eps) {
     pdl_launch_dependents();
     __shared__ float scratch[33];
@@ -1174,8 +1178,8 @@ extern "C" int mf_poly_norm(const float* z, const float* coef, void* out, int ou
 // `hist` [n_hist][hist_rows][width]; `last` (the newest stream) has the output's rows already.
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-depth_mix_kernel(const float* __restrict__ hist, long long hist_stride, int n_hist,
-                 const int* __restrict__ rows, const float* __restrict__ last,
+depth_mix_kernel(const float* hist, long long hist_stride, int n_hist,
+                 const int* __restrict__ rows, const float* last,
                  const float* __restrict__ w, float* __restrict__ out, int n_rows, int width) {
     pdl_prologue();
     const long long total = (long long)n_rows * width;
@@ -1208,7 +1212,7 @@ extern "C" int mf_depth_mix(const float* hist, long long hist_stride, int n_hist
 // optional bias.  A block per row; the row's y is kept in shared memory between the two passes.
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024)
-norm_add_kernel(float* __restrict__ h, const float* __restrict__ base, const float* __restrict__ partial,
+norm_add_kernel(float* h, const float* base, const float* partial,
                 int n_partials, long long split_stride, const float* __restrict__ bias,
                 const float* __restrict__ w, int width, float eps, float mult,
                 __nv_bfloat16* __restrict__ x_out) {
@@ -1276,7 +1280,7 @@ __device__ __forceinline__ float act_gelu_tanh(float z) {
 }
 
 template <typename TO>
-__global__ void unary_act_kernel(const float* __restrict__ z, TO* __restrict__ out, long long n, int kind) {
+__global__ void unary_act_kernel(const float* z, TO* __restrict__ out, long long n, int kind) {
     pdl_prologue();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
@@ -1306,8 +1310,8 @@ extern "C" int mf_unary_act(const float* z, void* out, int out_dtype, long long 
 }
 
 template <typename TO>
-__global__ void gated_act_kernel(const float* __restrict__ gu, TO* __restrict__ out, long long total, int ff,
-                                 int kind, float limit, float alpha, const float* __restrict__ row_gate,
+__global__ void gated_act_kernel(const float* gu, TO* __restrict__ out, long long total, int ff,
+                                 int kind, float limit, float alpha, const float* row_gate,
                                  long long row_gate_stride, int interleaved) {
     pdl_prologue();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -1346,7 +1350,7 @@ extern "C" int mf_gated_act(const float* gu, void* out, int out_dtype, int n_row
 }
 
 template <typename T>
-__global__ void gate_mul_kernel(T* __restrict__ o, const float* __restrict__ gate, long long gate_width,
+__global__ void gate_mul_kernel(T* o, const float* gate, long long gate_width,
                                 int gate_off, long long total, int width, float mul) {
     pdl_prologue();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -1373,7 +1377,7 @@ extern "C" int mf_gate_mul(void* o, int dtype, const float* gate, long long gate
 }
 
 template <typename T>
-__global__ void row_gate_mul_kernel(T* __restrict__ o, const float* __restrict__ gate, long long gate_stride,
+__global__ void row_gate_mul_kernel(T* o, const float* gate, long long gate_stride,
                                     long long total, int width) {
     pdl_prologue();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -1398,8 +1402,8 @@ extern "C" int mf_row_gate_mul(void* o, int dtype, const float* gate, long long 
 }
 
 template <typename TT, typename TO>
-__global__ void table_gate_kernel(const float* __restrict__ a, const TT* __restrict__ table, long long table_width,
-                                  int off, const int* __restrict__ ids, const int* __restrict__ rows,
+__global__ void table_gate_kernel(const float* a, const TT* __restrict__ table, long long table_width,
+                                  int off, const int* ids, const int* __restrict__ rows,
                                   TO* __restrict__ out, long long total, int dim, int vocab,
                                   unsigned* __restrict__ status) {
     pdl_prologue();
@@ -1463,7 +1467,7 @@ __device__ __forceinline__ void row_store(T* p, const float* v) {
 
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256)
-shift_mix_kernel(const T* __restrict__ x, const float* __restrict__ mu, int n_mix, int n_tokens, int width,
+shift_mix_kernel(const T* x, const float* __restrict__ mu, int n_mix, int n_tokens, int width,
                  const int* __restrict__ token_row, const int* __restrict__ cu_seqlens,
                  const int* __restrict__ slots, float* prev, T* __restrict__ out, int single) {
     pdl_launch_dependents();
@@ -1493,8 +1497,8 @@ shift_mix_kernel(const T* __restrict__ x, const float* __restrict__ mu, int n_mi
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-shift_keep_kernel(const T* __restrict__ x, int width, const int* __restrict__ cu_seqlens,
-                  const int* __restrict__ slots, float* __restrict__ prev) {
+shift_keep_kernel(const T* x, int width, const int* __restrict__ cu_seqlens,
+                  const int* __restrict__ slots, float* prev) {
     pdl_prologue();
     const int b = blockIdx.x, last = cu_seqlens[b + 1] - 1;
     if (last < cu_seqlens[b]) return;
@@ -1559,7 +1563,7 @@ __device__ __forceinline__ void term_value(const ScaledTerm& s, size_t at, size_
 
 template <typename TO, int VEC>
 __global__ void __launch_bounds__(1024)
-scaled_add_kernel(float* __restrict__ h, ScaledTerm s1, ScaledTerm s2, int width, const float* __restrict__ norm_w,
+scaled_add_kernel(float* h, ScaledTerm s1, ScaledTerm s2, int width, const float* __restrict__ norm_w,
                   float eps, TO* __restrict__ x_out) {
     pdl_prologue();
     __shared__ float scratch[33];
@@ -1589,8 +1593,12 @@ scaled_add_kernel(float* __restrict__ h, ScaledTerm s1, ScaledTerm s2, int width
                 row[r][j] += v[j];
                 ss = fmaf(row[r][j], row[r][j], ss);
             }
-            row_store<float, VEC>(h + base + i, row[r]);
         }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {                     // (behind all loads: none waits behind a store)
+        const int i = (threadIdx.x + r * blockDim.x) * VEC;
+        if (i < width) row_store<float, VEC>(h + base + i, row[r]);
     }
     if (x_out == nullptr) return;
     ss = block_sum(ss, scratch);

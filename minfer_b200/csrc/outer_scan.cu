@@ -529,7 +529,7 @@ extern "C" int mf_gla_scan(const OuterScanArgs* args, int max_tokens, cudaStream
 
 template <int NT, bool SIGMOID>
 __global__ void __launch_bounds__(128)
-low_rank_decay_kernel(const float* __restrict__ t1, long long t1_width, const float* __restrict__ w2t,
+low_rank_decay_kernel(const float* t1, long long t1_width, const float* __restrict__ w2t,
                  const float* __restrict__ w0, float* __restrict__ out, int n_tokens, int rank, int channels,
                       float inv_tau) {
     pdl_prologue();

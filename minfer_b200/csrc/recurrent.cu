@@ -35,9 +35,9 @@ __device__ __forceinline__ float rc_softplus(float v) {
 // one thread per (token, channel); `single`: every row brings one token and the thread also
 // writes the state
 __global__ void __launch_bounds__(256)
-conv_silu_kernel(const float* __restrict__ proj, long long in_width, int x_off, int channels,
+conv_silu_kernel(const float* proj, long long in_width, int x_off, int channels,
                  int taps, const float* __restrict__ w, const float* __restrict__ bias,
-                 float* __restrict__ state, const int* __restrict__ token_row,
+                 float* state, const int* __restrict__ token_row,
                  const int* __restrict__ cu_seqlens, const int* __restrict__ slots,
                  float* __restrict__ out, long long total, int single, int plain) {
     pdl_launch_dependents();
@@ -82,9 +82,9 @@ conv_silu_kernel(const float* __restrict__ proj, long long in_width, int x_off, 
 // the row's earlier tokens or from the slot's state).
 #define RC_CONV_TB 16
 __global__ void __launch_bounds__(256)
-conv_silu_run_kernel(const float* __restrict__ proj, long long in_width, int x_off, int channels,
+conv_silu_run_kernel(const float* proj, long long in_width, int x_off, int channels,
                      int taps, const float* __restrict__ w, const float* __restrict__ bias,
-                     const float* __restrict__ state, const int* __restrict__ token_row,
+                     const float* state, const int* __restrict__ token_row,
                      const int* __restrict__ cu_seqlens, const int* __restrict__ slots,
                      float* __restrict__ out, int n_tokens, int plain) {
     pdl_launch_dependents();
@@ -128,8 +128,8 @@ conv_silu_run_kernel(const float* __restrict__ proj, long long in_width, int x_o
 
 // one thread per (row, channel): the state after the row's tokens
 __global__ void __launch_bounds__(256)
-conv_state_kernel(const float* __restrict__ proj, long long in_width, int x_off, int channels,
-                  int taps, float* __restrict__ state, const int* __restrict__ cu_seqlens,
+conv_state_kernel(const float* proj, long long in_width, int x_off, int channels,
+                  int taps, float* state, const int* __restrict__ cu_seqlens,
                   const int* __restrict__ slots, long long total) {
     pdl_launch_dependents();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -523,7 +523,7 @@ extern "C" int mf_ssm_scan(const float* u, const float* proj, long long in_width
 // ------------------------------------------------------------------------------------------
 template <typename TO>
 __global__ void __launch_bounds__(256)
-gated_group_norm_kernel(const float* __restrict__ y, const float* __restrict__ proj,
+gated_group_norm_kernel(const float* y, const float* proj,
                         long long in_width, int z_off, const float* __restrict__ w,
                         TO* __restrict__ out, int inner, int groups, float eps) {
     pdl_prologue();
@@ -566,7 +566,7 @@ template <> struct RcStore4<__nv_bfloat16> {
 #define GN_MAXV 4
 template <typename TO>
 __global__ void __launch_bounds__(1024)
-gated_group_norm_vec_kernel(const float* __restrict__ y, const float* __restrict__ proj,
+gated_group_norm_vec_kernel(const float* y, const float* proj,
                             long long in_width, int z_off, const float* __restrict__ w,
                             TO* __restrict__ out, int inner, int groups, float eps) {
     pdl_launch_dependents();

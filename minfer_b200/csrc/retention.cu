@@ -211,9 +211,9 @@ extern "C" int mf_retention_scan(const RetentionArgs* args, cudaStream_t stream)
 
 template <typename TO>
 __global__ void __launch_bounds__(256)
-unit_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ gate, long long gate_width,
+unit_norm_gate_kernel(const float* o, const float* gate, long long gate_width,
                       int gate_off, TO* __restrict__ out, long long items, int heads, int Dv, float eps,
-                      int act, float mul, const float* __restrict__ den, const float* __restrict__ weight) {
+                      int act, float mul, const float* den, const float* __restrict__ weight) {
     pdl_prologue();
     const int lane = threadIdx.x & 31;
     const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
