@@ -136,11 +136,12 @@ def _sig_ops(lib: ctypes.CDLL) -> None:
     lib.mf_copy_back.argtypes = [c_void_p, c_void_p, c_longlong] + [c_void_p] * 4
 
 
-def made_event() -> torch.cuda.Event:
-    """An event whose handle exists (torch creates it at the first record)."""
-    event = torch.cuda.Event()
-    event.record()
-    return event
+def _event_handle(event: torch.cuda.Event) -> int:
+    """The handle of an event, made here if it has none: torch makes it at the first record, on the device
+    that is current then, and only that device's streams can record it.  So not before its first use."""
+    if not event.cuda_event:
+        event.record()
+    return event.cuda_event
 
 
 class PinnedSlot:
@@ -150,7 +151,7 @@ class PinnedSlot:
 
     def __init__(self, n: int):
         self.host = torch.zeros(n, dtype=torch.int32).pin_memory()
-        self.event = made_event()
+        self.event = torch.cuda.Event()
 
     def __del__(self):
         try:
@@ -174,7 +175,7 @@ def step_inputs(dev: torch.Tensor, slot: PinnedSlot, tokens: Optional[torch.Tens
         if not tokens.is_contiguous():
             tokens = tokens.contiguous()
     _check(_lib("ops").mf_step_inputs(_ptr(dev, "dev"), host.data_ptr(), host.numel() * 4,
-                                      _i32(tokens, "tokens"), n * 4, slot.event.cuda_event, _stream()),
+                                      _i32(tokens, "tokens"), n * 4, _event_handle(slot.event), _stream()),
            "step_inputs", 0)
 
 
@@ -187,8 +188,8 @@ def copy_back(slot: PinnedSlot, dev: torch.Tensor, ready: Optional[torch.cuda.Ev
     if n < 1 or n > slot.host.numel():
         raise KernelError("copy_back: the buffer is too small")
     _check(_lib("ops").mf_copy_back(
-        slot.host.data_ptr(), _i32(dev, "dev"), n * 4, ready.cuda_event if ready is not None else None,
-        slot.event.cuda_event, side.cuda_stream if side is not None else None, _stream()), "copy_back", 0)
+        slot.host.data_ptr(), _i32(dev, "dev"), n * 4, _event_handle(ready) if ready is not None else None,
+        _event_handle(slot.event), side.cuda_stream if side is not None else None, _stream()), "copy_back", 0)
 
 
 def _sig_gemm_simt(lib: ctypes.CDLL) -> None:

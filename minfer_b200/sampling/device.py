@@ -83,7 +83,7 @@ class DeviceSampler:
         # after its tokens were read
         n = tokens.numel()
         if not self._pinned or self._pinned[0][0].host.numel() < n:
-            self._pinned = [(K.PinnedSlot(max(n, 64)), K.made_event()) for _ in range(self.RING)]
+            self._pinned = [(K.PinnedSlot(max(n, 64)), torch.cuda.Event()) for _ in range(self.RING)]
         slot, ready = self._pinned[self._next_pinned % self.RING]
         self._next_pinned += 1
         return TokenFetch(tokens, self._copy_stream, slot, ready)
