@@ -1829,3 +1829,15 @@ extern "C" int mf_copy_back(void* host, const void* dev, long long bytes, cudaEv
     if (e == cudaSuccess) e = cudaEventRecord(done, on);
     return (int)e;
 }
+
+// Waits for an event where that may happen at any time (a buffer is freed, perhaps by a garbage collection
+// while this thread or another captures a graph): a wait counts as unsafe then, is refused and ends the
+// capture, unless the thread says that it has nothing to do with it.
+extern "C" int mf_event_wait(cudaEvent_t event) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return (int)e;
+    e = cudaEventSynchronize(event);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return (int)e;
+}

@@ -134,6 +134,7 @@ def _sig_ops(lib: ctypes.CDLL) -> None:
     lib.mf_norm_terms.argtypes = [c_void_p, c_int, c_int, c_void_p]
     lib.mf_step_inputs.argtypes = [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p]
     lib.mf_copy_back.argtypes = [c_void_p, c_void_p, c_longlong] + [c_void_p] * 4
+    lib.mf_event_wait.argtypes = [c_void_p]
 
 
 def _event_handle(event: torch.cuda.Event) -> int:
@@ -147,7 +148,7 @@ def _event_handle(event: torch.cuda.Event) -> int:
 class PinnedSlot:
     """A pinned int32 buffer with the event behind the copy that last used it.  The copies below are not
     known to torch's allocator of pinned memory, which would hand the buffer out again at once: a slot
-    that goes waits for its copy first."""
+    that goes waits for its copy first (also in the middle of somebody's graph capture)."""
 
     def __init__(self, n: int):
         self.host = torch.zeros(n, dtype=torch.int32).pin_memory()
@@ -155,8 +156,9 @@ class PinnedSlot:
 
     def __del__(self):
         try:
-            self.event.synchronize()
-        except Exception:       # (no event was made, or the context is gone)
+            if self.event.cuda_event:
+                _lib("ops").mf_event_wait(self.event.cuda_event)
+        except Exception:       # (the interpreter or the context is going)
             pass
 
 

@@ -112,3 +112,29 @@ def test_a_pinned_slot_waits_for_its_copy_before_its_memory_goes_back():
     assert not event.query()
     del slot
     assert event.query()
+
+
+@pytest.mark.parametrize("thread", ["the capturing one", "another one"])
+def test_a_pinned_slot_that_goes_during_a_capture_leaves_the_capture_alone(thread):
+    """A garbage collection may free an engine while another engine's step is captured: the slot's wait for
+    its copy must not end the capture, in which such a call is refused unless it is marked."""
+    import threading
+
+    from minfer_b200.kernels import api as K
+    slots = [K.PinnedSlot(8)]
+    K.copy_back(slots[0], torch.arange(8, dtype=torch.int32, device="cuda"))
+    x = torch.zeros(4, device="cuda")
+    x.add_(1)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        x.add_(1)
+        if thread == "the capturing one":
+            slots.clear()
+        else:
+            t = threading.Thread(target=slots.clear)
+            t.start()
+            t.join()
+        x.add_(1)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [3.0] * 4
