@@ -78,6 +78,8 @@ class DeviceSampler:
         """Starts copying ``tokens`` to the host on a side stream; ``.get()`` waits for that
         copy only, not for whatever was launched after it."""
         self.engine.d2h_bytes += tokens.numel() * 4
+        # (what the native copy does not take: other integers, strided ones, ones on the host)
+        tokens = tokens.to(self.device, torch.int32).contiguous()
         # pinned buffers are made once and reused in turn (allocating pinned memory is slow and
         # synchronises with the device); a buffer comes around again after RING fetches, long
         # after its tokens were read
@@ -100,7 +102,8 @@ class TokenFetch:
     def __init__(self, tokens: torch.Tensor, copy_stream: torch.cuda.Stream, slot: K.PinnedSlot,
                  ready: torch.cuda.Event):
         self.slot = slot
-        K.copy_back(slot, tokens, ready, copy_stream)   # behind the sampling kernel
+        if tokens.numel():
+            K.copy_back(slot, tokens, ready, copy_stream)   # behind the sampling kernel
         self._keep = tokens                             # not freed before the copy has run
 
     def get(self) -> List[int]:

@@ -230,3 +230,15 @@ def test_sampling_kernel_at_a_large_vocabulary():
             want = P.sample(logits[r].double(), case["temp"], case["top_k"], case["top_p"],
                             1.0, 0.0, 0.0, [], u)
             assert got[r] == want, (case, r)
+
+
+def test_fetch_takes_any_integers():
+    """The sampler's own tokens are int32 on the device; whoever fetches others gets them too."""
+    from minfer_b200.sampling.device import DeviceSampler
+    from minfer_b200.sampling.params import SamplingParams
+    engine = _generator(make_folder("A")).engine
+    sampler = DeviceSampler(engine, SamplingParams.greedy())
+    wide = torch.arange(10, device="cuda")
+    for tokens in (wide, wide[::3], wide.int()[1::2], wide.cpu(), wide[:0], wide.int()[:0]):
+        assert sampler.fetch(tokens).get() == tokens.tolist()
+    assert sampler.sample(torch.empty(0, engine.model.plan.vocab_size, device="cuda"), [], []) == []
