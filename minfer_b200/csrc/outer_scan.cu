@@ -148,8 +148,9 @@ __device__ __forceinline__ float os_soft_cap(float z, float cap) { return cap * 
 
 // LD: lanes that share a pair of columns; ND4: float4 groups of a column a lane holds (D <= 4 LD ND4);
 // tc: tokens of a chunk; PAIRS: pairs of columns a lane has (2 c and 2 c + 1, then the same TV / PAIRS on):
-// what it reads of r, k and the decays serves them all
-template <int LD, int ND4, int MODE, int PAIRS>
+// what it reads of r, k and the decays serves them all; HOLD: the state's addresses stay in registers over
+// the walk (false: they are formed again behind it), see os_choose
+template <int LD, int ND4, int MODE, int PAIRS, bool HOLD>
 __global__ void __launch_bounds__(OS_THREADS + 32 * OS_FEED) outer_scan_kernel(OuterScanArgs a, int tc) {
     pdl_launch_dependents();
     constexpr int DP = 4 * LD * ND4;                   // padded key size
@@ -355,13 +356,16 @@ __global__ void __launch_bounds__(OS_THREADS + 32 * OS_FEED) outer_scan_kernel(O
         }
         return x;
     };
+    float *st0[PAIRS], *st1[PAIRS];                    // a column that is not there: its neighbour's, unused
 #pragma unroll
     for (int p = 0; p < PAIRS; ++p) {
-        const int c0 = column(p, 0), c1 = column(p, 1);
+        const bool live0 = column(p, 0) < n_cols, live1 = column(p, 1) < n_cols;
+        st0[p] = st + (size_t)(live0 ? column(p, 0) : 0) * D;
+        st1[p] = live1 ? st0[p] + D : st0[p];
 #pragma unroll
         for (int i = 0; i < ND4; ++i) {
-            S0[p][i] = get(st + (size_t)min(c0, n_cols - 1) * D, 4 * (l + LD * i), c0 < n_cols);
-            S1[p][i] = get(st + (size_t)min(c1, n_cols - 1) * D, 4 * (l + LD * i), c1 < n_cols);
+            S0[p][i] = get(st0[p], 4 * (l + LD * i), live0);
+            S1[p][i] = get(st1[p], 4 * (l + LD * i), live1);
         }
     }
     const size_t out_row = (size_t)a.heads * Dv;
@@ -456,16 +460,19 @@ __global__ void __launch_bounds__(OS_THREADS + 32 * OS_FEED) outer_scan_kernel(O
     };
 #pragma unroll
     for (int p = 0; p < PAIRS; ++p) {
-        const int c0 = column(p, 0), c1 = column(p, 1);
+        if (!HOLD) {
+            st0[p] = st + (size_t)column(p, 0) * D;
+            st1[p] = st0[p] + D;
+        }
 #pragma unroll
         for (int i = 0; i < ND4; ++i) {
-            if (c0 < n_cols) put(st + (size_t)c0 * D, 4 * (l + LD * i), S0[p][i]);
-            if (c1 < n_cols) put(st + (size_t)c1 * D, 4 * (l + LD * i), S1[p][i]);
+            if (column(p, 0) < n_cols) put(st0[p], 4 * (l + LD * i), S0[p][i]);
+            if (column(p, 1) < n_cols) put(st1[p], 4 * (l + LD * i), S1[p][i]);
         }
     }
 }
 
-template <int LD, int ND4, int MODE, int PAIRS = 1>
+template <int LD, int ND4, int MODE, int PAIRS, bool HOLD>
 static int os_launch(const OuterScanArgs& a, int max_tokens, cudaStream_t stream) {
     constexpr int DP = 4 * LD * ND4, TV = PAIRS * 2 * (OS_THREADS / LD), NVEC = OuterTraits<MODE>::DECAYS ? 3 : 2;
     // (short rows take shorter chunks, so that more blocks fit an SM: single tokens most of all)
@@ -475,14 +482,14 @@ static int os_launch(const OuterScanArgs& a, int max_tokens, cudaStream_t stream
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MF_ERR_UNSUPPORTED;
     if (!configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(outer_scan_kernel<LD, ND4, MODE, PAIRS>,
+        cudaError_t e = cudaFuncSetAttribute(outer_scan_kernel<LD, ND4, MODE, PAIRS, HOLD>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(OS_TC));
         if (e != cudaSuccess) return (int)e;
         configured[dev] = true;
     }
     const int cols = OuterTraits<MODE>::GATES ? a.Dv + 1 : a.Dv;
     const int tiles = (cols + TV - 1) / TV;
-    mf_launch(outer_scan_kernel<LD, ND4, MODE, PAIRS>, dim3(a.heads * tiles, a.n_rows), dim3(OS_THREADS + 32 * OS_FEED), bytes(tc),
+    mf_launch(outer_scan_kernel<LD, ND4, MODE, PAIRS, HOLD>, dim3(a.heads * tiles, a.n_rows), dim3(OS_THREADS + 32 * OS_FEED), bytes(tc),
               stream, a, tc);
     return MF_LAUNCH_CHECK();
 }
@@ -492,20 +499,30 @@ static int os_choose(const OuterScanArgs& a, int max_tokens, cudaStream_t stream
     if (a.n_rows <= 0) return 0;
     if (a.D < 1 || a.D > OS_MAX_D || a.Dv < 1 || a.heads < 1 || a.n_rows > 65535) return MF_ERR_UNSUPPORTED;
     if (((uintptr_t)a.state & 15) != 0) return MF_ERR_UNSUPPORTED;
-    // Prompts that give every SM the two blocks it has room for also with four columns a lane take them:
-    // a lane then reads 3 float4 from shared memory for 48 multiply-adds instead of 24.  GLA_MEASURED
     // Prompts that fill the GPU's room (two blocks an SM) also with four columns a lane take them: a lane then
     // reads 3 float4 from shared memory for 48 multiply-adds instead of 24.  Eight prompts of 601 to 1,300
     // tokens, 8 heads of 128 x 256: 603 -> 452 us.  (The other recurrences: not measured, left as they are.)
     if constexpr (MODE == OS_GLA) {
         if (a.D > 32 && a.D <= 128 && max_tokens >= 4 * OS_TC &&
             (long long)a.n_rows * a.heads * ((a.Dv + 31) / 32) >= 2LL * mf_sm_count())
-            return a.D <= 64 ? os_launch<16, 1, MODE, 2>(a, max_tokens, stream) : os_launch<16, 2, MODE, 2>(a, max_tokens, stream);
+            return a.D <= 64 ? os_launch<16, 1, MODE, 2, false>(a, max_tokens, stream)
+                             : os_launch<16, 2, MODE, 2, false>(a, max_tokens, stream);
     }
-    if (a.D <= 32) return os_launch<8, 1, MODE>(a, max_tokens, stream);
-    if (a.D <= 64) return os_launch<16, 1, MODE>(a, max_tokens, stream);
-    if (a.D <= 128) return os_launch<16, 2, MODE>(a, max_tokens, stream);
-    return os_launch<32, 2, MODE>(a, max_tokens, stream);
+    // HOLD changes no operation, only how many registers the walk has left and how many blocks an SM takes.
+    // Rows of few tokens are bound by the state they read and write, long ones by the walk; us, held against
+    // formed again, 64 rows of one token and one row of 2,048:
+    //     D 32 (64 heads of 32 columns)    wkv 20.8 [21.9], 171.6 [172.5]    gla 19.3 [20.4], 169 [157]
+    //     D 128 (16 heads of 128)          wkv 68.4 [68.8], 334 [337]        gla 54.5 [41.3], 283 [288]
+    //     D 100 (16 heads of 70)           gla 46.5 [35.2], 236 [264]        mlstm at D 128 60.6 [62.0]
+    const bool brief = max_tokens >= 1 && max_tokens < OS_TC;
+    if (a.D <= 32)
+        return brief || MODE == OS_MLSTM ? os_launch<8, 1, MODE, 1, true>(a, max_tokens, stream)
+                                         : os_launch<8, 1, MODE, 1, false>(a, max_tokens, stream);
+    if (a.D <= 64) return os_launch<16, 1, MODE, 1, false>(a, max_tokens, stream);
+    if (a.D <= 128)
+        return brief && MODE == OS_GLA ? os_launch<16, 2, MODE, 1, false>(a, max_tokens, stream)
+                                       : os_launch<16, 2, MODE, 1, true>(a, max_tokens, stream);
+    return os_launch<32, 2, MODE, 1, false>(a, max_tokens, stream);
 }
 
 // max_tokens: the most tokens a row brings (0: not known; it only sizes the chunks)
