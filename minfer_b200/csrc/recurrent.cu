@@ -299,8 +299,10 @@ __device__ __forceinline__ void rc_walk(float (&S)[CPT][NREG], const float* xs, 
     }
 }
 
-template <int NREG, bool VEC, int NS, int CPT>
-__global__ void __launch_bounds__(RC_PB * NS) ssm_scan_kernel(ScanArgs a) {
+// BRIEF: for rows of few tokens, which are bound by the state they read and write and so by the blocks an SM
+// takes: the state's address is formed again behind the walk and does not cost it registers.
+template <int NREG, bool VEC, int NS, int CPT, bool BRIEF = false>
+__global__ void __launch_bounds__(RC_PB * NS, BRIEF && NREG == 4 ? 5 : 0) ssm_scan_kernel(ScanArgs a) {
     // (the kernel behind this one is let in only after the walk, further down: a block here runs
     // for as long as its row is, and blocks of the next kernel that wait beside it on the same SM
     // slowed it down: a prompt of 2,048 tokens through six layer runs 3.54 ms against 2.89 ms
@@ -420,6 +422,7 @@ __global__ void __launch_bounds__(RC_PB * NS) ssm_scan_kernel(ScanArgs a) {
 #pragma unroll
     for (int c = 0; c < CPT; ++c) {
         if (pl + RC_PB * c >= n_p) continue;
+        if (BRIEF && NREG > 4) st[c] = a.state + (((size_t)slot * a.heads + h) * P + p + RC_PB * c) * N;
         if (VEC) {
 #pragma unroll
             for (int j = 0; j < NREG / 4; ++j) {
@@ -487,12 +490,13 @@ extern "C" int mf_ssm_scan(const float* u, const float* proj, long long in_width
         const size_t pad = most / (size_t)(share + 1) + 1024;
         if (pad > smem && pad <= most - 1024) smem = pad;
     }
+    const bool brief = (long long)n_tokens < 16LL * n_rows && N <= RC_NS * 16;
     const int nreg = vec ? 4 * ((N / 4 + ns - 1) / ns) : (N + ns - 1) / ns;
-#define MF_SCAN(NR, V, S_, C_) \
+#define MF_SCAN(...) \
     do { \
         if (smem > 48 * 1024) \
-            cudaFuncSetAttribute(ssm_scan_kernel<NR, V, S_, C_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        mf_launch(ssm_scan_kernel<NR, V, S_, C_>, grid, block, smem, stream, a); \
+            cudaFuncSetAttribute(ssm_scan_kernel<__VA_ARGS__>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        mf_launch(ssm_scan_kernel<__VA_ARGS__>, grid, block, smem, stream, a); \
     } while (0)
     if (vec && ns == 16) {
         if (nreg <= 8) MF_SCAN(8, true, 16, 1);
@@ -502,6 +506,10 @@ extern "C" int mf_ssm_scan(const float* u, const float* proj, long long in_width
         else if (nreg <= 8) MF_SCAN(8, true, 8, 2);
         else if (nreg <= 16) MF_SCAN(16, true, 8, 2);
         else MF_SCAN(32, true, 8, 2);
+    } else if (vec && brief) {
+        if (nreg <= 4) MF_SCAN(4, true, 8, 1, true);
+        else if (nreg <= 8) MF_SCAN(8, true, 8, 1, true);
+        else MF_SCAN(16, true, 8, 1, true);
     } else if (vec) {
         if (nreg <= 4) MF_SCAN(4, true, 8, 1);
         else if (nreg <= 8) MF_SCAN(8, true, 8, 1);
