@@ -439,11 +439,32 @@ __global__ void __launch_bounds__(RC_PB * NS, BRIEF && NREG == 4 ? 5 : 0) ssm_sc
     }
 }
 
+// Columns of a thread (1 or 2).  With one, a thread reads 8 float4 of B and C from shared memory for 48
+// multiply-adds, and with blocks enough the shared memory is what the kernel waits for; with two the same
+// reads serve 96.  But a token's chain is longer with two, and a block runs for as long as its row is.  So
+// two only where the rows are long (a step of few tokens is bound by the state) and together make as many
+// blocks of the longest row's length as there are SMs; twice as many for state sizes that gain little
+// (up to 64 numbers, whose chains weigh more, and 129 to 208, whose last registers are empty), half as
+// many again where half of a head's last block would be padding, which those sizes never pay for.
+// max_tokens: the longest row, 0 if not known.
+// us, one -> two (not taken in brackets): eight prompts of 601 to 1,300 tokens, 64 heads of 64 columns, state
+// 128, 1,422 -> 1,041, of 96 columns 2,021 -> 1,757, of 80 columns and state 200 [3,009 -> 3,568]; 24 heads of
+// 64 columns and state 64 [392 -> 452]; 400 tokens beside seven rows of 3, 24 heads of 64, state 128
+// [119 -> 167].  Of 998 mixes of rows, heads and sizes 353 take two; two of them are 4 % slower, none more.
+extern "C" int mf_ssm_scan_columns(int n_tokens, int n_rows, int max_tokens, int heads, int P, int N, int sms) {
+    const int half = (P + RC_PB - 1) / RC_PB, whole = (P + 2 * RC_PB - 1) / (2 * RC_PB);
+    const bool gains = (N > 64 && N <= 128) || N > 208, padded = 2 * whole > half;
+    if (n_rows <= 0 || P <= RC_PB || (long long)n_tokens < 16LL * n_rows || (padded && !gains)) return 1;
+    const long long longest = max_tokens > 0 ? max_tokens : n_tokens - (n_rows - 1);
+    const long long blocks = (long long)n_tokens * heads * whole;          // times the longest row
+    return 2 * blocks >= (gains ? (padded ? 3 : 2) : 4) * longest * sms ? 2 : 1;
+}
+
 extern "C" int mf_ssm_scan(const float* u, const float* proj, long long in_width, int dt_off,
                            int channels, const float* dt_bias, const float* a_log,
                            const float* d_skip, float* state, const int* cu_seqlens,
-                           const int* slots, float* y, int n_tokens, int n_rows, int heads, int P,
-                           int N, int groups, cudaStream_t stream) {
+                           const int* slots, float* y, int n_tokens, int n_rows, int max_tokens,
+                           int heads, int P, int N, int groups, cudaStream_t stream) {
     if (n_rows <= 0 || n_tokens <= 0) return 0;
     if (heads < 1 || P < 1 || N < 1 || N > RC_NS * 32) return MF_ERR_UNSUPPORTED;
     if (groups < 1 || heads % groups != 0) return MF_ERR_ARGUMENT;
@@ -468,13 +489,7 @@ extern "C" int mf_ssm_scan(const float* u, const float* proj, long long in_width
     const long long n_blocks = (long long)n_rows * heads * ((P + RC_PB - 1) / RC_PB);
     int ns = (vec && N >= 128 && (long long)n_tokens >= 64LL * n_rows && n_blocks <= mf_sm_count()) ? 16 : RC_NS;
     if (vec && N >= 64 && (forced == 8 || forced == 16)) ns = forced;
-    // Columns of a thread: two for prompts.  With one, a thread reads 8 float4 of B and C from shared
-    // memory for 48 multiply-adds and the shared memory is what the kernel waits for; with two the same
-    // reads serve 96.  Not where that leaves SMs without a block, nor for a step of few tokens, which is
-    // bound by the state it reads and writes.  Eight prompts of 601 to 1,300 tokens, 64 heads of 64
-    // columns, state 128, one column a thread -> two: 1.43 -> 1.06 ms.
-    const bool two = vec && ns == RC_NS && P > RC_PB && (long long)n_tokens >= 16LL * n_rows &&
-                     (long long)n_rows * heads * ((P + 2 * RC_PB - 1) / (2 * RC_PB)) >= mf_sm_count();
+    const bool two = vec && ns == RC_NS && mf_ssm_scan_columns(n_tokens, n_rows, max_tokens, heads, P, N, mf_sm_count()) == 2;
     const int cols = two ? 2 * RC_PB : RC_PB;
     dim3 grid(n_rows, heads, (P + cols - 1) / cols), block(((pb * ns + 31) / 32) * 32);
     size_t smem = (size_t)(2 * RC_TC * (cols + 2 * N + 2)) * sizeof(float);

@@ -291,7 +291,8 @@ def _sig_recurrent(lib: ctypes.CDLL) -> None:
                                  [c_int, c_int, c_int, c_int, c_void_p])
     lib.mf_conv_state.argtypes = [c_void_p, c_longlong, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p]
     lib.mf_ssm_scan.argtypes = ([c_void_p, c_void_p, c_longlong, c_int, c_int] + [c_void_p] * 7 +
-                                [c_int] * 6 + [c_void_p])
+                                [c_int] * 7 + [c_void_p])
+    lib.mf_ssm_scan_columns.argtypes = [c_int] * 7
     lib.mf_gated_group_norm.argtypes = [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p,
                                         c_int, c_int, c_int, c_int, c_float, c_void_p]
     lib.mf_selective_scan.argtypes = [c_void_p, c_int, c_void_p]
@@ -1006,11 +1007,12 @@ def conv_silu(proj: torch.Tensor, x_off: int, channels: int, weight: torch.Tenso
 def ssm_scan(u: torch.Tensor, proj: torch.Tensor, dt_off: int, dt_bias: torch.Tensor,
              a_log: torch.Tensor, d_skip: torch.Tensor, state: torch.Tensor,
              cu_seqlens: torch.Tensor, slots: torch.Tensor, y: torch.Tensor, n_rows: int,
-             heads: int, head_dim: int, n_state: int, groups: int) -> None:
+             heads: int, head_dim: int, n_state: int, groups: int, max_tokens: int = 0) -> None:
     """The selective recurrence per (row, head), tokens one after another:
     dt = softplus(proj[t][dt_off + h] + dt_bias[h]); S <- exp(-exp(a_log[h]) dt) S + dt B x^T;
     y = S^T C + d_skip[h] x, with x | B | C the columns of ``u`` (float32 [tokens, channels]) and
-    S float32 in ``state`` [slots, heads, head_dim, n_state]."""
+    S float32 in ``state`` [slots, heads, head_dim, n_state].  ``max_tokens``: the most tokens a row brings
+    (0: not known)."""
     n = u.shape[0]
     inner = heads * head_dim
     if (u.shape[1] != inner + 2 * groups * n_state or y.shape != (n, inner)
@@ -1019,8 +1021,8 @@ def ssm_scan(u: torch.Tensor, proj: torch.Tensor, dt_off: int, dt_bias: torch.Te
     _check(_lib("recurrent").mf_ssm_scan(
         _f32(u, "u"), _f32(proj, "proj"), proj.shape[1], int(dt_off), u.shape[1],
         _f32(dt_bias, "dt_bias"), _f32(a_log, "a_log"), _f32(d_skip, "d_skip"), _f32(state, "state"),
-        _i32(cu_seqlens, "cu_seqlens"), _i32(slots, "slots"), _f32(y, "y"), n, int(n_rows), heads,
-        head_dim, n_state, groups, _stream()), "ssm_scan")
+        _i32(cu_seqlens, "cu_seqlens"), _i32(slots, "slots"), _f32(y, "y"), n, int(n_rows),
+        int(max_tokens), heads, head_dim, n_state, groups, _stream()), "ssm_scan")
 
 
 def gated_group_norm(y: torch.Tensor, proj: torch.Tensor, z_off: int, weight: torch.Tensor,

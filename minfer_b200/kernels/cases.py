@@ -468,7 +468,7 @@ def _ssm_inputs(n, rows, heads=64, head_dim=64, n_state=128):
     cu = torch.arange(rows + 1, dtype=torch.int32, device="cuda") * (n // rows)
     slots = torch.arange(rows, dtype=torch.int32, device="cuda")
     return (lambda: K.ssm_scan(u, proj, inner + ch, z, z, z, state, cu, slots, y, rows, heads, head_dim,
-                               n_state, 1)), n * (ch + inner + heads) * 4 + rows * heads * head_dim * n_state * 8
+                               n_state, 1, max_tokens=n // rows)), n * (ch + inner + heads) * 4 + rows * heads * head_dim * n_state * 8
 
 
 def ssm_scan_prompt(reps, tokens=2048):

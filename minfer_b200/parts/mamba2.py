@@ -112,7 +112,7 @@ class Mamba2(Mixer):
         y = torch.empty((n, self.inner), dtype=torch.float32, device=dev)
         K.ssm_scan(u, proj, self.inner + self.channels, self.w["dt_bias"], self.w["A_log"],
                    self.w["D"], binding.state[SSM_STATE], ctx.cu_seqlens, ctx.slots, y, ctx.n_rows,
-                   self.n_heads, self.head_dim, self.n_state, self.groups)
+                   self.n_heads, self.head_dim, self.n_state, self.groups, max_tokens=ctx.max_row_tokens)
         gated = torch.empty((n, self.inner), dtype=ctx.act_dtype, device=dev)
         K.gated_group_norm(y, proj, 0, self.w["norm"], gated, self.norm_groups, self.norm_eps)
         project_out(self.out, gated, ctx, residual)

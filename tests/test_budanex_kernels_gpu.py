@@ -280,24 +280,27 @@ def test_state_space_kernels_over_cuts(sizes, cuts):
     assert float(ssm[1].min()) == 7.0 and float(ssm[2].abs().max()) == 0.0
 
 
-@pytest.mark.parametrize("P_, N", [(33, 64), (40, 12), (64, 128), (64, 32), (65, 200), (100, 256), (128, 16)])
+@pytest.mark.parametrize("P_, N", [(33, 64), (40, 12), (64, 128), (64, 32), (65, 200), (65, 100), (100, 256), (128, 16)])
 def test_state_space_scan_of_long_rows_gives_the_bits_of_short_pieces(P_, N):
     """Long rows on a grid that fills the GPU give a thread two columns, pieces of a few tokens one; a
     column's operations are the same in both, so the outputs and states are too."""
     from minfer_b200.kernels import api as K
-    heads, groups = 80, 2
+    heads, groups = 120, 2
     inner = heads * P_
     ch = inner + 2 * groups * N
-    lens = [131, 64, 40]
+    lens = [131, 120, 110]
     n = sum(lens)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert K._lib("recurrent").mf_ssm_scan_columns(n, 3, 131, heads, P_, N, sms) == (1 if (P_, N) == (65, 200) else 2)
     g = torch.Generator().manual_seed(P_ * 1000 + N)
     rnd = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
     u, proj, state0 = rnd(n, ch), rnd(n, heads + 4), rnd(4, heads, P_, N)
     dt_bias, a_log, d = rnd(heads), rnd(heads) * 0.3, rnd(heads)
     slots = torch.tensor([2, 0, 3], dtype=torch.int32, device=DEV)
-    cu = torch.tensor([0, 131, 195, 235], dtype=torch.int32, device=DEV)
+    cu = torch.tensor([0, 131, 251, 361], dtype=torch.int32, device=DEV)
     whole, y = state0.clone(), torch.empty((n, inner), device=DEV)
-    K.ssm_scan(u, proj, 4, dt_bias, a_log, d, whole, cu, slots, y, 3, heads, P_, N, groups)
+    K.ssm_scan(u, proj, 4, dt_bias, a_log, d, whole, cu, slots, y, 3, heads, P_, N, groups,
+               max_tokens=max(lens))
     pieces, want = state0.clone(), torch.empty((n, inner), device=DEV)
     for b in range(3):
         lo = int(cu[b])

@@ -1,0 +1,33 @@
+"""Which kernel a call takes: host functions of sizes, each with the sizes that were measured on either side
+of its line (148 SMs, no GPU)."""
+import pytest
+
+from minfer_b200.kernels import api as K
+
+SMS = 148
+EIGHT = [601, 700, 800, 900, 1000, 1100, 1200, 1300]
+
+
+@pytest.mark.parametrize("lens,heads,P,N,columns", [
+    (EIGHT, 64, 64, 128, 2),
+    (EIGHT, 32, 128, 128, 2),
+    ([17] * 16, 64, 64, 128, 2),
+    ([15] * 16, 64, 64, 128, 1),            # few tokens a row
+    ([1] * 64, 64, 64, 128, 1),
+    ([3] * 7 + [400], 64, 64, 128, 1),      # one long row: its chain is what counts
+    ([3] * 7 + [400], 128, 64, 128, 1),
+    (EIGHT, 24, 64, 64, 1),                 # small states want more blocks
+    (EIGHT, 64, 64, 64, 2),
+    (EIGHT, 64, 80, 200, 1),                # half a block of padding
+    (EIGHT, 64, 96, 128, 2),                # the same where two columns gain more
+    ([500] * 3, 35, 96, 128, 1),            # fewer blocks than that takes
+    (EIGHT, 64, 96, 64, 1),
+    (EIGHT, 64, 33, 128, 2),
+    (EIGHT, 64, 32, 128, 1),
+    ([5000], 64, 64, 128, 1),
+])
+def test_columns_of_a_thread_of_the_state_space_scan(lens, heads, P, N, columns):
+    choose = K._lib("recurrent").mf_ssm_scan_columns
+    assert choose(sum(lens), len(lens), max(lens), heads, P, N, SMS) == columns
+    # without the longest row's length it is taken to be as long as it can be
+    assert choose(sum(lens), len(lens), 0, heads, P, N, SMS) <= columns
