@@ -494,17 +494,29 @@ static int os_launch(const OuterScanArgs& a, int max_tokens, cudaStream_t stream
     return MF_LAUNCH_CHECK();
 }
 
+// Columns of a lane of gated linear attention over keys of 33 to 128 (2 or 4).  With four a lane reads 3
+// float4 from shared memory for 48 multiply-adds instead of 24, but a token's chain is longer, and a block
+// runs for as long as its row is.  So four only where the rows are long and together make one and a half
+// blocks of the longest row's length for every SM; two and a half where half of a head's last block would
+// be padding, which keys of up to 64 never pay for.  max_tokens: the longest row, 0 if not known.
+// us, two -> four (not taken in brackets): eight prompts of 601 to 1,300 tokens, 8 heads of 128 x 256,
+// 603 -> 452; 400 tokens beside seven rows of 3 [79 -> 97]; three rows of 300 [86 -> 102]; 60 heads of 36 x 40
+// [501 -> 549].  Of 488 mixes of rows, heads and sizes 85 take four, none of them is slower; by the count of rows
+// 127 did, of which 30 were, up to 1.28 times.  (The other recurrences: not measured, they keep two.)
+extern "C" int mf_gla_scan_columns(int n_tokens, int max_tokens, int heads, int D, int Dv, int sms) {
+    const int half = (Dv + 15) / 16, whole = (Dv + 31) / 32;
+    const bool padded = 2 * whole > half;
+    if (D <= 32 || D > 128 || max_tokens < 4 * OS_TC || (padded && D <= 64)) return 2;
+    return 2LL * n_tokens * heads * whole >= (padded ? 5LL : 3LL) * max_tokens * sms ? 4 : 2;
+}
+
 template <int MODE>
-static int os_choose(const OuterScanArgs& a, int max_tokens, cudaStream_t stream) {
+static int os_choose(const OuterScanArgs& a, int max_tokens, int n_tokens, cudaStream_t stream) {
     if (a.n_rows <= 0) return 0;
     if (a.D < 1 || a.D > OS_MAX_D || a.Dv < 1 || a.heads < 1 || a.n_rows > 65535) return MF_ERR_UNSUPPORTED;
     if (((uintptr_t)a.state & 15) != 0) return MF_ERR_UNSUPPORTED;
-    // Prompts that fill the GPU's room (two blocks an SM) also with four columns a lane take them: a lane then
-    // reads 3 float4 from shared memory for 48 multiply-adds instead of 24.  Eight prompts of 601 to 1,300
-    // tokens, 8 heads of 128 x 256: 603 -> 452 us.  (The other recurrences: not measured, left as they are.)
     if constexpr (MODE == OS_GLA) {
-        if (a.D > 32 && a.D <= 128 && max_tokens >= 4 * OS_TC &&
-            (long long)a.n_rows * a.heads * ((a.Dv + 31) / 32) >= 2LL * mf_sm_count())
+        if (mf_gla_scan_columns(n_tokens, max_tokens, a.heads, a.D, a.Dv, mf_sm_count()) == 4)
             return a.D <= 64 ? os_launch<16, 1, MODE, 2, false>(a, max_tokens, stream)
                              : os_launch<16, 2, MODE, 2, false>(a, max_tokens, stream);
     }
@@ -527,14 +539,14 @@ static int os_choose(const OuterScanArgs& a, int max_tokens, cudaStream_t stream
 
 // max_tokens: the most tokens a row brings (0: not known; it only sizes the chunks)
 extern "C" int mf_wkv_scan(const OuterScanArgs* args, int max_tokens, cudaStream_t stream) {
-    return os_choose<OS_WKV>(*args, max_tokens, stream);
+    return os_choose<OS_WKV>(*args, max_tokens, 0, stream);
 }
 extern "C" int mf_mlstm_scan(const OuterScanArgs* args, int max_tokens, cudaStream_t stream) {
     if (!(args->cap > 0.0f)) return MF_ERR_ARGUMENT;
-    return os_choose<OS_MLSTM>(*args, max_tokens, stream);
+    return os_choose<OS_MLSTM>(*args, max_tokens, 0, stream);
 }
-extern "C" int mf_gla_scan(const OuterScanArgs* args, int max_tokens, cudaStream_t stream) {
-    return os_choose<OS_GLA>(*args, max_tokens, stream);
+extern "C" int mf_gla_scan(const OuterScanArgs* args, int max_tokens, int n_tokens, cudaStream_t stream) {
+    return os_choose<OS_GLA>(*args, max_tokens, n_tokens, stream);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -308,7 +308,8 @@ def _sig_retention(lib: ctypes.CDLL) -> None:
 def _sig_outer_scan(lib: ctypes.CDLL) -> None:
     lib.mf_wkv_scan.argtypes = [c_void_p, c_int, c_void_p]
     lib.mf_mlstm_scan.argtypes = [c_void_p, c_int, c_void_p]
-    lib.mf_gla_scan.argtypes = [c_void_p, c_int, c_void_p]
+    lib.mf_gla_scan.argtypes = [c_void_p, c_int, c_int, c_void_p]
+    lib.mf_gla_scan_columns.argtypes = [c_int] * 6
     lib.mf_sigmoid_decay.argtypes = [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                      c_int, c_float, c_void_p]
     lib.mf_wkv_decay.argtypes = [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int,
@@ -1888,7 +1889,7 @@ def gla_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, decay: torc
     a.cu_seqlens, a.slots, a.out = _i32(cu_seqlens, "cu_seqlens"), _i32(slots, "slots"), _f32(out, "out")
     a.n_rows, a.heads, a.D, a.Dv = int(n_rows), heads, d, dv
     a.r_scale = float(q_scale)
-    _check(_lib("outer_scan").mf_gla_scan(ctypes.addressof(a), int(max_tokens), _stream()), "gla_scan")
+    _check(_lib("outer_scan").mf_gla_scan(ctypes.addressof(a), int(max_tokens), n, _stream()), "gla_scan")
 
 
 def mlstm_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, i_off: int, f_off: int,

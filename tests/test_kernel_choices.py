@@ -31,3 +31,22 @@ def test_columns_of_a_thread_of_the_state_space_scan(lens, heads, P, N, columns)
     assert choose(sum(lens), len(lens), max(lens), heads, P, N, SMS) == columns
     # without the longest row's length it is taken to be as long as it can be
     assert choose(sum(lens), len(lens), 0, heads, P, N, SMS) <= columns
+
+
+@pytest.mark.parametrize("lens,heads,D,Dv,columns", [
+    (EIGHT, 8, 128, 256, 4),
+    ([100] * 40, 8, 100, 250, 4),
+    ([300] * 5, 8, 128, 256, 4),
+    ([300] * 3, 8, 128, 256, 2),            # fewer blocks than one and a half an SM
+    ([3] * 7 + [400], 8, 128, 256, 2),      # one long row: its chain is what counts
+    ([63] * 8, 32, 128, 128, 2),            # few tokens a row
+    (EIGHT, 60, 36, 40, 2),                 # half a block of padding, short keys
+    (EIGHT, 60, 128, 33, 4),
+    (EIGHT, 19, 128, 33, 2),
+    (EIGHT, 40, 32, 64, 2),
+    (EIGHT, 40, 129, 64, 2),
+])
+def test_columns_of_a_lane_of_gated_linear_attention(lens, heads, D, Dv, columns):
+    choose = K._lib("outer_scan").mf_gla_scan_columns
+    assert choose(sum(lens), max(lens), heads, D, Dv, SMS) == columns
+    assert choose(sum(lens), 0, heads, D, Dv, SMS) == 2

@@ -88,13 +88,16 @@ def test_gla_scan_over_cuts_and_slots(H, D, Dv, known, off):
     assert torch.equal(state[[1, 3, 5]], stale)
 
 
-@pytest.mark.parametrize("D,Dv", [(33, 33), (64, 64), (100, 65), (128, 250), (128, 256), (36, 40)])
+@pytest.mark.parametrize("D,Dv", [(33, 33), (33, 32), (48, 50), (64, 64), (100, 65), (128, 250), (128, 256), (36, 40)])
 def test_gla_scan_of_long_rows_gives_the_bits_of_short_pieces(D, Dv):
     """Long rows on a grid that fills the GPU give a lane four columns, pieces two; a column's operations
     are the same in both, so outputs and states are too."""
     from minfer_b200.kernels import api as K
-    H, lens, slots = 60, [131, 64, 40], [4, 0, 2]
+    H, lens, slots = 100, [131, 120, 110], [4, 0, 2]
     n, width = sum(lens), H * (2 * D + Dv)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    four = K._lib("outer_scan").mf_gla_scan_columns(n, max(lens), H, D, Dv, sms) == 4
+    assert four == ((D, Dv) not in ((33, 33), (36, 40)))
     g = torch.Generator().manual_seed(D * 1000 + Dv)
     proj = torch.randn(n, width, generator=g).to(DEV)
     d = (torch.sigmoid(torch.randn(n, H * D, generator=g) * 3 + 2) ** 0.25).to(DEV)
