@@ -1173,11 +1173,28 @@ static int check_sizes(int n_heads, int n_kv, int hd) {
     return 0;
 }
 
-// Attention of a step over its own packed keys and values (whole prompts).
+// Whether float32 prompts take the kernel whose CTA walks 32 rows together.  It walks the sequences among
+// its rows one after another, 3 to 6 us each with a fetch and barriers, and only the warps that own those
+// rows work: many short sequences are what it is bad at, long ones what it is for.  A warp a query takes
+// 0.24 to 0.9 us a key of the longest, 4 heads of 16 to 32 of 128: so the longest has to outweigh the walks a
+// CTA may have to make, or the sequences are long on average.  `longest`: its tokens, 0 if not known.
+// us, a warp a query -> 32 rows (not taken in brackets), 14 heads of 64: 32 tokens 13.4 -> 9.7, 200 83 -> 34,
+// 8 of 64 46 -> 18, 63 of 1 beside one of 1,000 1,015 -> 201, 16 of 16 [11.5 -> 16.2], 64 of 1 [4.7 -> 131]; 4
+// heads of 16: 3 of 48 [13 -> 17].  Of 712 mixes of lengths and heads 208 take it, none of them is more than 3 %
+// slower (of 342 others two are, 5 and 15 % with 4 heads of 16); by 16 rows in all every one did, and 374 were, up
+// to 31 times.
+extern "C" int mf_attention_packed_tiled(int rows, int n_seqs, int longest) {
+    if (n_seqs <= 1) return rows >= 32;
+    const int walks = n_seqs < 32 ? n_seqs : 32;
+    return longest >= (14 * walks > 64 ? 14 * walks : 64) || (long long)rows >= 56LL * n_seqs;
+}
+
+// Attention of a step over its own packed keys and values (whole prompts).  `longest`: the longest
+// sequence's tokens, 0 if not known.
 extern "C" int mf_attention_packed(const void* q, const void* k, const void* v, const int* row_seq,
                                    const int* row_pos, const int* cu_seqlens, void* out, int rows,
-                                   int n_heads, int n_kv, int hd, int window, float scale, int dtype,
-                                   cudaStream_t stream) {
+                                   int n_seqs, int longest, int n_heads, int n_kv, int hd, int window,
+                                   float scale, int dtype, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (int e = check_sizes(n_heads, n_kv, hd)) return e;
     AttnArgs a{};
@@ -1187,10 +1204,10 @@ extern "C" int mf_attention_packed(const void* q, const void* k, const void* v, 
     a.chunk = 0; a.n_chunks = 1; a.scale = scale;
     const long long items = (long long)rows * n_heads;
     const unsigned blocks = (unsigned)((items + ATT_WARPS - 1) / ATT_WARPS);
-    // float32 over all earlier keys (a window's tiles would start at another key for every row), from
-    // where 32 rows share their keys; 16 bytes at a time
-    if (dtype == MF_DTYPE_F32 && window == 0 && rows >= 16 && hd <= 128 && n_heads <= 65535 &&
-        (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0)
+    // float32 over all earlier keys (a window's tiles would start at another key for every row), 16 bytes
+    // at a time
+    if (dtype == MF_DTYPE_F32 && window == 0 && mf_attention_packed_tiled(rows, n_seqs, longest) && hd <= 128 &&
+        n_heads <= 65535 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0)
         return hd <= 32 ? launch_packed_f32<1>(a, stream) : hd <= 64 ? launch_packed_f32<2>(a, stream)
                                                                      : launch_packed_f32<4>(a, stream);
     if (dtype == MF_DTYPE_F32)

@@ -201,7 +201,8 @@ def _sig_gemm_simt(lib: ctypes.CDLL) -> None:
 
 
 def _sig_attention(lib: ctypes.CDLL) -> None:
-    lib.mf_attention_packed.argtypes = [c_void_p] * 7 + [c_int] * 5 + [c_float, c_int, c_void_p]
+    lib.mf_attention_packed.argtypes = [c_void_p] * 7 + [c_int] * 7 + [c_float, c_int, c_void_p]
+    lib.mf_attention_packed_tiled.argtypes = [c_int] * 3
     lib.mf_attention_paged.argtypes = ([c_void_p] * 6 + [c_int, c_int, c_void_p, c_void_p] +
                                        [c_int] * 7 + [c_float, c_int, c_int, c_longlong, c_void_p,
                                                       c_int, c_void_p])
@@ -886,14 +887,18 @@ def splitk_reduce(partial: torch.Tensor, bias: Optional[torch.Tensor], out: torc
 # ---------------------------------------------------------------------------------------
 def attention_packed(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, row_seq: torch.Tensor,
                      row_pos: torch.Tensor, cu_seqlens: torch.Tensor, out: torch.Tensor,
-                     n_heads: int, n_kv: int, head_dim: int, window: int, scale: float) -> None:
+                     n_heads: int, n_kv: int, head_dim: int, window: int, scale: float,
+                     longest: int = 0) -> None:
+    """Attention of whole prompts over their own packed keys; ``longest``: the longest one's tokens (0: not
+    known)."""
     rows = q.shape[0]
     if q.dtype != k.dtype or q.dtype != v.dtype or q.dtype != out.dtype:
         raise KernelError("attention: q, k, v and out must share one dtype")
     _check(_lib("attention").mf_attention_packed(
         _ptr(q, "q"), _ptr(k, "k"), _ptr(v, "v"), _i32(row_seq, "row_seq"), _i32(row_pos, "row_pos"),
-        _i32(cu_seqlens, "cu_seqlens"), _ptr(out, "out"), rows, n_heads, n_kv, head_dim,
-        int(window), float(scale), dtype_code(q.dtype), _stream()), "attention_packed")
+        _i32(cu_seqlens, "cu_seqlens"), _ptr(out, "out"), rows, cu_seqlens.numel() - 1,
+        int(longest), n_heads, n_kv, head_dim, int(window), float(scale), dtype_code(q.dtype), _stream()),
+        "attention_packed")
 
 
 def attention_prefill_supported(q: torch.Tensor, n_heads: int, n_kv: int, head_dim: int) -> bool:

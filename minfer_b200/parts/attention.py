@@ -218,7 +218,8 @@ class Attention(Mixer):
                                            ctx.status)
             else:
                 K.attention_packed(q, k_step, v_step, ctx.token_row, ctx.positions,
-                                   ctx.cu_seqlens, o, nh, nk, hd, self.window, self.scale)
+                                   ctx.cu_seqlens, o, nh, nk, hd, self.window, self.scale,
+                                   longest=ctx.max_row_tokens)
         else:
             # keys and values come from the cache, the step's own among them: each token is a
             # query at its position

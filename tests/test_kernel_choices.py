@@ -50,3 +50,19 @@ def test_columns_of_a_lane_of_gated_linear_attention(lens, heads, D, Dv, columns
     choose = K._lib("outer_scan").mf_gla_scan_columns
     assert choose(sum(lens), max(lens), heads, D, Dv, SMS) == columns
     assert choose(sum(lens), 0, heads, D, Dv, SMS) == 2
+
+
+@pytest.mark.parametrize("lens,tiled", [
+    ([16], False), ([31], False), ([32], True), ([200], True),
+    ([1] * 64, False),                      # many short sequences: a CTA would walk 32 of them in turn
+    ([2] * 32, False), ([16] * 16, False), ([48] * 3, False),
+    ([56] * 3, True), ([130, 255], True), ([64] * 8, True),
+    ([1] * 31 + [200], False),
+    ([1] * 63 + [1000], True),              # one that is worth it
+    ([40] * 2, False), ([5, 60], False), ([5, 64], True),
+    ([400] * 64, True),
+])
+def test_which_float32_prompts_walk_their_keys_by_tiles(lens, tiled):
+    choose = K._lib("attention").mf_attention_packed_tiled
+    assert bool(choose(sum(lens), len(lens), max(lens))) == tiled
+    assert choose(sum(lens), len(lens), 0) <= tiled

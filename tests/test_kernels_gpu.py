@@ -135,7 +135,8 @@ def test_float32_product_waits_for_the_kernel_that_writes_its_input(m):
 
 
 @pytest.mark.parametrize("heads,kv,hd", [(4, 1, 16), (2, 2, 32), (6, 2, 48), (14, 2, 64), (5, 5, 80), (4, 2, 128)])
-@pytest.mark.parametrize("lens", [[16], [33], [5, 1, 40, 7], [130, 255], [64, 300, 31]])
+@pytest.mark.parametrize("lens", [[16], [33], [5, 1, 40, 7], [130, 255], [64, 300, 31],
+                                  [3, 1, 2, 300, 1, 5, 17], [1] * 40 + [1030] + [2] * 5])
 def test_float32_prompt_attention_gives_the_generic_kernels_bits(heads, kv, hd, lens):
     """Tiles of 32 queries by 32 keys against a warp a query (a window beyond every position leads there):
     the same operations in the same order.  Values a row does not see take no part, whatever they hold."""
@@ -148,7 +149,7 @@ def test_float32_prompt_attention_gives_the_generic_kernels_bits(heads, kv, hd, 
     pos = torch.tensor([i for c in lens for i in range(c)], dtype=torch.int32).cuda()
     cu = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32).cuda()
     got, want = torch.zeros(n, heads * hd, device="cuda"), torch.zeros(n, heads * hd, device="cuda")
-    K.attention_packed(q, k, v, row, pos, cu, got, heads, kv, hd, 0, hd ** -0.5)
+    K.attention_packed(q, k, v, row, pos, cu, got, heads, kv, hd, 0, hd ** -0.5, longest=max(lens))
     K.attention_packed(q, k, v, row, pos, cu, want, heads, kv, hd, 1 << 20, hd ** -0.5)
     assert torch.equal(got.nan_to_num(1e9), want.nan_to_num(1e9))
     assert got[:lens[0] - 1].isfinite().all()
