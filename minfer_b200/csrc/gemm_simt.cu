@@ -90,10 +90,10 @@ gemm_simt_kernel(const TA* A, const TW* __restrict__ W, const float* __restrict_
 // issue).  Tiles lie in shared memory by k (a warp reads 4 rows x 8 column groups), the columns of a
 // k swizzled by its quarter so that the transposing stores do not conflict; the next tile's loads are
 // in flight in registers while this one is multiplied.
-// Measured (us, the 64 x 64 x 16 kernel above in brackets): 385 x 9,728 x 896 194 [387],
-// 385 x 896 x 4,864 228 [480], 64 x 896 x 4,864 95 [469], 385 x 151,936 x 896 2,630 [5,617],
-// 1,600 x 8,448 x 2,048 1,080 [2,505] = 51 TFLOP/s of the pipe's 74.  Plain multiply-adds instead of
-// packed ones: 2 to 7 % slower.  AHEAD 2 (loads two tiles ahead) for the smallest tile, whose product of
+// Measured (us back to back, the tile that is chosen and the 64 x 64 x 16 kernel above in brackets):
+// 385 x 9,728 x 896 192 (64 x 64) [387], 385 x 896 x 4,864 216 (32 x 64) [480], 64 x 896 x 4,864 93 (32 x 64)
+// [469], 385 x 151,936 x 896 2,546 (128 x 128) [5,617], 1,600 x 8,448 x 2,048 1,080 (128 x 128) [2,505] = 51
+// TFLOP/s of the pipe's 74.  Plain multiply-adds instead of packed ones: 2 to 7 % slower.  AHEAD 2 (loads two tiles ahead) for the smallest tile, whose product of
 // a tile is shorter than a trip to memory: 64 x 896 x 4,864 129 -> 95; for 64 x 64 it lost (240 -> 280).
 __device__ __forceinline__ unsigned long long f32x2(float lo, float hi) {
     unsigned long long r;
@@ -348,6 +348,31 @@ static void launch_f32_tile(const float* A, const float* W, const float* bias, f
               dim3(F32Tile<BM_, BN_, TM, TN>::THREADS), 0, stream, A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate);
 }
 
+// The tile of a float32 product of more than 16 rows (an index into `tiles`; -1: the general kernel, whose
+// grid takes more columns): the one whose fullest SM is done first.  `shared`: what a CTA takes of a full
+// SM.  `few`: what the product takes when its CTAs are few: launched while the kernel before still runs, they
+// pile up on the SMs that are free, as many as one takes (2, 4 and 3 of these tiles).  Both in units of the
+// 64 x 64 tile's share, 27 us a thousand k, fitted to 255 products of 17 to 4,096 rows behind a norm, each
+// timed with every tile: the choice is within 0.1 % of the best tile on average (13 % at worst), and within
+// 1.1 % (21 %) of 109 products back to back; 66 others 0.2 % (6 %) and 0.6 % (24 %).  us, 128 x 128 / 64 x 64 /
+// 32 x 64, norm and product: 200 x 4,096 x 2,048 373 / 224 / 136, 385 x 9,728 x 896 241 / 194 / 205,
+// 385 x 896 x 4,864 467 / 276 / 242, 1,600 x 8,448 x 2,048 1,086 / 1,243 / 1,471.
+extern "C" int mf_gemm_f32_tile(int M, int N, int sms) {
+    static const struct { int bm, bn; double few, shared; } tiles[] = {
+        {128, 128, 6.4, 3.3}, {64, 64, 3.9, 1.0}, {32, 64, 1.8, 0.58}};
+    int best = -1;
+    double least = 0.0;
+    for (int i = 0; i < 3; ++i) {
+        const long long nt = ((long long)N + tiles[i].bn - 1) / tiles[i].bn;
+        const long long mt = ((long long)M + tiles[i].bm - 1) / tiles[i].bm;
+        if (nt > 65535) continue;                                    // the grid's second dimension
+        const double share = (double)((nt * mt + sms - 1) / sms) * tiles[i].shared;
+        const double cost = share > tiles[i].few ? share : tiles[i].few;
+        if (best < 0 || cost < least) { best = i; least = cost; }
+    }
+    return best;
+}
+
 // Float32 operands whose rows start on 16 bytes; false: the general kernel has to run.
 static bool launch_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
                        long long lda, long long ldw, long long ldc, int accumulate, cudaStream_t stream) {
@@ -363,22 +388,7 @@ static bool launch_f32(const float* A, const float* W, const float* bias, float*
 #undef MF_FEW
         return true;
     }
-    // The tile whose fullest SM is done first.  A CTA alone on its SM waits for its own loads and barriers
-    // (`alone`); with others beside it, it takes its share of the pipe (`shared`).  Both measured, in units
-    // of the 64 x 64 tile's share: 28 us a thousand k.
-    static const struct { int bm, bn; double alone, shared; } tiles[] = {
-        {128, 128, 4.25, 3.83}, {64, 64, 1.79, 1.0}, {32, 64, 0.70, 0.61}};
-    const int sms = mf_sm_count();
-    int best = -1;
-    double least = 0.0;
-    for (int i = 0; i < 3; ++i) {
-        const long long nt = ((long long)N + tiles[i].bn - 1) / tiles[i].bn;
-        const long long mt = ((long long)M + tiles[i].bm - 1) / tiles[i].bm;
-        if (nt > 65535) continue;                                    // the grid's second dimension
-        const double share = (double)((nt * mt + sms - 1) / sms) * tiles[i].shared;
-        const double cost = share > tiles[i].alone ? share : tiles[i].alone;
-        if (best < 0 || cost < least) { best = i; least = cost; }
-    }
+    const int best = mf_gemm_f32_tile(M, N, mf_sm_count());
     switch (best) {
         case 0: launch_f32_tile<128, 128, 8, 8, 16, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;
         case 1: launch_f32_tile<64, 64, 4, 8, 32, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;

@@ -198,6 +198,7 @@ def _sig_gemm_simt(lib: ctypes.CDLL) -> None:
     lib.mf_gemm_simt.argtypes = [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                  c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int,
                                  c_void_p]
+    lib.mf_gemm_f32_tile.argtypes = [c_int] * 3
 
 
 def _sig_attention(lib: ctypes.CDLL) -> None:

@@ -66,3 +66,16 @@ def test_which_float32_prompts_walk_their_keys_by_tiles(lens, tiled):
     choose = K._lib("attention").mf_attention_packed_tiled
     assert bool(choose(sum(lens), len(lens), max(lens))) == tiled
     assert choose(sum(lens), len(lens), 0) <= tiled
+
+
+@pytest.mark.parametrize("m,n,tile", [
+    # (rows and columns of the products whose bits and whose wait are tested, among others)
+    (17, 31, 2), (129, 1157, 2), (385, 1152, 2), (200, 4096, 2), (385, 896, 2), (1500, 1152, 2),
+    (260, 9001, 1), (333, 9031, 1), (385, 9728, 1), (2500, 1152, 1),
+    (700, 9001, 0), (2170, 2175, 0), (4096, 1152, 0), (1600, 8448, 0), (385, 151936, 0),
+    (20, 4_000_000, 2), (20, 5_000_000, 0),         # 65,535 tiles of 64 columns end at 4,194,240
+    (20, 9_000_000, -1),
+])
+def test_tile_of_a_float32_product(m, n, tile):
+    """0: 128 x 128, 1: 64 x 64, 2: 32 x 64, -1: the general kernel."""
+    assert K._lib("gemm_simt").mf_gemm_f32_tile(m, n, SMS) == tile

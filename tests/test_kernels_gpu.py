@@ -96,7 +96,8 @@ def test_gemm_rows_do_not_depend_on_the_batch():
 
 @pytest.mark.parametrize("m,n,k", [(1, 1, 4), (3, 7, 20), (4, 256, 128), (5, 9, 132), (8, 33, 64), (9, 17, 68),
                                    (16, 65, 260), (17, 31, 36), (33, 65, 68), (65, 130, 100), (129, 1157, 20),
-                                   (200, 333, 1000), (385, 2600, 132), (1300, 3000, 36)])
+                                   (200, 333, 1000), (385, 2600, 132), (1300, 3000, 36), (260, 9001, 36),
+                                   (333, 9031, 100), (700, 9001, 100), (2170, 2175, 132)])
 def test_float32_products_of_every_size_keep_the_order_of_the_sum(m, n, k):
     """The kernels for aligned float32 operands (few rows, three tiles) give the bits of the general one,
     which rows off 16 bytes go to: the same additions in the same order."""
@@ -113,7 +114,7 @@ def test_float32_products_of_every_size_keep_the_order_of_the_sum(m, n, k):
         assert torch.equal(got, want)
 
 
-@pytest.mark.parametrize("m", [3, 12, 40, 385, 1500])
+@pytest.mark.parametrize("m", [3, 12, 40, 385, 1500, 2500, 4096])
 def test_float32_product_waits_for_the_kernel_that_writes_its_input(m):
     """Launched while a norm still writes the rows it reads (programmatic dependent launch), the product
     gives the bits it gives when launched after the norm has ended."""
