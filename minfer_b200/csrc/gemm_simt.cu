@@ -354,7 +354,7 @@ static void launch_f32_tile(const float* A, const float* W, const float* bias, f
 // pile up on the SMs that are free, as many as one takes (2, 4 and 3 of these tiles).  Both in units of the
 // 64 x 64 tile's share, 27 us a thousand k, fitted to 255 products of 17 to 4,096 rows behind a norm, each
 // timed with every tile: the choice is within 0.1 % of the best tile on average (13 % at worst), and within
-// 1.1 % (21 %) of 109 products back to back; 66 others 0.2 % (6 %) and 0.6 % (24 %).  us, 128 x 128 / 64 x 64 /
+// 1.1 % (21 %) of 109 products back to back; 66 others 0.3 % (6 %) and 0.7 % (24 %).  us, 128 x 128 / 64 x 64 /
 // 32 x 64, norm and product: 200 x 4,096 x 2,048 373 / 224 / 136, 385 x 9,728 x 896 241 / 194 / 205,
 // 385 x 896 x 4,864 467 / 276 / 242, 1,600 x 8,448 x 2,048 1,086 / 1,243 / 1,471.
 extern "C" int mf_gemm_f32_tile(int M, int N, int sms) {

@@ -433,7 +433,7 @@ class Engine:
         slot_i = entry["next"] % len(ring)
         entry["next"] += 1
         slot = ring[slot_i]
-        slot.event.synchronize()                    # the copy that last used this buffer is done
+        slot.wait()                                 # the copy that last used this buffer is done
         slot.host.numpy()[:] = flat
         K.step_inputs(entry["dev"], slot, device_tokens)
         self.h2d_bytes += slot.host.numel() * 4

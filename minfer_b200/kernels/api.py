@@ -137,27 +137,42 @@ def _sig_ops(lib: ctypes.CDLL) -> None:
     lib.mf_event_wait.argtypes = [c_void_p]
 
 
-def _event_handle(event: torch.cuda.Event) -> int:
-    """The handle of an event, made here if it has none: torch makes it at the first record, on the device
-    that is current then, and only that device's streams can record it.  So not before its first use."""
-    if not event.cuda_event:
-        event.record()
-    return event.cuda_event
-
-
 class PinnedSlot:
     """A pinned int32 buffer with the event behind the copy that last used it.  The copies below are not
     known to torch's allocator of pinned memory, which would hand the buffer out again at once: a slot
-    that goes waits for its copy first (also in the middle of somebody's graph capture)."""
+    that goes while its copy may be under way waits for it (also in the middle of somebody's graph capture).
+
+    Events get their handles at the first copy: torch makes them at the first record, on the device that is
+    current then, and only that device's streams can record them."""
 
     def __init__(self, n: int):
         self.host = torch.zeros(n, dtype=torch.int32).pin_memory()
         self.event = torch.cuda.Event()
+        self.handle = self.ready_handle = 0
+        self.ready = self.wait_native = None    # (wait_native: from a copy on until somebody has waited)
+
+    def made(self) -> int:
+        if not self.handle:
+            self.event.record()
+            self.handle = self.event.cuda_event
+        return self.handle
+
+    def made_ready(self) -> int:
+        if not self.ready_handle:
+            self.ready = torch.cuda.Event()
+            self.ready.record()
+            self.ready_handle = self.ready.cuda_event
+        return self.ready_handle
+
+    def wait(self) -> None:
+        """Returns when the copy that last used the buffer is done."""
+        self.event.synchronize()
+        self.wait_native = None
 
     def __del__(self):
         try:
-            if self.event.cuda_event:
-                _lib("ops").mf_event_wait(self.event.cuda_event)
+            if self.wait_native is not None:
+                self.wait_native(self.handle)
         except Exception:       # (the interpreter or the context is going)
             pass
 
@@ -176,22 +191,25 @@ def step_inputs(dev: torch.Tensor, slot: PinnedSlot, tokens: Optional[torch.Tens
             raise KernelError("step_inputs: more tokens than the buffer takes")
         if not tokens.is_contiguous():
             tokens = tokens.contiguous()
-    _check(_lib("ops").mf_step_inputs(_ptr(dev, "dev"), host.data_ptr(), host.numel() * 4,
-                                      _i32(tokens, "tokens"), n * 4, _event_handle(slot.event), _stream()),
-           "step_inputs", 0)
+    lib = _lib("ops")
+    args = (_ptr(dev, "dev"), host.data_ptr(), host.numel() * 4, _i32(tokens, "tokens"), n * 4,
+            slot.handle or slot.made(), _stream())
+    slot.wait_native = lib.mf_event_wait
+    _check(lib.mf_step_inputs(*args), "step_inputs", 0)
 
 
-def copy_back(slot: PinnedSlot, dev: torch.Tensor, ready: Optional[torch.cuda.Event] = None,
-              side: Optional[torch.cuda.Stream] = None) -> None:
+def copy_back(slot: PinnedSlot, dev: torch.Tensor, side: Optional[torch.cuda.Stream] = None) -> None:
     """Copies int32 ``dev`` to the first integers of the slot behind what the current stream holds, on
-    stream ``side`` if one is given (``ready`` is recorded on the current one then), and records the
-    slot's event behind the copy."""
+    stream ``side`` if one is given, and records the slot's event behind the copy."""
     n = dev.numel()
     if n < 1 or n > slot.host.numel():
         raise KernelError("copy_back: the buffer is too small")
-    _check(_lib("ops").mf_copy_back(
-        slot.host.data_ptr(), _i32(dev, "dev"), n * 4, _event_handle(ready) if ready is not None else None,
-        _event_handle(slot.event), side.cuda_stream if side is not None else None, _stream()), "copy_back", 0)
+    lib = _lib("ops")
+    args = (slot.host.data_ptr(), _i32(dev, "dev"), n * 4,
+            None if side is None else slot.ready_handle or slot.made_ready(), slot.handle or slot.made(),
+            None if side is None else side.cuda_stream, _stream())
+    slot.wait_native = lib.mf_event_wait
+    _check(lib.mf_copy_back(*args), "copy_back", 0)
 
 
 def _sig_gemm_simt(lib: ctypes.CDLL) -> None:

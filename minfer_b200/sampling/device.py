@@ -78,17 +78,20 @@ class DeviceSampler:
         """Starts copying ``tokens`` to the host on a side stream; ``.get()`` waits for that
         copy only, not for whatever was launched after it."""
         self.engine.d2h_bytes += tokens.numel() * 4
-        # (what the native copy does not take: other integers, strided ones, ones on the host)
-        tokens = tokens.to(self.device, torch.int32).contiguous()
+        if tokens.dtype != torch.int32 or tokens.device != self.device or not tokens.is_contiguous():
+            tokens = tokens.to(self.device, torch.int32).contiguous()      # what the native copy takes
         # pinned buffers are made once and reused in turn (allocating pinned memory is slow and
         # synchronises with the device); a buffer comes around again after RING fetches, long
         # after its tokens were read
         n = tokens.numel()
-        if not self._pinned or self._pinned[0][0].host.numel() < n:
-            self._pinned = [(K.PinnedSlot(max(n, 64)), torch.cuda.Event()) for _ in range(self.RING)]
-        slot, ready = self._pinned[self._next_pinned % self.RING]
+        if not self._pinned or self._pinned[0].host.numel() < n:
+            self._pinned = [K.PinnedSlot(max(n, 64)) for _ in range(self.RING)]
+            for slot in self._pinned:               # (their events now, while the device has the prompt)
+                slot.made()
+                slot.made_ready()
+        slot = self._pinned[self._next_pinned % self.RING]
         self._next_pinned += 1
-        return TokenFetch(tokens, self._copy_stream, slot, ready)
+        return TokenFetch(tokens, self._copy_stream, slot)
 
     def sample(self, logits: torch.Tensor, slots: Sequence[int],
                streams: Sequence[int]) -> List[int]:
@@ -99,13 +102,12 @@ class DeviceSampler:
 class TokenFetch:
     """A device-to-host copy of a few token ids that does not wait for later work."""
 
-    def __init__(self, tokens: torch.Tensor, copy_stream: torch.cuda.Stream, slot: K.PinnedSlot,
-                 ready: torch.cuda.Event):
+    def __init__(self, tokens: torch.Tensor, copy_stream: torch.cuda.Stream, slot: K.PinnedSlot):
         self.slot = slot
         if tokens.numel():
-            K.copy_back(slot, tokens, ready, copy_stream)   # behind the sampling kernel
+            K.copy_back(slot, tokens, copy_stream)   # behind the sampling kernel
         self._keep = tokens                             # not freed before the copy has run
 
     def get(self) -> List[int]:
-        self.slot.event.synchronize()
+        self.slot.wait()
         return self.slot.host[:self._keep.numel()].tolist()
