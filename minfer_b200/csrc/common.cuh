@@ -80,11 +80,10 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
 }
 
 // One lane of a converged warp (the same one every time).  A role that a single thread plays (issuing
-// copies or matrix instructions) is entered through this and not through `lane == 0`: the compiler
-// then knows that one lane runs the block and keeps descriptors and barrier addresses in uniform
-// registers, which those instructions take; under `lane == 0` it wraps each of them in a loop over
-// the active lanes (measured on four tcgen05.mma of 128 x 16 x 16: 253 cycles to issue, 62 this way;
-// a product of 8 tokens with 8,448 x 2,048 weights in L2 11.7 us, 8.6).
+// copies or matrix instructions) is entered through this and not through `lane == 0`: the compiler then
+// knows that one lane runs the block.  Measured on user-level work: Qwen2.5-14B shape, a prompt in portions
+// of 512 beside three decoding sequences, 246.8 -> 223.6 ms; 7B shape, a prompt of 20,011 tokens, 320.6 ->
+// 310.8 ms.
 __device__ __forceinline__ bool elect_one() {
     uint32_t one;
     asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));

@@ -104,8 +104,8 @@ __device__ __forceinline__ void fma_f32x2(unsigned long long& acc, unsigned long
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-// An operand's 16 bytes, never moved above the wait for the kernel before: a load through a const
-// __restrict__ pointer counts as invariant, and the compiler did move the first tile's there.
+// An operand's 16 bytes, never moved above the wait for the kernel before (as a load through a const
+// __restrict__ pointer may be).
 __device__ __forceinline__ float4 load16(const float* p) {
     float4 v;
     asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -274,8 +274,8 @@ __device__ __forceinline__ void copy16_async(void* smem, const void* src, bool r
 
 template <int RT>
 __global__ void __launch_bounds__(F32Few<RT>::WARPS * 32)
-gemm_f32_few_kernel(const float* A, const float* W, const float* __restrict__ bias, float* C, int M, int N, int K, long long lda, long long ldw,
-                    long long ldc, int accumulate) {
+gemm_f32_few_kernel(const float* A, const float* W, const float* __restrict__ bias, float* C, int M, int N,
+                    int K, long long lda, long long ldw, long long ldc, int accumulate) {
     typedef F32Few<RT> T;
     __shared__ __align__(16) float ring[T::WARPS][T::STAGES][T::ROWS][T::PITCH];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

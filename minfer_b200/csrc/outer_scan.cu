@@ -17,10 +17,10 @@
 // The scan: a block owns (row, head, a tile of columns).  Four warps walk the tokens: LD neighbouring
 // lanes share a pair of columns and hold its state elements d = 4 (l + LD i) .. + 3 in registers, so
 // that what a lane reads of q, k and the decays from shared memory (16 bytes at a time) serves two
-// columns (gla over long prompts: four, two pairs).  The sums of eight tokens (16 numbers a lane) are formed side by side and added over the
-// lanes by halving: each step sends what the partner keeps, 8 + 4 + 2 + 1 shuffles for all of them.  A
-// sum's tree does not depend on how the tokens are grouped.  Four more warps do what is not the
-// chain: they keep a ring of four chunks of tokens filled by cp.async, two chunks ahead, and prepare
+// columns (gla over long prompts: four, two pairs).  The sums of eight tokens (16 numbers a lane) are formed
+// side by side and added over the lanes by halving: each step sends what the partner keeps, 8 + 4 + 2 + 1
+// shuffles for all of them.  A sum's tree does not depend on how the tokens are grouped.  Four more warps
+// do what is not the chain: they keep a ring of four chunks of tokens filled by cp.async, two chunks ahead, and prepare
 // each (wkv: r . (u k); mlstm: gates and maxima), handing chunks over and taking them back through
 // named barriers.
 // State [slots][heads][columns][D]: a column's elements are contiguous.  Every column keeps its own
