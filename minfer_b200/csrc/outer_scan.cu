@@ -149,9 +149,10 @@ __device__ __forceinline__ float os_soft_cap(float z, float cap) { return cap * 
 // LD: lanes that share a pair of columns; ND4: float4 groups of a column a lane holds (D <= 4 LD ND4);
 // tc: tokens of a chunk; PAIRS: pairs of columns a lane has (2 c and 2 c + 1, then the same TV / PAIRS on):
 // what it reads of r, k and the decays serves them all; HOLD: the state's addresses stay in registers over
-// the walk (false: they are formed again behind it), see os_choose
-template <int LD, int ND4, int MODE, int PAIRS, bool HOLD>
-__global__ void __launch_bounds__(OS_THREADS + 32 * OS_FEED) outer_scan_kernel(OuterScanArgs a, int tc) {
+// the walk (false: they are formed again behind it); BLOCKS: blocks an SM that the registers are for (0: not
+// asked), see os_choose
+template <int LD, int ND4, int MODE, int PAIRS, bool HOLD, int BLOCKS>
+__global__ void __launch_bounds__(OS_THREADS + 32 * OS_FEED, BLOCKS) outer_scan_kernel(OuterScanArgs a, int tc) {
     pdl_launch_dependents();
     constexpr int DP = 4 * LD * ND4;                   // padded key size
     constexpr int TP = 2 * (OS_THREADS / LD), TV = PAIRS * TP;          // columns of one pair a lane, of the block
@@ -472,7 +473,7 @@ __global__ void __launch_bounds__(OS_THREADS + 32 * OS_FEED) outer_scan_kernel(O
     }
 }
 
-template <int LD, int ND4, int MODE, int PAIRS, bool HOLD>
+template <int LD, int ND4, int MODE, int PAIRS, bool HOLD, int BLOCKS = 0>
 static int os_launch(const OuterScanArgs& a, int max_tokens, cudaStream_t stream) {
     constexpr int DP = 4 * LD * ND4, TV = PAIRS * 2 * (OS_THREADS / LD), NVEC = OuterTraits<MODE>::DECAYS ? 3 : 2;
     // (short rows take shorter chunks, so that more blocks fit an SM: single tokens most of all)
@@ -482,14 +483,14 @@ static int os_launch(const OuterScanArgs& a, int max_tokens, cudaStream_t stream
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MF_ERR_UNSUPPORTED;
     if (!configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(outer_scan_kernel<LD, ND4, MODE, PAIRS, HOLD>,
+        cudaError_t e = cudaFuncSetAttribute(outer_scan_kernel<LD, ND4, MODE, PAIRS, HOLD, BLOCKS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(OS_TC));
         if (e != cudaSuccess) return (int)e;
         configured[dev] = true;
     }
     const int cols = OuterTraits<MODE>::GATES ? a.Dv + 1 : a.Dv;
     const int tiles = (cols + TV - 1) / TV;
-    mf_launch(outer_scan_kernel<LD, ND4, MODE, PAIRS, HOLD>, dim3(a.heads * tiles, a.n_rows), dim3(OS_THREADS + 32 * OS_FEED), bytes(tc),
+    mf_launch(outer_scan_kernel<LD, ND4, MODE, PAIRS, HOLD, BLOCKS>, dim3(a.heads * tiles, a.n_rows), dim3(OS_THREADS + 32 * OS_FEED), bytes(tc),
               stream, a, tc);
     return MF_LAUNCH_CHECK();
 }
@@ -520,20 +521,27 @@ static int os_choose(const OuterScanArgs& a, int max_tokens, int n_tokens, cudaS
             return a.D <= 64 ? os_launch<16, 1, MODE, 2, false>(a, max_tokens, stream)
                              : os_launch<16, 2, MODE, 2, false>(a, max_tokens, stream);
     }
-    // HOLD changes no operation, only how many registers the walk has left and how many blocks an SM takes.
-    // Rows of few tokens are bound by the state they read and write, long ones by the walk; us, held against
-    // formed again, 64 rows of one token and one row of 2,048:
-    //     D 32 (64 heads of 32 columns)    wkv 20.8 [21.9], 171.6 [172.5]    gla 19.3 [20.4], 169 [157]
-    //     D 128 (16 heads of 128)          wkv 68.4 [68.8], 334 [337]        gla 54.5 [41.3], 283 [288]
-    //     D 100 (16 heads of 70)           gla 46.5 [35.2], 236 [264]        mlstm at D 128 60.6 [62.0]
+    // HOLD and BLOCKS change no operation, only how many registers the walk has and how many blocks an SM takes.
+    // Rows of few tokens are bound by the state they read and write, long ones by the walk.  us for 64 rows of
+    // one token and for one row of 2,048, with the other choice in brackets:
+    //     D 32, 64 heads of 32 columns: held (wkv, gla of few tokens)   wkv 20.8 [21.9], 172 [173]; gla 19.3 [20.4], 169 [157]
+    //     D 128, 16 heads of 128: held (wkv, mlstm)                     wkv 68.4 [68.8], 334 [337]; mlstm 60.6 [62.0], 279 [278]
+    //     gla: two blocks asked for (not for few tokens: three fit)     53.6 [41.7], 258 [288]
+    //     D 100, 16 heads of 70, gla                                    46.3 [35.2], 215 [264]
     const bool brief = max_tokens >= 1 && max_tokens < OS_TC;
-    if (a.D <= 32)
-        return brief || MODE == OS_MLSTM ? os_launch<8, 1, MODE, 1, true>(a, max_tokens, stream)
-                                         : os_launch<8, 1, MODE, 1, false>(a, max_tokens, stream);
+    if (a.D <= 32) {
+        if constexpr (MODE != OS_MLSTM)
+            if (!brief) return os_launch<8, 1, MODE, 1, false>(a, max_tokens, stream);
+        return os_launch<8, 1, MODE, 1, true>(a, max_tokens, stream);
+    }
     if (a.D <= 64) return os_launch<16, 1, MODE, 1, false>(a, max_tokens, stream);
-    if (a.D <= 128)
-        return brief && MODE == OS_GLA ? os_launch<16, 2, MODE, 1, false>(a, max_tokens, stream)
-                                       : os_launch<16, 2, MODE, 1, true>(a, max_tokens, stream);
+    if (a.D <= 128) {
+        if constexpr (MODE == OS_GLA)
+            return brief ? os_launch<16, 2, MODE, 1, false>(a, max_tokens, stream)
+                         : os_launch<16, 2, MODE, 1, false, 2>(a, max_tokens, stream);
+        else
+            return os_launch<16, 2, MODE, 1, true>(a, max_tokens, stream);
+    }
     return os_launch<32, 2, MODE, 1, false>(a, max_tokens, stream);
 }
 
