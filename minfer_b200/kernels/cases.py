@@ -664,6 +664,96 @@ def pazatar_step_decode(reps, batch=8, ctx=2048):
     print(f"pazatar decode step, batch {batch} at {ctx} positions, two layers: {us:.1f} us")
 
 
+# ---- kernels whose form is chosen by the sizes of a call -------------------------------------------
+def float32_products(reps):
+    """Float32 products behind a norm and alone, with the tile each size takes."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    names = {0: "128 x 128", 1: "64 x 64", 2: "32 x 64", -1: "general"}
+    for m, n, k in ((8, 896, 4864), (64, 896, 4864), (200, 4096, 2048), (385, 1152, 896), (385, 9728, 896),
+                    (385, 896, 4864), (385, 151936, 896), (1600, 8448, 2048), (4096, 9728, 896)):
+        h, g = torch.randn(m, k, device="cuda"), torch.rand(k, device="cuda")
+        x, w = torch.empty(m, k, device="cuda"), torch.randn(n, k, device="cuda")
+        out = torch.empty(m, n, device="cuda")
+
+        def both():
+            K.rmsnorm(h, g, 1e-5, x)
+            K.gemm_simt(x, w, None, out)
+        after, alone = _time(both, reps), _time(lambda: K.gemm_simt(x, w, None, out), reps)
+        tile = "few rows" if m <= 16 else names[K._lib("gemm_simt").mf_gemm_f32_tile(m, n, sms)]
+        print(f"float32 {m} x {n} x {k} ({tile}): norm and product {after:.1f} us, product alone {alone:.1f} us, "
+              f"{2.0 * m * n * k / alone / 1e6:.1f} TFLOP/s")
+
+
+def _rows(lens):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    return torch.tensor(cu, dtype=torch.int32, device="cuda")
+
+
+def float32_prompt_attention(reps):
+    """Float32 prompts of several lengths, 14 heads of 64: as chosen, and a warp a query."""
+    for lens in ([32], [200], [1] * 64, [16] * 16, [64] * 8, [130, 255], [400] * 4, [1] * 63 + [1000],
+                 [1] * 31 + [200]):
+        n = sum(lens)
+        q, k, v = (torch.randn(n, h, 64, device="cuda") for h in (14, 2, 2))
+        row = torch.tensor([b for b, c in enumerate(lens) for _ in range(c)], dtype=torch.int32, device="cuda")
+        pos = torch.tensor([i for c in lens for i in range(c)], dtype=torch.int32, device="cuda")
+        cu, out = _rows(lens), torch.empty(n, 14 * 64, device="cuda")
+        us = [_time(lambda: K.attention_packed(q, k, v, row, pos, cu, out, 14, 2, 64, w, 0.125, longest=max(lens)),
+                    reps) for w in (0, 1 << 20)]           # (a window beyond every position: a warp a query)
+        tiled = K._lib("attention").mf_attention_packed_tiled(n, len(lens), max(lens))
+        print(f"float32 attention, {len(lens)} prompts of {min(lens)} to {max(lens)}, {n} tokens "
+              f"({'32 rows together' if tiled else 'a warp a query'}): {us[0]:.1f} us, a warp a query {us[1]:.1f} us")
+
+
+def scans_of_row_mixes(reps):
+    """The state-space scan and gated linear attention over rows of several lengths, with the columns chosen."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    eight = [601, 700, 800, 900, 1000, 1100, 1200, 1300]
+    mixes = ([1] * 8, [1] * 64, [16] * 8, [300] * 3, [3] * 7 + [400], eight, [2048])
+    for heads, width, n_state in ((64, 64, 128), (24, 64, 64), (64, 96, 128)):
+        for lens in mixes:
+            n, rows, inner = sum(lens), len(lens), heads * width
+            u = torch.randn(n, inner + 2 * n_state, device="cuda") * 0.3
+            proj, y = torch.randn(n, heads, device="cuda"), torch.empty(n, inner, device="cuda")
+            z = torch.zeros(heads, device="cuda")
+            state = torch.zeros(rows, heads, width, n_state, device="cuda")
+            cu, slots = _rows(lens), torch.arange(rows, dtype=torch.int32, device="cuda")
+            us = _time(lambda: K.ssm_scan(u, proj, 0, z, z, z, state, cu, slots, y, rows, heads, width, n_state, 1,
+                                          max_tokens=max(lens)), reps)
+            cols = K._lib("recurrent").mf_ssm_scan_columns(n, rows, max(lens), heads, width, n_state, sms)
+            print(f"ssm_scan {heads} heads of {width}, state {n_state}, {rows} rows, {n} tokens, the longest "
+                  f"{max(lens)} (columns a thread: {cols}): {us:.1f} us")
+    for heads, d, dv in ((8, 128, 256), (60, 36, 40)):
+        for lens in mixes:
+            n, rows = sum(lens), len(lens)
+            proj = torch.randn(n, heads * (2 * d + dv), device="cuda")
+            decay, out = torch.rand(n, heads * d, device="cuda"), torch.empty(n, heads * dv, device="cuda")
+            state = torch.zeros(rows, heads, dv, d, device="cuda")
+            cu, slots = _rows(lens), torch.arange(rows, dtype=torch.int32, device="cuda")
+            us = _time(lambda: K.gla_scan(proj, 0, heads * d, 2 * heads * d, decay, d ** -0.5, state, cu, slots, out,
+                                          rows, max(lens)), reps)
+            cols = K._lib("outer_scan").mf_gla_scan_columns(n, max(lens), heads, d, dv, sms)
+            print(f"gla_scan {heads} heads of {d} x {dv}, {rows} rows, {n} tokens, the longest {max(lens)} "
+                  f"(columns a lane: {cols}): {us:.1f} us")
+
+
+def gemm_m65_to_255(reps):
+    """Products of 65 to 255 tokens (tiles of 128), and grouped ones of 20 to 300 rows a group."""
+    for m in (65, 128, 200, 255):
+        for n, k in ((2 * NF, NE), (NE, NF), (9728, 896)):
+            _gemm(m, n, k, K.EPI_STORE, reps)
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    w = torch.randn(16, 1408, 2048, device="cuda", dtype=torch.bfloat16)
+    for rows in (20, 40, 64, 128, 300):
+        x = torch.randn(16 * rows, 2048, device="cuda", dtype=torch.bfloat16)
+        out = torch.empty(16 * rows, 1408, device="cuda")
+        us = _time(lambda: K.gemm_tc_grouped(x, w, out, None, st), reps)
+        print(f"gemm_tc_grouped 16 groups of {rows} x 1,408 x 2,048: {us:.1f} us, "
+              f"{2.0 * 16 * rows * 1408 * 2048 / us / 1e6:.1f} TFLOP/s")
+
+
 CASES = {f.__name__: f for f in (gemm_decode, gemm_decode_split, gemm_decode_m64, gemm_decode_split_m64, gemm_prefill, gemm_prefill_down,
                                  gemm_decode_cluster, gemm_decode_cluster_o, gemm_decode_cluster_m64,
                                  attention_decode, attention_decode_b8, attention_decode_long, attention_prefill,
@@ -674,7 +764,8 @@ CASES = {f.__name__: f for f in (gemm_decode, gemm_decode_split, gemm_decode_m64
                                  ssm_scan_prompt, ssm_scan_decode, budanex_step_prefill, budanex_step_decode,
                                  zanelorn_step_prefill, zanelorn_step_decode,
                                  pikavik_step_prefill, pikavik_step_decode,
-                                 pazatar_step_prefill, pazatar_step_decode)}
+                                 pazatar_step_prefill, pazatar_step_decode,
+                                 float32_products, float32_prompt_attention, scans_of_row_mixes, gemm_m65_to_255)}
 
 
 def main(argv=None) -> int:
