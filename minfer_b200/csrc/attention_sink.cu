@@ -825,6 +825,7 @@ struct SinkDecodeArgs {
     int keep_first;           // > 0: keys at positions below it stay visible beyond the window
     int tiles_per_cta, n_splits;
     int n_bufs;               // buffers a warp has: 2, or 1 when it takes one tile only
+    int old_keys_final;       // 1: of the keys a row sees, only the one at its own position is of this step
     float scale_log2;
     const float* sink_logit;  // [n_heads] score of the sink, or null for 0
     float cap_log2;           // soft cap * log2(e); 0: no cap
@@ -880,8 +881,6 @@ __global__ void __launch_bounds__(SD_WARPS * 32) sink_attention_decode_kernel(Si
         if (g < Gb) { r1v[0] = a.r1[hk * G + g0 + g]; r2v[0] = a.r2[hk * G + g0 + g]; }
         if (g + 8 < Gb) { r1v[1] = a.r1[hk * G + g0 + g + 8]; r2v[1] = a.r2[hk * G + g0 + g + 8]; }
     }
-    pdl_wait();
-
     const uint32_t my_s = (uint32_t)__cvta_generic_to_shared(sd_smem) + (uint32_t)(warp * a.n_bufs * TILE_BYTES);
     auto load_tile = [&](int tile, int buf) {
         const int key0 = tile * SD_KEYS;
@@ -895,7 +894,16 @@ __global__ void __launch_bounds__(SD_WARPS * 32) sink_attention_decode_kernel(Si
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     int tile = tile_lo + warp;
-    if (tile <= tile_hi) load_tile(real_tile(tile), 0);
+    // In a step of one token a row the kernel before this one writes one position of the row, its own: a
+    // tile that lies below it (and, in a ring, does not share its slot) is copied before the wait.
+    auto old_tile = [&](int vt) {
+        const int key0 = real_tile(vt) * SD_KEYS;
+        return a.old_keys_final != 0 && key0 + SD_KEYS - 1 < pos && (a.ring == 0 || key0 + a.ring > pos);
+    };
+    const bool early = tile <= tile_hi && old_tile(tile);
+    if (early) load_tile(real_tile(tile), 0);
+    pdl_wait();
+    if (tile <= tile_hi && !early) load_tile(real_tile(tile), 0);
 
     float m_r[2] = {-INFINITY, -INFINITY}, l_r[2] = {0.0f, 0.0f};
     float o[VDP / 8][4];
@@ -1071,6 +1079,35 @@ __global__ void sink_decode_combine_kernel(const float* partial,
     const size_t stride = (size_t)(vd + 2);
     const float* p = partial + rh * n_splits * stride;
     const float sink2 = (sink && sink_logit) ? sink_logit[rh % n_heads] * 1.4426950408889634f : 0.0f;
+    if (n_splits <= 16) {
+        // the usual case: every maximum, sum and value a thread needs in one trip (the loops below make
+        // three and more); the same operations in the same order
+        float mc[16], lc[16], oc[16];
+        const int d = threadIdx.x;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+            mc[c] = -INFINITY;
+            if (c < n_splits) {
+                mc[c] = p[c * stride];
+                lc[c] = p[c * stride + 1];
+                oc[c] = d < vd ? p[c * stride + 2 + d] : 0.0f;
+            }
+        }
+        float m = sink ? sink2 : -INFINITY;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) m = fmaxf(m, mc[c]);
+        float l = sink ? exp2f(sink2 - m) : 0.0f, acc = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+            if (mc[c] > -INFINITY) {
+                const float f = exp2f(mc[c] - m);
+                l = fmaf(lc[c], f, l);
+                acc = fmaf(oc[c], f, acc);
+            }
+        }
+        if (d < vd) out[rh * vd + d] = __float2bfloat16_rn(acc * (1.0f / l));
+        return;
+    }
     float m = sink ? sink2 : -INFINITY;
     for (int c = 0; c < n_splits; ++c) m = fmaxf(m, p[c * stride]);
     float l = sink ? exp2f(sink2 - m) : 0.0f;
@@ -1130,7 +1167,8 @@ static int launch_sink_decode(const SinkDecodeArgs& a, int rows, cudaStream_t st
 // Every row of q [rows][n_heads][hd] (bfloat16) is a query at row_pos over the paged cache.
 // `reach_keys`: the most keys a query sees (chunk, window, or the longest sequence's length).
 // `partial`: float32 scratch of rows * n_heads * splits * (vd + 2) floats when the plan has
-// more than one split (mf_sink_decode_plan), else unused.
+// more than one split (mf_sink_decode_plan), else unused.  `old_keys_final`: every row is its
+// sequence's only new token in this step, so the keys below its position are earlier steps'.
 extern "C" int mf_sink_attention_decode(const void* q, const void* k_cache, const void* v_cache,
                                         const int* row_seq, const int* row_pos,
                                         const int* page_table, int table_stride, int ring,
@@ -1138,7 +1176,7 @@ extern "C" int mf_sink_attention_decode(const void* q, const void* k_cache, cons
                                         const float* r2, int rows, int n_heads, int n_kv, int hd,
                                         int vd, int window, int chunk, int sink, float scale,
                                         int reach_keys, const float* sink_logit, float softcap,
-                                        int keep_first, cudaStream_t stream) {
+                                        int keep_first, int old_keys_final, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (keep_first < 0 || (keep_first > 0 && (ring > 0 || chunk > 0))) return MF_ERR_UNSUPPORTED;
     if (softcap < 0.0f) return MF_ERR_ARGUMENT;
@@ -1160,6 +1198,7 @@ extern "C" int mf_sink_attention_decode(const void* q, const void* k_cache, cons
     a.scale_over_cap = softcap > 0.0f ? scale / softcap : 0.0f;
     mf_sink_decode_plan(rows, head_blocks, reach_keys, &a.tiles_per_cta, &a.n_splits);
     a.n_bufs = a.tiles_per_cta > SD_WARPS ? 2 : 1;
+    a.old_keys_final = old_keys_final;
     if (a.n_splits > 1 && partial == nullptr) return MF_ERR_ARGUMENT;
     int e;
     if (hd <= 64) e = vd <= 64 ? launch_sink_decode<64, 64>(a, rows, stream)

@@ -96,17 +96,23 @@ __host__ __device__ constexpr bool epi_needs_whole_sum(int epi) {
     return epi == EPI_SWIGLU || epi == EPI_XIELU;
 }
 
-// 1 / rms of the token rows m0 + t, t = first, first + step, .. < n_tok, into out[t] (shared
-// memory): a thread adds a token's parts in order, all of its loads in flight together.
-__device__ __forceinline__ void row_scales(const GemmArgs& a, int m0, int n_tok, float* out, int first, int step) {
-    for (int t = first; t < n_tok; t += step) {
+// 1 / rms of the token rows m0 + t, t < n_tok, into out[t] (shared memory), by `warps` whole warps of
+// which the calling one is number `warp`: a warp takes eight tokens at a time, four lanes a token, each
+// lane every fourth part with eight loads in flight, then the four sums in a fixed order.
+__device__ __forceinline__ void row_scales(const GemmArgs& a, int m0, int n_tok, float* out, int warp, int warps,
+                                           int lane) {
+    for (int t0 = warp * 8; t0 < n_tok; t0 += warps * 8) {
+        if (m0 + t0 >= a.M) break;                   // (rows beyond the last token are never stored)
+        const int t = t0 + (lane & 7);
         float sum = 0.0f;
         if (m0 + t < a.M) {
             const float* col = a.row_ssq + m0 + t;
 #pragma unroll 8
-            for (int p = 0; p < a.ssq_parts; ++p) sum += col[(size_t)p * a.M];
+            for (int p = lane >> 3; p < a.ssq_parts; p += 4) sum += col[(size_t)p * a.M];
         }
-        out[t] = rsqrtf(sum / (float)a.ssq_width + a.ssq_eps);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+        if (lane < 8) out[t] = rsqrtf(sum / (float)a.ssq_width + a.ssq_eps);
     }
 }
 
@@ -210,6 +216,26 @@ __host__ __device__ constexpr uint32_t umma_idesc(int nt) {
            ((uint32_t)(TILE_N >> 4) << 24);
 }
 
+// EPI_SWIGLU: act(g) * u for the gate's activation
+__device__ __forceinline__ float gated_act(const GemmArgs& a, float g, float u) {
+    if (a.gate_act == EPI_GATE_GELU_TANH) {
+        // 0.5 g (1 + tanh(c (g + 0.044715 g^3))) = g / (1 + exp(-2 c (g + 0.044715 g^3)))
+        const float z = 1.5957691216057308f * fmaf(0.044715f * g, g * g, g);
+        return __fdividef(g * u, 1.0f + __expf(-z));
+    }
+    if (a.gate_act == EPI_GATE_CLAMPED_SWISH) {
+        const float gc = fminf(g, a.act_p), uc = fminf(fmaxf(u, -a.act_p), a.act_p);
+        return __fdividef(gc * (uc + 1.0f), 1.0f + __expf(-a.act_n * gc));
+    }
+    return __fdividef(g * u, 1.0f + __expf(-g));
+}
+
+// EPI_XIELU
+__device__ __forceinline__ float xielu_act(const GemmArgs& a, float v) {
+    return v > 0.0f ? fmaf(a.act_p * v, v, a.act_l * v)
+                    : fmaf(a.act_n, (__expf(v) - 1.0f) - v, a.act_l * v);
+}
+
 // One chunk of the epilogue: this thread's 16 consecutive tokens (tok0 ..) of output row n.
 // `scale` (may be null): 1 / rms of these 16 tokens, applied to the accumulators first.
 __device__ __forceinline__ void store_chunk(const GemmArgs& a, const uint32_t* r_in, int n, bool n_ok,
@@ -233,17 +259,7 @@ __device__ __forceinline__ void store_chunk(const GemmArgs& a, const uint32_t* r
             const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
             const float g = even ? keep : recv, u = even ? recv : keep;
             const int tok = tok0 + 2 * jj + (even ? 0 : 1);
-            float y;
-            if (a.gate_act == EPI_GATE_GELU_TANH) {
-                // 0.5 g (1 + tanh(c (g + 0.044715 g^3))) = g / (1 + exp(-2 c (g + 0.044715 g^3)))
-                const float z = 1.5957691216057308f * fmaf(0.044715f * g, g * g, g);
-                y = __fdividef(g * u, 1.0f + __expf(-z));
-            } else if (a.gate_act == EPI_GATE_CLAMPED_SWISH) {
-                const float gc = fminf(g, a.act_p), uc = fminf(fmaxf(u, -a.act_p), a.act_p);
-                y = __fdividef(gc * (uc + 1.0f), 1.0f + __expf(-a.act_n * gc));
-            } else {
-                y = __fdividef(g * u, 1.0f + __expf(-g));
-            }
+            const float y = gated_act(a, g, u);
             if (tok < a.M && n_ok) o[(size_t)(2 * jj) * a.ldo] = __float2bfloat16_rn(y);
         }
     } else if (a.epi == EPI_ACCUM && a.bias == nullptr) {
@@ -286,8 +302,8 @@ __device__ __forceinline__ void store_chunk(const GemmArgs& a, const uint32_t* r
                 v0 = a.act_p * p0 * p0;
                 v1 = a.act_p * p1 * p1;
             } else if (a.epi == EPI_XIELU) {
-                v0 = v0 > 0.0f ? fmaf(a.act_p * v0, v0, a.act_l * v0) : fmaf(a.act_n, (__expf(v0) - 1.0f) - v0, a.act_l * v0);
-                v1 = v1 > 0.0f ? fmaf(a.act_p * v1, v1, a.act_l * v1) : fmaf(a.act_n, (__expf(v1) - 1.0f) - v1, a.act_l * v1);
+                v0 = xielu_act(a, v0);
+                v1 = xielu_act(a, v1);
             }
             const float keep = even ? v0 : v1, send = even ? v1 : v0;
             const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
@@ -302,9 +318,7 @@ __device__ __forceinline__ void store_chunk(const GemmArgs& a, const uint32_t* r
         for (int j = 0; j < 16; ++j) {
             const int tok = tok0 + j;
             float v = __uint_as_float(r[j]) + bias;
-            if (a.epi == EPI_XIELU)
-                v = v > 0.0f ? fmaf(a.act_p * v, v, a.act_l * v)
-                             : fmaf(a.act_n, (__expf(v) - 1.0f) - v, a.act_l * v);
+            if (a.epi == EPI_XIELU) v = xielu_act(a, v);
             if (tok < a.M && n_ok) {
                 if (a.epi == EPI_PARTIAL)
                     a.partial[((size_t)split * a.M + tok) * a.N + n] = v;
@@ -458,7 +472,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         pdl_wait();          // every other thread: nothing below may run ahead of the kernel before
     }
     // the tokens' 1 / rms, by the warps from the third on, which have nothing to do while the weights stream
-    if (a.row_ssq != nullptr && warp >= 2) row_scales(a, m0, NT, scale_s, tid - 64, few_threads(NT) - 64);
+    if (a.row_ssq != nullptr && warp >= 2) row_scales(a, m0, NT, scale_s, warp - 2, few_threads(NT) / 32 - 2, lane);
     if (warp == 1 && elect_one()) {
         // ---- MMA issuer --------------------------------------------------------------
         constexpr uint32_t idesc = umma_idesc(NT);
@@ -632,7 +646,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     } else {
         pdl_wait();
     }
-    if (a.row_ssq != nullptr && warp >= 2) row_scales(a, m0, NT, scale_s, tid - 64, few_threads(NT) - 64);
+    if (a.row_ssq != nullptr && warp >= 2) row_scales(a, m0, NT, scale_s, warp - 2, few_threads(NT) / 32 - 2, lane);
     if (warp == 1 && elect_one()) {
         // ---- MMA issuer ---------------------------------------------------------------------
         constexpr uint32_t idesc = umma_idesc(NT);
@@ -744,6 +758,278 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;"
                      ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS) : "memory");
     }
+}
+
+// ------------------------------------------------------------------------------------------
+// A handful of tokens (decoding): the weights go through shared memory that only the lane that
+// copied them reads (cp.async, no barrier, no roles, no hand-over) into mma.sync.m16n8k16 as its B
+// operand, 8 rows of W and 16 k; the tokens, up to 16 of them, are its A operand.
+//   * A CTA owns `row_tiles` tiles of 8 rows of W; its warps cut K between them.  The order
+//     of k inside a product is free as long as both operands agree, so a lane takes 8 consecutive k
+//     (16 bytes) of a row where the fragments of two products would want 2 + 2 each.
+//   * A warp has DEPTH units (8 rows x 64 k, 1 KB) in flight, the first ones asked for BEFORE
+//     griddepcontrol.wait: weights are constant over the step.  Where a product's weights fit the
+//     rings of all CTAs they are on the chip when the kernel before ends; what lies beyond is asked
+//     for in L2.  A CTA takes half of an SM, so that the next product's CTA does this while this one
+//     computes.
+//   * The tokens come after the wait, every lane's own fragments, all in flight together.  Where a
+//     CTA's share of them is too large, or rows alone leave SMs idle, a cluster of CTAs shares the
+//     rows and cuts K.
+//   * The warps' sums meet in shared memory and are added in warp order, a cluster's in rank order:
+//     reproducible, and complete, so no next kernel has K splits to add.
+// ------------------------------------------------------------------------------------------
+#define FEW_WARPS 16
+#define FEW_THREADS (32 * FEW_WARPS)
+#define FEW_MAX_M 16
+#define FEW_BUDGET (112 * 1024)       // shared memory of a CTA
+#define FEW_LIMIT_MB 64
+#define FEW_L2 1
+
+struct FewArgs {
+    const __nv_bfloat16* w;
+    const __nv_bfloat16* x;
+    long long ldw, ldx;
+    int row_tiles;            // tiles of 8 rows a CTA
+    int warp_units;           // units of 64 k a warp
+    int tok_stride;           // floats between two tokens' sums
+    int cluster;              // CTAs that share the same rows and cut K between them (1, 2 or 4)
+};
+
+__device__ __forceinline__ void few_copy_w(uint32_t dst, const __nv_bfloat16* p, bool ok) {
+    asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(p), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void few_mma(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9},"
+        " {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// NT: tokens in tiles of 8 (1 or 2 of them)
+template <int NT, int DEPTH>
+__global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const FewArgs f, const GemmArgs a) {
+    extern __shared__ __align__(16) uint8_t few_smem[];
+    pdl_launch_dependents();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int rank = f.cluster > 1 ? (int)rank_in_cluster() : 0, group = blockIdx.x / f.cluster;
+    const int n0 = group * 8 * f.row_tiles;
+    const int tiles = min(f.row_tiles, (a.N - n0 + 7) >> 3);
+    const int units = (a.K + 63) >> 6;
+    const int u0 = min((rank * FEW_WARPS + warp) * f.warp_units, units);
+    const int nu = min(f.warp_units, units - u0);
+    const int items = tiles * nu;
+    const int rows = 8 * f.row_tiles;
+    const int warp_red = a.M * f.tok_stride;
+    uint8_t* ring = few_smem + warp * DEPTH * 1024 + lane * 16;                // [depth][2][32 lanes][16 bytes]
+    uint8_t* x_s = few_smem + FEW_WARPS * DEPTH * 1024 + (size_t)warp * f.warp_units * a.M * 128;
+    float* red = (float*)(few_smem + FEW_WARPS * (DEPTH * 1024 + f.warp_units * a.M * 128));   // [warps][tokens][tok_stride]
+    float* scale_s = red + FEW_WARPS * warp_red;                               // [16]
+    float* sq_s = scale_s + 16;                                                // [tokens][row_tiles]
+    float* own_s = sq_s + a.M * f.row_tiles;                                   // cluster > 1: [tokens][rows] this CTA's sums
+
+    // ---- weights: the first units before the wait ------------------------------------------------
+    const int k_lane = u0 * 64 + 8 * t;                              // this lane's first k of unit 0
+    const __nv_bfloat16* wp = f.w + (size_t)(n0 + g) * f.ldw + k_lane;
+    const uint32_t ring_u = smem_u32(ring);
+    int ln = n0 + g, lu = 0, to_load = items;                        // the load cursor: row, unit
+    auto load_next = [&](uint32_t dst) {
+        if (to_load > 0) {
+            const int k = k_lane + lu * 64;
+            const bool oa = ln < a.N && k < a.K, ob = ln < a.N && k + 32 < a.K;
+            few_copy_w(dst, oa ? wp + lu * 64 : f.w, oa);
+            few_copy_w(dst + 512, ob ? wp + lu * 64 + 32 : f.w, ob);
+            --to_load;
+            if (++lu == nu) { lu = 0; ln += 8; wp += 8 * f.ldw; }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d) load_next(ring_u + d * 1024);
+    if (FEW_L2 && lane < 8 && nu > 0) {
+        // whole rows of this warp's stretch of k: the tiles that the ring has not reached
+        for (int r = DEPTH / nu; r < tiles; ++r) {
+            const int n = n0 + 8 * r + lane;
+            if (n < a.N)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
+                             ::"l"(f.w + (size_t)n * f.ldw + u0 * 64), "r"(min(nu * 64, a.K - u0 * 64) * 2) : "memory");
+        }
+    }
+
+    pdl_wait();
+    // ---- tokens: this lane's own fragments, [unit][half][token][4 lanes][16 bytes] -----------------
+    {
+        const uint32_t dst = smem_u32(x_s) + (uint32_t)(g * 64 + t * 16);
+        for (int u = 0; u < nu; ++u) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    const int tok = 8 * j + g, k = k_lane + u * 64 + h * 32;
+                    if (tok < a.M)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                                     ::"r"(dst + (uint32_t)(((2 * u + h) * a.M + 8 * j) * 64)),
+                                       "l"(f.x + (size_t)tok * f.ldx + (k < a.K ? k : 0)), "r"(k < a.K ? 16 : 0)
+                                     : "memory");
+                }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    // what the end of the kernel needs besides the sums is asked for now.  (token, row) pairs this CTA
+    // finishes, rows fastest: all, or in a cluster those of tokens rank, rank + cluster, ..
+    const int my_tokens = (a.M - rank + f.cluster - 1) / f.cluster, work = my_tokens * rows;
+    float old[2] = {0.0f, 0.0f};
+    if (a.epi == EPI_ACCUM) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int idx = tid + i * FEW_THREADS, mine = idx / rows, n = n0 + idx - mine * rows;
+            const int tok = rank + mine * f.cluster;
+            if (idx < work && n < a.N) old[i] = ((const float*)a.out)[(size_t)tok * a.ldo + n];
+        }
+    }
+    if (a.row_ssq != nullptr) {
+        for (int tok = warp; tok < a.M; tok += FEW_WARPS) {
+            float sum = 0.0f;
+#pragma unroll 8
+            for (int p = lane; p < a.ssq_parts; p += 32) sum += a.row_ssq[(size_t)p * a.M + tok];
+            sum = warp_sum(sum);
+            if (lane == 0) scale_s[tok] = rsqrtf(sum / (float)a.ssq_width + a.ssq_eps);
+        }
+    }
+    // (the weights asked for before the wait have had the time of the kernel before to arrive)
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+
+    // ---- products -----------------------------------------------------------------------------------
+    float acc[2][4];                                                 // two chains of sums
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[c >> 2][c & 3] = 0.0f;
+    float* red_w = red + (size_t)warp * warp_red + g * f.tok_stride + 2 * t;
+    const bool has0 = g < a.M, has1 = NT > 1 && 8 + g < a.M;
+    const uint8_t* xp = x_s + g * 64 + t * 16;
+    int u = 0, slot = 0;
+    for (int i = 0; i < items; ++i) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(DEPTH - 1) : "memory");
+        const uint4 w0 = *(const uint4*)(ring + slot * 1024), w1 = *(const uint4*)(ring + slot * 1024 + 512);
+        uint4 x0 = make_uint4(0u, 0u, 0u, 0u), x1 = x0, y0 = x0, y1 = x0;
+        if (has0) {
+            x0 = *(const uint4*)(xp + (2 * u) * a.M * 64);
+            x1 = *(const uint4*)(xp + (2 * u + 1) * a.M * 64);
+        }
+        if (has1) {
+            y0 = *(const uint4*)(xp + ((2 * u) * a.M + 8) * 64);
+            y1 = *(const uint4*)(xp + ((2 * u + 1) * a.M + 8) * 64);
+        }
+        few_mma(acc[0], x0.x, y0.x, x0.y, y0.y, w0.x, w0.y);
+        few_mma(acc[1], x0.z, y0.z, x0.w, y0.w, w0.z, w0.w);
+        few_mma(acc[0], x1.x, y1.x, x1.y, y1.y, w1.x, w1.y);
+        few_mma(acc[1], x1.z, y1.z, x1.w, y1.w, w1.z, w1.w);
+        load_next(ring_u + slot * 1024);
+        if (++slot == DEPTH) slot = 0;
+        if (++u == nu) {                                             // a row tile is complete
+            u = 0;
+            float s[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) s[c] = acc[0][c] + acc[1][c];
+            if (has0) *(float2*)red_w = make_float2(s[0], s[1]);
+            if (has1) *(float2*)(red_w + 8 * f.tok_stride) = make_float2(s[2], s[3]);
+            red_w += 8;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) acc[c >> 2][c & 3] = 0.0f;
+        }
+    }
+    // warps of this CTA that have k
+    const int live = min(FEW_WARPS, max(0, (units - rank * FEW_WARPS * f.warp_units + f.warp_units - 1) / f.warp_units));
+    __syncthreads();
+
+    // ---- epilogue ---------------------------------------------------------------------------------
+    auto warps_sum = [&](int tok, int row) {
+        const float* r = red + tok * f.tok_stride + row;
+        float v = 0.0f;
+#pragma unroll
+        for (int s = 0; s < FEW_WARPS; ++s)
+            if (s < live) v += r[s * warp_red];
+        return v;
+    };
+    if (f.cluster > 1) {
+        // every CTA's sums for all tokens, then across the cluster in rank order
+        for (int idx = tid; idx < a.M * rows; idx += FEW_THREADS) {
+            const int tok = idx / rows, row = idx - tok * rows;
+            if (row < 8 * tiles) own_s[idx] = warps_sum(tok, row);
+        }
+        __syncwarp();
+        cluster_barrier();
+    }
+    auto sum_of = [&](int tok, int row) {
+        float v = 0.0f;
+        if (f.cluster > 1) {
+            const uint32_t at = smem_u32(own_s + tok * rows + row);
+            for (int r = 0; r < f.cluster; ++r) {
+                float part;
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(part) : "r"(map_to_rank(at, (uint32_t)r)) : "memory");
+                v += part;
+            }
+        } else {
+            v = warps_sum(tok, row);
+        }
+        return a.row_ssq != nullptr ? v * scale_s[tok] : v;
+    };
+    if (a.epi == EPI_SWIGLU) {
+        const int half = rows >> 1;
+        for (int idx = tid; idx < my_tokens * half; idx += FEW_THREADS) {
+            const int mine = idx / half, c = idx - mine * half, tok = rank + mine * f.cluster;
+            if (n0 + 2 * c < a.N)
+                ((__nv_bfloat16*)a.out)[(size_t)tok * a.ldo + (n0 >> 1) + c] =
+                    __float2bfloat16_rn(gated_act(a, sum_of(tok, 2 * c), sum_of(tok, 2 * c + 1)));
+        }
+    } else {
+        // (whole groups of 8 lanes: their pairs belong to one token and one row tile)
+        for (int idx = tid, i = 0; idx - lane < work; idx += FEW_THREADS, ++i) {
+            const int mine = idx / rows, row = idx - mine * rows, n = n0 + row, tok = rank + mine * f.cluster;
+            const bool ok = idx < work && n < a.N;
+            float sq = 0.0f;
+            if (ok) {
+                float v = sum_of(tok, row);
+                if (a.bias != nullptr) v += a.bias[n];
+                if (a.epi == EPI_ACCUM) {
+                    float* o = (float*)a.out + (size_t)tok * a.ldo + n;
+                    v += i == 0 ? old[0] : i == 1 ? old[1] : *o;
+                    *o = v;
+                    if (a.prep_x != nullptr) {
+                        a.prep_x[(size_t)tok * a.ldp + n] = __float2bfloat16_rn(v * a.prep_g[n]);
+                        sq = v * v;
+                    }
+                } else {
+                    if (a.epi == EPI_XIELU) {
+                        if (a.out_dtype == MF_DTYPE_BF16 && a.act_n == 0.0f && a.act_l == 0.0f) {
+                            const float p = fmaxf(v, 0.0f);
+                            v = a.act_p * p * p;
+                        } else {
+                            v = xielu_act(a, v);
+                        }
+                    }
+                    if (a.out_dtype == MF_DTYPE_F32) ((float*)a.out)[(size_t)tok * a.ldo + n] = v;
+                    else ((__nv_bfloat16*)a.out)[(size_t)tok * a.ldo + n] = __float2bfloat16_rn(v);
+                }
+            }
+            if (a.prep_x != nullptr) {
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+                if ((lane & 7) == 0 && idx < work) sq_s[tok * f.row_tiles + (row >> 3)] = sq;
+            }
+        }
+        if (a.prep_x != nullptr) {
+            __syncthreads();
+            if (tid < my_tokens) {
+                const int tok = rank + tid * f.cluster;
+                float sum = 0.0f;
+                for (int r = 0; r < f.row_tiles; ++r) sum += sq_s[tok * f.row_tiles + r];
+                a.prep_ssq[(size_t)group * a.M + tok] = sum;
+            }
+        }
+    }
+    __syncwarp();
+    if (f.cluster > 1) cluster_barrier();                            // nobody reads this CTA's sums any more
 }
 
 // What a wait that runs out does, shown without a product around it: one thread waits, with
@@ -1311,6 +1597,80 @@ extern "C" long long mf_gemm_tc_workspace_floats(int M, int N, int K, int epi) {
     return s > 1 ? (long long)s * M * N : 0;
 }
 
+// How gemm_few_kernel cuts a product, or groups 0: another kernel takes it.
+struct FewPlan { int row_tiles, warp_units, tok_stride, depth, cluster, groups; size_t smem; };
+static int g_few_mode = 1;                // 0 never (measurement, tests of the other kernels), 1 where the rule says so
+extern "C" void mf_gemm_few_mode(int mode) { g_few_mode = mode; }
+static FewPlan few_plan(int M, int N, int K) {
+    FewPlan p = {0, 0, 0, 0, 0, 0, 0};
+    if (g_few_mode == 0 || M < 1 || M > FEW_MAX_M || N < 1 || K < 1) return p;
+    if ((long long)N * K * 2 > ((long long)FEW_LIMIT_MB << 20)) return p;
+    const int units = (K + 63) / 64, tiles = (N + 7) / 8, sms = sm_count();
+    for (int cluster = 1; cluster <= 4; cluster *= 2) {
+        const int slots = cluster == 4 ? (sms - 16) / 4 : sms / cluster;       // clusters that fit at once
+        const int rt = (tiles + slots - 1) / slots, wu = (units + cluster * FEW_WARPS - 1) / (cluster * FEW_WARPS);
+        const int stride = 8 * (rt | 1);
+        const size_t fixed = sizeof(float) * ((size_t)FEW_WARPS * M * stride + 16 + (size_t)M * rt +
+                                              (cluster > 1 ? (size_t)M * 8 * rt : 0)) + (size_t)FEW_WARPS * wu * M * 128;
+        const int depths[] = {2, 4, 6};
+        int depth = 0;
+        for (int d : depths) {
+            if (depth > 0 && fixed + (size_t)FEW_WARPS * d * 1024 > FEW_BUDGET) break;
+            depth = d;
+            if (d >= rt * wu) break;
+        }
+        const int groups = (tiles + rt - 1) / rt;
+        if (fixed + (size_t)FEW_WARPS * depth * 1024 > FEW_BUDGET) continue;
+        // K is cut between CTAs only where one CTA's share of the tokens does not fit, or where the rows
+        // alone leave a quarter of the SMs without work and K is long
+        const bool idle = groups * cluster * 4 < sms * 3 && wu > 4;
+        if (p.groups == 0 || !idle) {
+            p.row_tiles = rt; p.warp_units = wu; p.tok_stride = stride; p.depth = depth; p.cluster = cluster;
+            p.groups = groups; p.smem = fixed + (size_t)FEW_WARPS * depth * 1024;
+        }
+        if (!idle) break;
+    }
+    return p;
+}
+// Column groups of a product of these sizes on gemm_few_kernel, 0: another kernel takes it.
+extern "C" int mf_gemm_few_groups(int M, int N, int K) { return few_plan(M, N, K).groups; }
+
+template <int NT, int DEPTH>
+static int launch_few(const FewPlan& p, const FewArgs& f, const GemmArgs& a, cudaStream_t stream) {
+    static bool configured[64] = {false};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MF_ERR_UNSUPPORTED;
+    if (!configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<NT, DEPTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_BUDGET);
+        if (e != cudaSuccess) return (int)e;
+        configured[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.groups * p.cluster);
+    cfg.blockDim = dim3(FEW_THREADS);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = p.cluster;
+    attrs[1].val.clusterDim.y = 1;
+    attrs[1].val.clusterDim.z = 1;
+    cfg.attrs = mf_pdl_enabled() ? attrs : attrs + 1;
+    cfg.numAttrs = (mf_pdl_enabled() ? 1 : 0) + (p.cluster > 1 ? 1 : 0);
+    cudaLaunchKernelEx(&cfg, gemm_few_kernel<NT, DEPTH>, f, a);
+    return MF_LAUNCH_CHECK();
+}
+template <int NT>
+static int launch_few_depth(const FewPlan& p, const FewArgs& f, const GemmArgs& a, cudaStream_t stream) {
+    switch (p.depth) {
+        case 2: return launch_few<NT, 2>(p, f, a, stream);
+        case 4: return launch_few<NT, 4>(p, f, a, stream);
+        default: return launch_few<NT, 6>(p, f, a, stream);
+    }
+}
+
 // What the caller may fold into a product (all null / zero: a plain product).
 struct FusedNorm {
     const float* row_ssq;     // consumer: sums of squares [ssq_parts][M] of the norm whose x' this product reads
@@ -1335,6 +1695,7 @@ static int pair_mode_on() {
 // the product in the ordinary way and runs the norm as a kernel).
 extern "C" int mf_gemm_tc_prep_parts(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
+    if (const int groups = few_plan(M, N, K).groups) return groups;
     int nt, splits;
     mf_gemm_tc_plan(M, N, K, EPI_ACCUM, &nt, &splits);
     const int kblocks = (K + TILE_K - 1) / TILE_K;
@@ -1370,9 +1731,12 @@ static int gemm_tc_impl(const void* x, long long ldx, const void* w, long long l
     if (prep && mf_gemm_tc_prep_parts(M, N, K) == 0) return MF_ERR_UNSUPPORTED;
     int nt, splits;
     mf_gemm_tc_plan(M, N, K, epi, &nt, &splits);
-    if (splits > 1 && workspace == nullptr && !prep) return MF_ERR_ARGUMENT;
+    // (a caller that wants the K splits for its next kernel gets them from the kernel that splits)
+    const FewPlan few = deferred == nullptr ? few_plan(M, N, K) : FewPlan{0, 0, 0, 0, 0, 0, 0};
+    if (splits > 1 && workspace == nullptr && !prep && few.groups == 0) return MF_ERR_ARGUMENT;
     CUtensorMap mw, mx;
-    if (int e = weight_map(&mw, w, N, K, ldw)) return e;
+    if (few.groups == 0)
+        if (int e = weight_map(&mw, w, N, K, ldw)) return e;
     GemmArgs a = {};
     a.out = out; a.partial = nullptr; a.bias = bias; a.status = status; a.ldo = ldo;
     a.M = M; a.N = N; a.K = K; a.out_dtype = out_dtype; a.kblocks_per_split = 0; a.epi = epi;
@@ -1381,6 +1745,11 @@ static int gemm_tc_impl(const void* x, long long ldx, const void* w, long long l
         a.row_ssq = f->row_ssq; a.ssq_parts = f->ssq_parts; a.ssq_width = f->ssq_width; a.ssq_eps = f->ssq_eps;
         a.prep_x = f->prep_x; a.ldp = f->ldp; a.prep_g = f->prep_g; a.prep_ssq = f->prep_ssq;
         a.act_p = f->act_p; a.act_n = f->act_n; a.act_l = f->act_l;
+    }
+    if (few.groups != 0) {
+        const FewArgs fa = {(const __nv_bfloat16*)w, (const __nv_bfloat16*)x, ldw, ldx, few.row_tiles,
+                            few.warp_units, few.tok_stride, few.cluster};
+        return M <= 8 ? launch_few_depth<1>(few, fa, a, stream) : launch_few_depth<2>(few, fa, a, stream);
     }
     if (pair_mode_on() && M >= 256 && splits == 1) {
         if (a.row_ssq != nullptr) return MF_ERR_UNSUPPORTED;     // the CTA-pair kernel applies no row scale

@@ -244,7 +244,7 @@ def _sig_attention_sink(lib: ctypes.CDLL) -> None:
 
     lib.mf_sink_decode_plan.argtypes = [c_int, c_int, c_int, c_void_p, c_void_p]
     lib.mf_sink_attention_decode.argtypes = ([c_void_p] * 6 + [c_int, c_int] + [c_void_p] * 4 +
-                                             [c_int] * 8 + [c_float, c_int, c_void_p, c_float, c_int,
+                                             [c_int] * 8 + [c_float, c_int, c_void_p, c_float, c_int, c_int,
                                                             c_void_p])
 
 
@@ -289,6 +289,9 @@ def _sig_gemm_tc(lib: ctypes.CDLL) -> None:
     lib.mf_gemm_tc_gated.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong,
                                      c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p]
     lib.mf_gemm_tc_prep_parts.argtypes = [c_int, c_int, c_int]
+    lib.mf_gemm_few_groups.argtypes = [c_int, c_int, c_int]
+    lib.mf_gemm_few_mode.argtypes = [c_int]
+    lib.mf_gemm_few_mode.restype = None
     lib.mf_wait_probe.argtypes = [c_void_p, ctypes.c_uint, c_ulonglong, c_void_p, c_void_p]
 
 
@@ -660,6 +663,26 @@ def gemm_pair_group_m(group_m: int) -> None:
     _lib("gemm_tc").mf_gemm_pair_group_m(int(group_m))
 
 
+_FEW: dict = {}
+
+
+def gemm_few_groups(m: int, n: int, k: int) -> int:
+    """Column groups that the kernel for a handful of tokens cuts a product of these sizes into, 0 where another
+    kernel takes it (a function of the sizes only).  It completes its sums: there are no K splits to add."""
+    key = (m, n, k)
+    got = _FEW.get(key)
+    if got is None:
+        got = _FEW[key] = int(_lib("gemm_tc").mf_gemm_few_groups(m, n, k))
+    return got
+
+
+def gemm_few_mode(mode: int) -> None:
+    """0: the kernel for a handful of tokens takes no product; 1: those its rule names (the default)."""
+    _lib("gemm_tc").mf_gemm_few_mode(int(mode))
+    _FEW.clear()
+    _PREP_PARTS.clear()
+
+
 def _gemm_tc_shape(m: int, n: int, k: int, epi: int) -> tuple[int, int, int]:
     """(token tile, K splits, workspace floats) of a product of these sizes."""
     key = (m, n, k, epi)
@@ -689,7 +712,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out:
     if bias is not None and bias.numel() != n:
         raise KernelError("gemm: bias has the wrong length")
     lib = _lib("gemm_tc")
-    need = _gemm_tc_shape(m, n, k, epi & 0xff)[2]
+    need = 0 if gemm_few_groups(m, n, k) else _gemm_tc_shape(m, n, k, epi & 0xff)[2]
     ws = torch.empty(need, dtype=torch.float32, device=x.device) if need else None
     _check(lib.mf_gemm_tc(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), _f32(bias, "bias"),
                           out.data_ptr(), out.stride(0), dtype_code(out.dtype), m, n, k, epi,
@@ -823,7 +846,7 @@ def gemm_tc_fused(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
                 or prep_ssq.shape != (parts, m)):
             raise KernelError("gemm: the next norm's tensors have the wrong shapes")
     lib = _lib("gemm_tc")
-    need = _gemm_tc_shape(m, n, k, epi & 0xff)[2]
+    need = 0 if not defer and gemm_few_groups(m, n, k) else _gemm_tc_shape(m, n, k, epi & 0xff)[2]
     ws = None
     if need and prep_x is None:
         ws = torch.empty(need, dtype=torch.float32, device=x.device)
@@ -2143,10 +2166,12 @@ def sink_attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
                           r1: Optional[torch.Tensor], r2: Optional[torch.Tensor], n_heads: int,
                           n_kv: int, head_dim: int, value_dim: int, window: int, chunk: int,
                           sink: bool, scale: float, reach_keys: int,
-                          sink_logit: Optional[torch.Tensor] = None, softcap: float = 0.0, keep_first: int = 0) -> None:
+                          sink_logit: Optional[torch.Tensor] = None, softcap: float = 0.0, keep_first: int = 0,
+                          old_keys_final: bool = False) -> None:
     """Every row of ``q`` a query at its own position over the paged cache, on tensor cores
     (bfloat16; the query heads of a key/value head in blocks of up to 16).  ``reach_keys``: the most keys a query
-    sees (its chunk or window, or the longest sequence's length)."""
+    sees (its chunk or window, or the longest sequence's length).  ``old_keys_final``: every row is its sequence's
+    only new token in this step (keys below its position may be read before the kernel before ends)."""
     rows = q.shape[0]
     if q.dtype != torch.bfloat16 or out.shape != (rows, n_heads * value_dim):
         raise KernelError("sink_attention_decode: bfloat16 only, out [rows, heads * value size]")
@@ -2163,8 +2188,8 @@ def sink_attention_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
         _i32(row_pos, "row_pos"), _i32(page_table, "page_table"), int(table_stride), int(ring),
         _ptr(out, "out"), _f32(partial, "partial"), _f32(r1, "r1"), _f32(r2, "r2"), rows, n_heads,
         n_kv, head_dim, value_dim, int(window), int(chunk), 1 if sink else 0, float(scale),
-        int(reach_keys), _f32(sink_logit, "sink_logit"), float(softcap), int(keep_first), _stream()),
-        "sink_attention_decode", 2 if splits > 1 else 1)
+        int(reach_keys), _f32(sink_logit, "sink_logit"), float(softcap), int(keep_first),
+        1 if old_keys_final else 0, _stream()), "sink_attention_decode", 2 if splits > 1 else 1)
 
 
 def latent_decode_supported(dtype: torch.dtype, key_dim: int, value_dim: int) -> bool:

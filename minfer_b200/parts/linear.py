@@ -70,8 +70,9 @@ class Linear:
         from ..kernels import gemm
         from .base import Pending
         if (x.dtype != torch.bfloat16 or self.weight.dtype != torch.bfloat16 or x.shape[0] == 0
-                or not gemm.use_tensor_cores()):
-            return None
+                or not gemm.use_tensor_cores()
+                or K.gemm_few_groups(x.shape[0], self.out_features, self.in_features)):
+            return None                # (the kernel for a handful of tokens completes its sums)
         if row_scale is not None:
             if not K.gemm_tc_supported(x, self.weight):
                 return None

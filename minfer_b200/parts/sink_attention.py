@@ -78,7 +78,7 @@ def decode_reach(spec: ScoreSpec, max_end: int) -> int:
     tile's worth for the two stretches' ragged ends), or the longest sequence."""
     reach = spec.reach()
     if reach > 0:
-        return reach
+        return min(reach, max_end)
     if spec.window > 0 and spec.keep_first > 0:
         return min(max_end, spec.window + spec.keep_first + 64)
     return max_end
@@ -147,7 +147,7 @@ def scored_attention(spec: ScoreSpec, q: torch.Tensor, k_step: Optional[torch.Te
                                 cache.page_table, cache.table_stride, cache.ring, o, r1, r2, nh,
                                 nk, hd, vd, spec.window, spec.chunk, spec.sink, spec.scale,
                                 decode_reach(spec, ctx.max_end), sink_logit=sl, softcap=cap,
-                                keep_first=keep)
+                                keep_first=keep, old_keys_final=ctx.single_token)
         return
     K.sink_attention_paged(q, cache.k, cache.v, ctx.token_row, ctx.positions, cache.page_table,
                            cache.table_stride, cache.ring, o, r1, r2, nh, nk, hd, vd, spec.window,
