@@ -6,13 +6,20 @@
 // (src/graph/ops.rs:132-136; out[t*od+o] = dot(w[o], x[t]) + bias[o],
 // src/graph/cpu_backend.rs:214-247).
 //
-// Each output element is summed over k in ascending order by one thread, whatever M is and
-// wherever the row lies in the batch, so a token's result never depends on its neighbours.
+// Each output element is summed over k in ascending order by one thread; from K = 2,048 on four
+// stretches of k are, and their sums are added in order (`f32_stretch`, a function of K only).  Neither M
+// nor the place of a row in the batch matters, so a token's result never depends on its neighbours.
 // All three kernels below keep that order, so they give the same bits:
 //   gemm_f32_few_kernel    up to 16 rows, float32 operands on 16-byte rows
 //   gemm_f32_tile_kernel   more rows, the same operands
 //   gemm_simt_kernel       everything else (bfloat16 on either side, rows off 16 bytes)
 #include "common.cuh"
+
+// k of a stretch: K itself, or a quarter of it in whole 128s (always four stretches).  A product of few
+// columns and a long K has too few tiles for the SMs while one thread walks all of K; as a cluster of four
+// CTAs a tile it does not.
+__host__ __device__ constexpr int f32_stretch(int K) { return K < 2048 ? K : ((K + 511) / 512) * 128; }
+#define F32_STRETCHES 4
 
 #define BM 64
 #define BN 64
@@ -36,7 +43,18 @@ gemm_simt_kernel(const TA* A, const TW* __restrict__ W, const float* __restrict_
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
 
+    const int stretch = f32_stretch(K);
+    float done[4][4];                                // the stretches before this one
     for (int k0 = 0; k0 < K; k0 += BK) {
+        if (k0 > 0 && k0 % stretch == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    done[i][j] = k0 == stretch ? acc[i][j] : done[i][j] + acc[i][j];
+                    acc[i][j] = 0.0f;
+                }
+        }
         // 64 rows x 16 k per operand = 1024 elements, 4 per thread; k fastest for coalescing
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -74,7 +92,7 @@ gemm_simt_kernel(const TA* A, const TW* __restrict__ W, const float* __restrict_
         for (int j = 0; j < 4; ++j) {
             const int n = n0 + tx * 4 + j;
             if (n >= N) continue;
-            float v = acc[i][j];
+            float v = stretch < K ? done[i][j] + acc[i][j] : acc[i][j];
             if (bias) v += bias[n];
             TC* c = C + (size_t)m * ldc + n;
             if (accumulate) v += to_f32(*c);
@@ -113,6 +131,21 @@ __device__ __forceinline__ float4 load16(const float* p) {
     return v;
 }
 
+// every thread of the cluster's CTAs comes here; writes to shared memory before it are seen after it
+__device__ __forceinline__ void cluster_wait_all() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 load16_of_rank(unsigned smem, int rank) {
+    float4 v;
+    asm volatile(
+        "{\n .reg .b32 ra;\n mapa.shared::cluster.u32 ra, %4, %5;\n"
+        " ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n}\n"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(smem), "r"(rank) : "memory");
+    return v;
+}
+
 template <int ROWS, int THREADS, int BKT>
 __device__ __forceinline__ void f32_tile_fetch(const float* src, long long ld, int row0, int rows,
                                                int k0, int K, float4* held) {
@@ -144,17 +177,22 @@ struct F32Tile {
     static constexpr int THREADS = 32 * WARPS_N * (BM_ / (4 * TM));
 };
 
-template <int BM_, int BN_, int TM, int TN, int BKT, int AHEAD>
+// SPLIT: a cluster of four CTAs has a tile, CTA r the stretch r of k; they add their sums in order of the
+// stretches through distributed shared memory, each a quarter of the tile's rows.
+template <int BM_, int BN_, int TM, int TN, int BKT, int AHEAD, bool SPLIT>
 __global__ void __launch_bounds__(F32Tile<BM_, BN_, TM, TN>::THREADS,
                                   (AHEAD == 1 ? 512 : 384) / F32Tile<BM_, BN_, TM, TN>::THREADS)
 gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ bias, float* C,
-                     int M, int N, int K, long long lda, long long ldw,
+                     int M, int N, int K_all, long long lda, long long ldw,
                      long long ldc, int accumulate) {
     constexpr int THREADS = F32Tile<BM_, BN_, TM, TN>::THREADS;
     constexpr int WARPS_N = F32Tile<BM_, BN_, TM, TN>::WARPS_N;
     constexpr int FA = BM_ * (BKT / 4) / THREADS, FW = BN_ * (BKT / 4) / THREADS;
-    __shared__ __align__(16) float As[2][BKT][BM_];
-    __shared__ __align__(16) float Ws[2][BKT][BN_];
+    __shared__ __align__(16) float pool[2 * BKT * (BM_ + BN_)];
+    float (*As)[BKT][BM_] = reinterpret_cast<float (*)[BKT][BM_]>(pool);
+    float (*Ws)[BKT][BN_] = reinterpret_cast<float (*)[BKT][BN_]>(pool + 2 * BKT * BM_);
+    const int k_first = SPLIT ? (int)blockIdx.z * f32_stretch(K_all) : 0;
+    const int K = SPLIT ? min(K_all, k_first + f32_stretch(K_all)) : K_all;       // this CTA's end
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ty = (warp / WARPS_N) * 4 * TM + (lane >> 3) * 4;     // + 16 per group of 4 rows
     const int tx = (warp % WARPS_N) * 8 * TN + (lane & 7) * 4;      // + 32 per group of 4 columns
@@ -169,8 +207,8 @@ gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ b
     pdl_prologue();
     float4 ha[AHEAD][FA], hw[AHEAD][FW];              // the next AHEAD tiles, on their way
     auto fetch = [&](int t, int set) {
-        f32_tile_fetch<BM_, THREADS, BKT>(A, lda, m0, M, t * BKT, K, ha[set]);
-        f32_tile_fetch<BN_, THREADS, BKT>(W, ldw, n0, N, t * BKT, K, hw[set]);
+        f32_tile_fetch<BM_, THREADS, BKT>(A, lda, m0, M, k_first + t * BKT, K, ha[set]);
+        f32_tile_fetch<BN_, THREADS, BKT>(W, ldw, n0, N, k_first + t * BKT, K, hw[set]);
     };
     auto put = [&](int t, int set) {
         f32_tile_put<BM_, THREADS, BKT>(As[t & 1], ha[set]);
@@ -203,7 +241,7 @@ gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ b
         }
     };
     // tiles beyond the last are fetched as zeros (no load) and never multiplied
-    const int tiles = (K + BKT - 1) / BKT;
+    const int tiles = (K - k_first + BKT - 1) / BKT;
     fetch(0, 0);
     put(0, 0);
     if (AHEAD == 2) fetch(1, 1);
@@ -217,6 +255,56 @@ gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ b
             put(t + u + 1, (u + 1) % AHEAD);
             __syncthreads();
         }
+    }
+    if (SPLIT) {
+        // a group of columns at a time: BM_ rows x COLS sums of every CTA, its own in `pool`
+        constexpr int COLS = 32 * WARPS_N, QUADS = COLS / 4, MINE = BM_ / F32_STRETCHES;
+        static_assert(BM_ * COLS <= 2 * BKT * (BM_ + BN_), "a group of columns fits the tiles' memory");
+        const int own = (int)blockIdx.z * MINE;
+#pragma unroll
+        for (int h = 0; h < TN / 4; ++h) {
+            if (h > 0) cluster_wait_all();                            // the group before has been read
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                const unsigned long long p0 = acc[i][h * 2], p1 = acc[i][h * 2 + 1];
+                *reinterpret_cast<float4*>(pool + (ty + (i >> 2) * 16 + (i & 3)) * COLS +
+                                           (warp % WARPS_N) * 32 + (lane & 7) * 4) =
+                    make_float4(__uint_as_float((unsigned)p0), __uint_as_float((unsigned)(p0 >> 32)),
+                                __uint_as_float((unsigned)p1), __uint_as_float((unsigned)(p1 >> 32)));
+            }
+            cluster_wait_all();
+            for (int idx = threadIdx.x; idx < MINE * QUADS; idx += THREADS) {
+                const int r = own + idx / QUADS, q = idx % QUADS;
+                const int m = m0 + r, n = n0 + (q / 8) * 8 * TN + h * 32 + (q % 8) * 4;
+                const unsigned at = (unsigned)__cvta_generic_to_shared(pool + r * COLS + q * 4);
+                float v[4];
+#pragma unroll
+                for (int z = 0; z < F32_STRETCHES; ++z) {
+                    const float4 p = load16_of_rank(at, z);
+                    v[0] = z == 0 ? p.x : v[0] + p.x;
+                    v[1] = z == 0 ? p.y : v[1] + p.y;
+                    v[2] = z == 0 ? p.z : v[2] + p.z;
+                    v[3] = z == 0 ? p.w : v[3] + p.w;
+                }
+                if (m >= M) continue;
+                float* c = C + (size_t)m * ldc + n;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (n + j >= N) break;
+                    if (bias != nullptr) v[j] += bias[n + j];
+                    if (accumulate) v[j] += c[j];
+                }
+                if (n + 3 < N && ((((uintptr_t)c) & 15) == 0)) {
+                    *reinterpret_cast<float4*>(c) = make_float4(v[0], v[1], v[2], v[3]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (n + j < N) c[j] = v[j];
+                }
+            }
+        }
+        cluster_wait_all();                                           // nobody reads this CTA's sums any more
+        return;
     }
 #pragma unroll
     for (int h = 0; h < TN / 4; ++h) {
@@ -300,10 +388,18 @@ gemm_f32_few_kernel(const float* A, const float* W, const float* __restrict__ bi
     };
     const int chunks = (K + T::KC - 1) / T::KC;
     fetch(0);
-    float acc[RT];
+    float acc[RT], done[RT];                                         // done: the stretches before this one
 #pragma unroll
     for (int i = 0; i < RT; ++i) acc[i] = 0.0f;
+    const int stretch = f32_stretch(K);
     for (int c = 0; c < chunks; ++c) {
+        if (c > 0 && c * T::KC % stretch == 0) {
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                done[i] = c * T::KC == stretch ? acc[i] : done[i] + acc[i];
+                acc[i] = 0.0f;
+            }
+        }
         if (c + 1 < chunks) {
             fetch(c + 1);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -333,7 +429,7 @@ gemm_f32_few_kernel(const float* A, const float* W, const float* __restrict__ bi
     for (int i = 0; i < RT; ++i) {
         const int m = grp + 4 * i;
         if (m >= M) continue;
-        float v = acc[i];
+        float v = stretch < K ? done[i] + acc[i] : acc[i];
         if (bias != nullptr) v += bias[n];
         float* c = C + (size_t)m * ldc + n;
         if (accumulate) v += *c;
@@ -344,8 +440,28 @@ gemm_f32_few_kernel(const float* A, const float* W, const float* __restrict__ bi
 template <int BM_, int BN_, int TM, int TN, int BKT, int AHEAD>
 static void launch_f32_tile(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
                             long long lda, long long ldw, long long ldc, int accumulate, cudaStream_t stream) {
-    mf_launch(gemm_f32_tile_kernel<BM_, BN_, TM, TN, BKT, AHEAD>, dim3((M + BM_ - 1) / BM_, (N + BN_ - 1) / BN_),
-              dim3(F32Tile<BM_, BN_, TM, TN>::THREADS), 0, stream, A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate);
+    const dim3 grid((M + BM_ - 1) / BM_, (N + BN_ - 1) / BN_, f32_stretch(K) < K ? F32_STRETCHES : 1);
+    const dim3 block(F32Tile<BM_, BN_, TM, TN>::THREADS);
+    if (grid.z == 1) {
+        mf_launch(gemm_f32_tile_kernel<BM_, BN_, TM, TN, BKT, AHEAD, false>, grid, block, 0, stream, A, W, bias, C, M,
+                  N, K, lda, ldw, ldc, accumulate);
+        return;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = stream;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeClusterDimension;
+    attrs[0].val.clusterDim.x = 1;
+    attrs[0].val.clusterDim.y = 1;
+    attrs[0].val.clusterDim.z = F32_STRETCHES;
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = mf_pdl_enabled() ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<BM_, BN_, TM, TN, BKT, AHEAD, true>, A, W, bias, C, M, N, K, lda,
+                       ldw, ldc, accumulate);
 }
 
 // The tile of a float32 product of more than 16 rows (an index into `tiles`; -1: the general kernel, whose
@@ -357,7 +473,7 @@ static void launch_f32_tile(const float* A, const float* W, const float* bias, f
 // 1.1 % (21 %) of 109 products back to back; 66 others 0.3 % (6 %) and 0.7 % (24 %).  us, 128 x 128 / 64 x 64 /
 // 32 x 64, norm and product: 200 x 4,096 x 2,048 373 / 224 / 136, 385 x 9,728 x 896 241 / 194 / 205,
 // 385 x 896 x 4,864 467 / 276 / 242, 1,600 x 8,448 x 2,048 1,086 / 1,243 / 1,471.
-extern "C" int mf_gemm_f32_tile(int M, int N, int sms) {
+static int f32_tile(int M, int N, int sms, int stretches) {
     static const struct { int bm, bn; double few, shared; } tiles[] = {
         {128, 128, 6.4, 3.3}, {64, 64, 3.9, 1.0}, {32, 64, 1.8, 0.58}};
     int best = -1;
@@ -366,12 +482,13 @@ extern "C" int mf_gemm_f32_tile(int M, int N, int sms) {
         const long long nt = ((long long)N + tiles[i].bn - 1) / tiles[i].bn;
         const long long mt = ((long long)M + tiles[i].bm - 1) / tiles[i].bm;
         if (nt > 65535) continue;                                    // the grid's second dimension
-        const double share = (double)((nt * mt + sms - 1) / sms) * tiles[i].shared;
+        const double share = (double)((nt * mt * stretches + sms - 1) / sms) * tiles[i].shared;
         const double cost = share > tiles[i].few ? share : tiles[i].few;
         if (best < 0 || cost < least) { best = i; least = cost; }
     }
     return best;
 }
+extern "C" int mf_gemm_f32_tile(int M, int N, int sms) { return f32_tile(M, N, sms, 1); }
 
 // Float32 operands whose rows start on 16 bytes; false: the general kernel has to run.
 static bool launch_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
@@ -388,7 +505,8 @@ static bool launch_f32(const float* A, const float* W, const float* bias, float*
 #undef MF_FEW
         return true;
     }
-    const int best = mf_gemm_f32_tile(M, N, mf_sm_count());
+    // (four CTAs a tile, each with a quarter of the work: the same comparison at four times the CTAs)
+    const int best = f32_tile(M, N, mf_sm_count(), f32_stretch(K) < K ? F32_STRETCHES : 1);
     switch (best) {
         case 0: launch_f32_tile<128, 128, 8, 8, 16, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;
         case 1: launch_f32_tile<64, 64, 4, 8, 32, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;

@@ -1,0 +1,38 @@
+"""Float32 products whose K is cut into four stretches (2,048 and more): every kernel adds them in the same
+order, so a row has the same bits in all of them."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [5, 64, 200, 896, 5000])
+@pytest.mark.parametrize("k", [2044, 2048, 2052, 2180, 4864, 8448])
+def test_rows_have_the_same_bits_in_every_kernel(n, k):
+    """1 to 16 rows (a warp per 8 columns), more (32 x 64, 64 x 64 and 128 x 128 tiles, a cluster of CTAs a
+    tile from K = 2,048 on) and rows off 16 bytes (the general kernel); bias, accumulation, ragged edges."""
+    from minfer_b200.kernels import api as K
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    m = 700
+    x = torch.randn(m, k, generator=g, device="cuda")
+    w = torch.randn(n, k, generator=g, device="cuda") * k ** -0.5
+    bias, old = torch.randn(n, generator=g, device="cuda"), torch.randn(m, n, generator=g, device="cuda")
+    want = x.double() @ w.double().t() + bias.double()
+
+    def product(rows, accumulate):
+        out = old[rows].clone()
+        K.gemm_simt(x[rows].contiguous(), w, bias, out, accumulate)
+        return out
+
+    whole = {a: product(slice(0, m), a) for a in (False, True)}
+    # 32-bit sums of k products: 2^-24 a step, in four chains of at most k / 4 + 128
+    assert float((whole[False].double() - want).abs().max()) < 2 ** -24 * (k / 4 + 131) * float(want.abs().max())
+    for rows in (slice(0, 1), slice(3, 7), slice(5, 13), slice(100, 116), slice(1, 41), slice(200, 400)):
+        for a in (False, True):
+            assert torch.equal(product(rows, a), whole[a][rows]), (rows, a)
+    # rows that do not start on 16 bytes
+    odd_x, odd_w = torch.zeros(40, k + 1, device="cuda"), torch.zeros(n, k + 1, device="cuda")
+    odd_x[:, :k], odd_w[:, :k] = x[:40], w
+    out = torch.empty(40, n, device="cuda")
+    K.gemm_simt(odd_x[:, :k], odd_w[:, :k], bias, out, False)
+    assert torch.equal(out, whole[False][:40])
