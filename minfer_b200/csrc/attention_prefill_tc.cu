@@ -224,7 +224,7 @@ template <int HD, bool PAGED, bool MOD>
 __global__ void __launch_bounds__(FA_THREADS, 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const FaArgs a) {
-    pdl_prologue();
+    pdl_wait();
     constexpr int NB = HD / 64;                         // 64-column blocks per row
     constexpr int BLOCK = 128 * 128;                    // bytes of a [128 rows][64 cols] block
     constexpr int T_BYTES = NB * BLOCK;                 // a [128 rows][HD] tile
@@ -318,6 +318,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     }
     fa_fence_before();
     __syncthreads();
+    // The next kernel may start from here on, not earlier: a product's CTA allocates tensor memory before it
+    // waits, and on an SM it shares with this one (head size 64) could leave none.
+    pdl_launch_dependents();
     fa_fence_after();
     const uint32_t tmem = *tmem_slot;
 

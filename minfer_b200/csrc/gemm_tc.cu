@@ -1298,8 +1298,6 @@ template <int NT, int STAGES, bool DUAL>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  const GemmArgs a, int tiles_m, int tiles_n, int group_m, int total_tiles) {
-    pdl_launch_dependents();
-    pdl_wait();
     constexpr int HALF_B = (NT / 2) * TILE_K * 2;            // this CTA's half of one token tile
     constexpr int B_BYTES = (DUAL ? 2 : 1) * HALF_B;
     constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -1320,7 +1318,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int kblocks = (a.K + TILE_K - 1) / TILE_K;
 
+    // The barriers, and the weights of the first stages, which no kernel of the step writes: before the wait
+    // for the kernel before.
     if (tid == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(smem_u32(&full[s]), 1);
             mbar_init(smem_u32(&empty[s]), 1);
@@ -1333,6 +1335,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    __syncthreads();
+    cluster_sync_all();                                       // both CTAs' barriers exist
+    const int early = min(STAGES, kblocks);                   // stages of the first tile filled ahead
+    if (warp == 0 && elect_one()) {
+        int mi, ni;
+        pair_tile_at(pair, tiles_m, tiles_n, group_m, mi, ni);
+        const bool two = DUAL && mi * M_STEP + NT < a.M;
+        for (int s = 0; s < early; ++s) {
+            if (rank == 0) mbar_expect_tx(smem_u32(&full[s]), 2 * (A_BYTES + (two ? 2 : 1) * HALF_B));
+            tma_load_2d_pair(smem_u32(smem + s * STAGE_BYTES), &map_w, s * TILE_K, ni * 256 + (int)rank * TILE_N,
+                             smem_u32(&full[s]) & PEER_BIT_MASK);
+        }
+    }
+    __syncwarp();
+    pdl_wait();
+    // (tensor memory only now: a kernel before may still have to allocate its own)
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)TMEM_COLS) : "memory");
@@ -1340,7 +1358,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();                                       // both CTAs' barriers exist
+    cluster_sync_all();                                       // both CTAs have their tensor memory
+    // ... and only now the next kernel may come onto this SM, which may allocate before it waits
+    pdl_launch_dependents();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
@@ -1356,12 +1376,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             for (int kb = 0; kb < kblocks; ++kb, ++it) {
                 const int s = it % STAGES;
                 const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-                if (!mbar_wait(smem_u32(&empty[s]), ph ^ 1u, abort_flag)) { ok = false; break; }
                 const uint32_t leader_full = smem_u32(&full[s]) & PEER_BIT_MASK;
-                if (rank == 0)
-                    mbar_expect_tx(smem_u32(&full[s]), 2 * (A_BYTES + (two ? 2 : 1) * HALF_B));
                 const uint32_t dst = smem_u32(smem + s * STAGE_BYTES);
-                tma_load_2d_pair(dst, &map_w, kb * TILE_K, n0 + (int)rank * TILE_N, leader_full);
+                if (it >= early) {
+                    if (!mbar_wait(smem_u32(&empty[s]), ph ^ 1u, abort_flag)) { ok = false; break; }
+                    if (rank == 0)
+                        mbar_expect_tx(smem_u32(&full[s]), 2 * (A_BYTES + (two ? 2 : 1) * HALF_B));
+                    tma_load_2d_pair(dst, &map_w, kb * TILE_K, n0 + (int)rank * TILE_N, leader_full);
+                }
                 tma_load_2d_pair(dst + A_BYTES, &map_x, kb * TILE_K, m0 + (int)rank * (NT / 2),
                                  leader_full);
                 if (two)
@@ -1520,7 +1542,7 @@ static int g_pair_dual = -1;              // 0 never, 1 where the model says so,
 // MINFER_B200_PAIR_DUAL or this call (tests compare the two forms bit for bit) sets the mode.
 extern "C" void mf_gemm_pair_dual_mode(int mode) { g_pair_dual = mode; }
 static PairPlan pair_plan(int M, int N, int K) {
-    static const int candidates[] = {256, 224, 208, 192, 160};
+    static const int candidates[] = {256, 224, 208, 192, 176, 160};
     if (g_pair_dual < 0) { const char* ev = getenv("MINFER_B200_PAIR_DUAL"); g_pair_dual = ev ? atoi(ev) : 1; }
     const int allow_dual = g_pair_dual;
     const double pairs = sm_count() / 2, tiles_n = (N + 255) / 256, kb = (K + TILE_K - 1) / TILE_K;
@@ -1761,6 +1783,7 @@ static int gemm_tc_impl(const void* x, long long ldx, const void* w, long long l
                 case 224: return launch_pair<224, 5, true>(mw, mx, a, stream);
                 case 208: return launch_pair<208, 5, true>(mw, mx, a, stream);
                 case 192: return launch_pair<192, 5, true>(mw, mx, a, stream);
+                case 176: return launch_pair<176, 5, true>(mw, mx, a, stream);
                 case 160: return launch_pair<160, 6, true>(mw, mx, a, stream);
                 default: return launch_pair<256, 4, true>(mw, mx, a, stream);
             }
@@ -1768,6 +1791,7 @@ static int gemm_tc_impl(const void* x, long long ldx, const void* w, long long l
             case 224: return launch_pair<224, 6, false>(mw, mx, a, stream);
             case 208: return launch_pair<208, 6, false>(mw, mx, a, stream);
             case 192: return launch_pair<192, 6, false>(mw, mx, a, stream);
+            case 176: return launch_pair<176, 6, false>(mw, mx, a, stream);
             case 160: return launch_pair<160, 6, false>(mw, mx, a, stream);
             default: return launch_pair<256, 6, false>(mw, mx, a, stream);
         }

@@ -33,7 +33,7 @@ def test_products_of_a_handful_of_tokens(m, n, k):
     from minfer_b200.kernels import api as K
     parts = K.gemm_few_groups(m, n, k)
     if parts == 0:
-        assert m * k > 60000                  # only tokens that do not fit shared memory are left to others
+        assert m > 8 or m * k > 60000         # what does not fit shared memory is left to the other kernels
         return
     x, w, bias, h0 = _operands(m, n, k, m + n + k)
     st = torch.zeros(1, dtype=torch.int32, device="cuda")
