@@ -963,6 +963,79 @@ norm_shift_vec_kernel(const float* x, const float* __restrict__ w,
     }
 }
 
+// the form for decoding, every sequence one token: float4 accesses, the weights read and the state's lines
+// asked for in L2 before the wait, everything else in one trip behind it (the general form made three and
+// went over the row twice); widths that are multiples of 4 up to 8 * blockDim
+template <typename TO, bool SPLITS>
+__global__ void __launch_bounds__(512)
+norm_shift_one_kernel(float* x, const float* partial, int n_partials, const float* __restrict__ bias, int n_tokens,
+                      const float* __restrict__ w, const float* __restrict__ shift, const int* __restrict__ positions,
+                      const int* __restrict__ token_row, const int* __restrict__ slots, float* state,
+                      TO* __restrict__ y, int width, float eps) {
+    pdl_launch_dependents();
+    __shared__ float scratch[33];
+    const int t = blockIdx.x;
+    const bool fresh = positions[t] == 0;               // nothing before: zeros
+    float4* st = reinterpret_cast<float4*>(state + (size_t)slots[token_row[t]] * width);
+    const int nv = width >> 2;
+    float4 g[2], sh[2], bv[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        bv[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < nv) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(st + i));
+            g[j] = reinterpret_cast<const float4*>(w)[i];
+            sh[j] = reinterpret_cast<const float4*>(shift)[i];
+            if (SPLITS && bias != nullptr) bv[j] = reinterpret_cast<const float4*>(bias)[i];
+        }
+    }
+    pdl_wait();
+    float4* xr = reinterpret_cast<float4*>(x + (size_t)t * width);
+    float4 row[2], prev[2];
+    float ss = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < nv) {
+            float4 v = xr[i];
+            prev[j] = fresh ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : st[i];
+            if (SPLITS) {
+                // every split's load is in flight at once; the sums keep the split order
+                const size_t plane = (size_t)n_tokens * width;
+                const float* pr = partial + (size_t)t * width;
+                float4 pv[16];
+#pragma unroll
+                for (int s = 0; s < 16; ++s)
+                    if (s < n_partials) pv[s] = reinterpret_cast<const float4*>(pr + (size_t)s * plane)[i];
+                v.x += bv[j].x; v.y += bv[j].y; v.z += bv[j].z; v.w += bv[j].w;
+#pragma unroll
+                for (int s = 0; s < 16; ++s)
+                    if (s < n_partials) { v.x += pv[s].x; v.y += pv[s].y; v.z += pv[s].z; v.w += pv[s].w; }
+                xr[i] = v;
+            }
+            row[j] = v;
+            ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss);
+            ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
+        }
+    }
+    ss = block_sum(ss, scratch);
+    const float scale = 1.0f / sqrtf(ss / (float)width + eps);
+    TO* yr = y + (size_t)t * width;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int i = threadIdx.x + j * blockDim.x;
+        if (i < nv) {
+            const float4 v = row[j], u = prev[j], gg = g[j], s4 = sh[j];
+            const float n0 = v.x * scale * gg.x, n1 = v.y * scale * gg.y;
+            const float n2 = v.z * scale * gg.z, n3 = v.w * scale * gg.w;
+            Pack4<TO>::store(yr + 4 * i, n0 + (u.x - n0) * s4.x, n1 + (u.y - n1) * s4.y,
+                             n2 + (u.z - n2) * s4.z, n3 + (u.w - n3) * s4.w);
+            st[i] = make_float4(n0, n1, n2, n3);
+        }
+    }
+}
+
 __global__ void norm_shift_save_kernel(const float* x, const float* __restrict__ w,
                                        const int* __restrict__ cu_seqlens,
                                        const int* __restrict__ slots, float* state,
@@ -1012,6 +1085,23 @@ extern "C" int mf_norm_shift(float* x, const float* partial, int n_partials, con
         mf_launch(norm_shift_save_kernel, dim3(n_rows), dim3(threads), 0, stream, (const float*)x, w,
                   cu_seqlens, slots, state, width, eps);
         return MF_LAUNCH_CHECK();
+    }
+    if (!multi && (width & 3) == 0 && width <= 8 * threads && n_partials <= 16 &&
+        (((uintptr_t)x | (uintptr_t)state | (uintptr_t)y | (uintptr_t)w | (uintptr_t)shift | (uintptr_t)bias |
+          (uintptr_t)partial) & 15) == 0) {
+#define MF_NORM_SHIFT_ONE(TO, SPLITS) \
+    mf_launch(norm_shift_one_kernel<TO, SPLITS>, dim3(n_tokens), dim3(threads), 0, stream, x, partial, n_partials, \
+              bias, n_tokens, w, shift, positions, token_row, slots, state, (TO*)y, width, eps)
+        if (out_dtype == MF_DTYPE_F32) {
+            if (n_partials > 0) MF_NORM_SHIFT_ONE(float, true); else MF_NORM_SHIFT_ONE(float, false);
+            return MF_LAUNCH_CHECK();
+        }
+        if (out_dtype == MF_DTYPE_BF16) {
+            if (n_partials > 0) MF_NORM_SHIFT_ONE(__nv_bfloat16, true);
+            else MF_NORM_SHIFT_ONE(__nv_bfloat16, false);
+            return MF_LAUNCH_CHECK();
+        }
+#undef MF_NORM_SHIFT_ONE
     }
 #define MF_NORM_SHIFT(TO, SPLITS) \
     mf_launch(norm_shift_kernel<TO, SPLITS>, dim3(n_tokens), dim3(threads), 0, stream, x, partial, \

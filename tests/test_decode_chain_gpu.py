@@ -125,3 +125,31 @@ def test_old_keys_read_early_are_the_same_keys(chunk, ring):
                                 old_keys_final=final)
         outs.append(out)
     assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("width", [4, 200, 2048, 4096, 4100, 30])
+@pytest.mark.parametrize("splits", [0, 1, 8, 16, 17])
+def test_norm_and_shift_of_one_token_a_row(width, splits):
+    """Widths inside and beyond the single-pass form, K splits up to and beyond those it adds, a row at
+    position 0, rows that share a state tensor, two steps one behind the other."""
+    from minfer_b200.kernels import api as K
+    g = torch.Generator(device="cuda").manual_seed(width + splits)
+    rows, eps = 5, 1e-5
+    slots, positions = _i32([6, 0, 3, 2, 5]), _i32([0, 4, 9, 100, 1])
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")            # noqa: E731
+    w, shift, state, bias = 1 + 0.1 * rand(width), rand(width), rand(7, width), rand(width)
+    ref_state = state.double().clone()
+    for step in range(2):
+        x = rand(rows, width)
+        part = rand(splits, rows, width) if splits else None
+        full = x.double() + (part.double().sum(0) + bias.double() if splits else 0.0)
+        pos = positions + step
+        y = torch.empty(rows, width, device="cuda")
+        K.norm_shift(x, w, shift, eps, pos, _i32(list(range(rows))), _i32(list(range(rows + 1))), slots, state, y,
+                     False, partial=part, bias=bias if splits else None)
+        n = full / torch.sqrt((full ** 2).mean(-1, keepdim=True) + eps) * w.double()
+        before = torch.where(pos[:, None] > 0, ref_state[slots.long()], torch.zeros_like(n))
+        _close(y, n + (before - n) * shift.double())
+        ref_state[slots.long()] = n
+        _close(state, ref_state)
+        _close(x, full)
