@@ -769,9 +769,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 //     (16 bytes) of a row where the fragments of two products would want 2 + 2 each.
 //   * A warp has DEPTH units (8 rows x 64 k, 1 KB) in flight, the first ones asked for BEFORE
 //     griddepcontrol.wait: weights are constant over the step.  Where a product's weights fit the
-//     rings of all CTAs they are on the chip when the kernel before ends; what lies beyond is asked
-//     for in L2.  A CTA takes half of an SM, so that the next product's CTA does this while this one
-//     computes.
+//     rings of all CTAs they are on the chip when the kernel before ends.
 //   * The tokens come after the wait, every lane's own fragments, all in flight together.  Where a
 //     CTA's share of them is too large, or rows alone leave SMs idle, a cluster of CTAs shares the
 //     rows and cuts K.
@@ -782,8 +780,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 #define FEW_THREADS (32 * FEW_WARPS)
 #define FEW_MAX_M 16
 #define FEW_BUDGET (112 * 1024)       // shared memory of a CTA
-#define FEW_LIMIT_MB 64
-#define FEW_L2 1
+#define FEW_MAX_BYTES (64ll << 20)     // of weights: beyond, the TMA ring streams as fast as memory gives
 
 struct FewArgs {
     const __nv_bfloat16* w;
@@ -809,7 +806,7 @@ __device__ __forceinline__ void few_mma(float* c, uint32_t a0, uint32_t a1, uint
 
 // NT: tokens in tiles of 8 (1 or 2 of them)
 template <int NT, int DEPTH>
-__global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const FewArgs f, const GemmArgs a) {
+__global__ void __launch_bounds__(FEW_THREADS, 1) gemm_few_kernel(const FewArgs f, const GemmArgs a) {
     extern __shared__ __align__(16) uint8_t few_smem[];
     pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -847,15 +844,6 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) gemm_few_kernel(const FewArgs 
     };
 #pragma unroll
     for (int d = 0; d < DEPTH; ++d) load_next(ring_u + d * 1024);
-    if (FEW_L2 && lane < 8 && nu > 0) {
-        // whole rows of this warp's stretch of k: the tiles that the ring has not reached
-        for (int r = DEPTH / nu; r < tiles; ++r) {
-            const int n = n0 + 8 * r + lane;
-            if (n < a.N)
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
-                             ::"l"(f.w + (size_t)n * f.ldw + u0 * 64), "r"(min(nu * 64, a.K - u0 * 64) * 2) : "memory");
-        }
-    }
 
     pdl_wait();
     // ---- tokens: this lane's own fragments, [unit][half][token][4 lanes][16 bytes] -----------------
@@ -1626,7 +1614,7 @@ extern "C" void mf_gemm_few_mode(int mode) { g_few_mode = mode; }
 static FewPlan few_plan(int M, int N, int K) {
     FewPlan p = {0, 0, 0, 0, 0, 0, 0};
     if (g_few_mode == 0 || M < 1 || M > FEW_MAX_M || N < 1 || K < 1) return p;
-    if ((long long)N * K * 2 > ((long long)FEW_LIMIT_MB << 20)) return p;
+    if ((long long)N * K * 2 > FEW_MAX_BYTES) return p;
     const int units = (K + 63) / 64, tiles = (N + 7) / 8, sms = sm_count();
     for (int cluster = 1; cluster <= 4; cluster *= 2) {
         const int slots = cluster == 4 ? (sms - 16) / 4 : sms / cluster;       // clusters that fit at once
@@ -1634,7 +1622,7 @@ static FewPlan few_plan(int M, int N, int K) {
         const int stride = 8 * (rt | 1);
         const size_t fixed = sizeof(float) * ((size_t)FEW_WARPS * M * stride + 16 + (size_t)M * rt +
                                               (cluster > 1 ? (size_t)M * 8 * rt : 0)) + (size_t)FEW_WARPS * wu * M * 128;
-        const int depths[] = {2, 4, 6};
+        const int depths[] = {2, 4, 8};
         int depth = 0;
         for (int d : depths) {
             if (depth > 0 && fixed + (size_t)FEW_WARPS * d * 1024 > FEW_BUDGET) break;
@@ -1689,7 +1677,7 @@ static int launch_few_depth(const FewPlan& p, const FewArgs& f, const GemmArgs& 
     switch (p.depth) {
         case 2: return launch_few<NT, 2>(p, f, a, stream);
         case 4: return launch_few<NT, 4>(p, f, a, stream);
-        default: return launch_few<NT, 6>(p, f, a, stream);
+        default: return launch_few<NT, 8>(p, f, a, stream);
     }
 }
 
