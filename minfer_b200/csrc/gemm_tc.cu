@@ -775,11 +775,18 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 //     rows and cuts K.
 //   * The warps' sums meet in shared memory and are added in warp order, a cluster's in rank order:
 //     reproducible, and complete, so no next kernel has K splits to add.
+// Bound by latency: what is left after the wait is a trip for the tokens, the MMAs, the warps' sums and a
+// store.  Measured, us a layer's products in a chain (q|k|v, O, gate|up, down), tcgen05 tiles -> here, 1 / 8
+// tokens: 0.5B shape 23.3 -> 17.9 / 24.0 -> 18.0; width 2,048, feed-forward 8,448 39.2 -> 34.6 / 41.0 -> 37.2;
+// 7B (q|k|v and O only) 86.4 -> 82.3 / 87.5 -> 82.8.  q|k|v of the 0.5B shape alone 5.8 -> 2.3.
+// Slower: the weights in registers instead of shared memory (27.4), 16 rows a tile (22.4), 8 warps (19.6),
+// two CTAs of 8 warps an SM (18.6), registers for two CTAs of 16 and the rest of the weights asked for in L2
+// (21.3).
 // ------------------------------------------------------------------------------------------
 #define FEW_WARPS 16
 #define FEW_THREADS (32 * FEW_WARPS)
 #define FEW_MAX_M 16
-#define FEW_BUDGET (112 * 1024)       // shared memory of a CTA
+#define FEW_BUDGET (200 * 1024)       // shared memory of a CTA (112 KB: fewer products at 8 tokens fit, 0.6 us a layer more)
 #define FEW_MAX_BYTES (64ll << 20)     // of weights: beyond, the TMA ring streams as fast as memory gives
 
 struct FewArgs {
