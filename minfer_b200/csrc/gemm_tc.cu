@@ -787,6 +787,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 #define FEW_THREADS (32 * FEW_WARPS)
 #define FEW_MAX_M 16
 #define FEW_BUDGET (200 * 1024)       // shared memory of a CTA (112 KB: fewer products at 8 tokens fit, 0.6 us a layer more)
+#define FEW_MIN_BYTES (512ll << 10)    // of weights: below, a product is a launch whichever kernel runs it
 #define FEW_MAX_BYTES (64ll << 20)     // of weights: beyond, the TMA ring streams as fast as memory gives
 
 struct FewArgs {
@@ -1616,12 +1617,15 @@ extern "C" long long mf_gemm_tc_workspace_floats(int M, int N, int K, int epi) {
 
 // How gemm_few_kernel cuts a product, or groups 0: another kernel takes it.
 struct FewPlan { int row_tiles, warp_units, tok_stride, depth, cluster, groups; size_t smem; };
-static int g_few_mode = 1;                // 0 never (measurement, tests of the other kernels), 1 where the rule says so
+static int g_few_mode = 1;                // 0 never, 1 where the rule says so, 2 also below FEW_MIN_BYTES (tests, measurement)
 extern "C" void mf_gemm_few_mode(int mode) { g_few_mode = mode; }
 static FewPlan few_plan(int M, int N, int K) {
     FewPlan p = {0, 0, 0, 0, 0, 0, 0};
     if (g_few_mode == 0 || M < 1 || M > FEW_MAX_M || N < 1 || K < 1) return p;
-    if ((long long)N * K * 2 > FEW_MAX_BYTES) return p;
+    const long long bytes = (long long)N * K * 2;
+    // (with two tiles of tokens an SM reads twice as much shared memory for a byte of weights: 16 tokens, 7B
+    // q|k|v of 33 MB 11.4 -> 12.1 us, O of 26 MB 8.5 -> 10.3; 0.5B shape's layer 24.4 -> 20.9)
+    if (bytes > (M <= 8 ? FEW_MAX_BYTES : FEW_MAX_BYTES / 4) || (bytes < FEW_MIN_BYTES && g_few_mode != 2)) return p;
     const int units = (K + 63) / 64, tiles = (N + 7) / 8, sms = sm_count();
     for (int cluster = 1; cluster <= 4; cluster *= 2) {
         const int slots = cluster == 4 ? (sms - 16) / 4 : sms / cluster;       // clusters that fit at once

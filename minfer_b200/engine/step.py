@@ -459,9 +459,7 @@ class Engine:
         if self._graph_pool is None:
             self._graph_pool = graph.pool()
         ring = []
-        # steps the host may be ahead of the device: enough for a next prompt's launches (some 4 ms) to be
-        # issued behind the last steps of a small model (0.5 ms each)
-        for _ in range(16):
+        for _ in range(4):
             ring.append(K.PinnedSlot(total))
         entry = {"graph": graph, "dev": dev, "logits": logits, "ring": ring, "next": 0,
                  "kernels": captured}

@@ -677,7 +677,8 @@ def gemm_few_groups(m: int, n: int, k: int) -> int:
 
 
 def gemm_few_mode(mode: int) -> None:
-    """0: the kernel for a handful of tokens takes no product; 1: those its rule names (the default)."""
+    """0: the kernel for a handful of tokens takes no product; 1: those its rule names (the default); 2: smaller
+    ones too."""
     _lib("gemm_tc").mf_gemm_few_mode(int(mode))
     _FEW.clear()
     _PREP_PARTS.clear()
