@@ -1134,7 +1134,11 @@ extern "C" int mf_sink_decode_plan(int rows, int n_kv, int reach_keys, int* tile
     const int n_tiles = reach_keys / SD_KEYS + 2;                  // the range need not start on a tile
     int splits = (2 * mf_sm_count() + rows * n_kv - 1) / (rows * n_kv > 0 ? rows * n_kv : 1);
     const int most = (n_tiles + SD_WARPS - 1) / SD_WARPS;
-    if (splits > most) splits = most;
+    // A warp with one tile needs one buffer and has its keys on the way before it waits; with 64 KB a CTA (head
+    // size 128) three share an SM.  So a tile a warp while all CTAs are on the GPU at once: 8 sequences of up to
+    // 1,536 positions, 4 key/value heads, 13 splits of one tile a warp instead of 7 of two with 128 KB a CTA
+    // and two rounds.
+    if (splits > most || (long long)rows * n_kv * most <= 3 * mf_sm_count()) splits = most;
     if (splits < 1) splits = 1;
     int tpc = (n_tiles + splits - 1) / splits;
     tpc = ((tpc + SD_WARPS - 1) / SD_WARPS) * SD_WARPS;
