@@ -1777,6 +1777,14 @@ __global__ void __launch_bounds__(1024) norm_terms_kernel(NormTermsArgs a) {
     __shared__ float2 scratch[3][32];
     const int width = a.width;
     const size_t base = (size_t)blockIdx.x * width, split = (size_t)gridDim.x * width;
+    // The weights are read behind one sum over the block after another: asked for in L2 before the wait, so
+    // that none of those reads is a trip to memory (a line of 128 bytes: 32 numbers)
+    for (int i = threadIdx.x * 32; i < width; i += blockDim.x * 32) {
+        const float* weights[4] = {a.t1.scale, PAIR ? a.t2.scale : nullptr, a.out_w, a.next_w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (weights[k] != nullptr) asm volatile("prefetch.global.L2 [%0];" ::"l"(weights[k] + i));
+    }
     pdl_wait();
     float u[4][VEC], g[PAIR ? 4 : 1][VEC];
     float s1 = 0.0f, s2 = 0.0f;
