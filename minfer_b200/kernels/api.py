@@ -55,12 +55,13 @@ def _ptr(t: Optional[torch.Tensor], what: str = "tensor") -> Optional[int]:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream() -> int:
     """The current CUDA stream's handle (called once per launch: the short way where torch has it)."""
-    if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+    if _raw_stream is not None and _device is not None:
+        return _raw_stream(_device())       # (the tensors at hand are on a device: CUDA is set up)
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -82,14 +83,15 @@ def _f64(t: Optional[torch.Tensor], what: str) -> Optional[int]:
     return _ptr(t, what)
 
 
-_configured: set[str] = set()
+_configured: dict[str, ctypes.CDLL] = {}
 
 
 def _lib(name: str) -> ctypes.CDLL:
-    lib = load_library(name)
-    if name not in _configured:
+    lib = _configured.get(name)
+    if lib is None:
+        lib = load_library(name)
         _SIGNATURES[name](lib)
-        _configured.add(name)
+        _configured[name] = lib
     return lib
 
 
