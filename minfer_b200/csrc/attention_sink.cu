@@ -895,7 +895,9 @@ __global__ void __launch_bounds__(SD_WARPS * 32) sink_attention_decode_kernel(Si
     };
     int tile = tile_lo + warp;
     // In a step of one token a row the kernel before this one writes one position of the row, its own: a
-    // tile that lies below it (and, in a ring, does not share its slot) is copied before the wait.
+    // tile that lies below it (and, in a ring, does not share its slot) is copied before the wait.  With the
+    // merge in one trip and no splits beyond the longest sequence, us a layer at 8 rows of up to 1,300
+    // positions: mask of 8,192 positions 22.7 -> 11.5, window of 1,024 11.1 -> 9.2.
     auto old_tile = [&](int vt) {
         const int key0 = real_tile(vt) * SD_KEYS;
         return a.old_keys_final != 0 && key0 + SD_KEYS - 1 < pos && (a.ring == 0 || key0 + a.ring > pos);
