@@ -55,13 +55,12 @@ def _ptr(t: Optional[torch.Tensor], what: str = "tensor") -> Optional[int]:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream() -> int:
     """The current CUDA stream's handle (called once per launch: the short way where torch has it)."""
-    if _raw_stream is not None and _device is not None:
-        return _raw_stream(_device())       # (the tensors at hand are on a device: CUDA is set up)
+    if _raw_stream is not None:
+        return _raw_stream(torch.cuda.current_device())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -83,15 +82,14 @@ def _f64(t: Optional[torch.Tensor], what: str) -> Optional[int]:
     return _ptr(t, what)
 
 
-_configured: dict[str, ctypes.CDLL] = {}
+_configured: set[str] = set()
 
 
 def _lib(name: str) -> ctypes.CDLL:
-    lib = _configured.get(name)
-    if lib is None:
-        lib = load_library(name)
+    lib = load_library(name)
+    if name not in _configured:
         _SIGNATURES[name](lib)
-        _configured[name] = lib
+        _configured.add(name)
     return lib
 
 

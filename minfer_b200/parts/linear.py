@@ -14,8 +14,6 @@ import torch
 import os
 
 from ..kernels import api as K
-from ..kernels import gemm
-from .base import Pending, Prepared
 
 # MINFER_B200_FOLD_NORMS=0: every norm runs as a kernel of its own (for comparison)
 FOLD_NORMS = os.environ.get("MINFER_B200_FOLD_NORMS", "1") != "0"
@@ -32,6 +30,7 @@ class Linear:
 
     def takes_row_scale(self) -> bool:
         """The tensor-core kernel multiplies this projection (only it can apply a row scale)."""
+        from ..kernels import gemm
         w = self.weight
         return (w.dtype == torch.bfloat16 and gemm.use_tensor_cores() and w.shape[1] % 8 == 0
                 and w.stride(1) == 1 and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0)
@@ -51,12 +50,14 @@ class Linear:
         if x.shape[0] == 0:
             return out
         if row_scale is not None:
+            from ..kernels import gemm
             if not (self.takes_row_scale() and K.gemm_tc_supported(x, self.weight)):
                 raise K.KernelError("a row scale needs the tensor-core product")
             K.gemm_tc_fused(x, self.weight, self.bias, out, K.EPI_ACCUM if accumulate else K.EPI_STORE,
                             gemm.status_word(x.device), row_scale=row_scale)
             return out
         if x.dtype == torch.bfloat16 and self.weight.dtype == torch.bfloat16:
+            from ..kernels import gemm
             gemm.gemm_bf16(x, self.weight, self.bias, out, accumulate)
         else:
             K.gemm_simt(x, self.weight, self.bias, out, accumulate)
@@ -66,6 +67,8 @@ class Linear:
         """If the tensor-core kernel would split this product along K (few tokens, few output
         rows), runs the splits and returns them as a ``Pending`` (bias included) for the next
         kernel to add; otherwise returns None and the caller uses ``forward``."""
+        from ..kernels import gemm
+        from .base import Pending
         if (x.dtype != torch.bfloat16 or self.weight.dtype != torch.bfloat16 or x.shape[0] == 0
                 or not gemm.use_tensor_cores()
                 or K.gemm_few_groups(x.shape[0], self.out_features, self.in_features)):
@@ -83,6 +86,8 @@ class Linear:
         """``residual`` += x W^T + b, complete when the call returns, together with what ``norm``
         (which reads ``residual`` next) needs: returns a ``Prepared``, or None (and does nothing)
         if ``norm`` is not foldable or no kernel does this at these sizes."""
+        from ..kernels import gemm
+        from .base import Prepared
         fold = norm.foldable() if norm is not None else None
         m = x.shape[0]
         if (fold is None or m == 0 or x.dtype != torch.bfloat16 or not self.takes_row_scale()
@@ -117,6 +122,7 @@ class GroupedLinear:
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         """``x`` [groups, rows, in] -> float32 [groups, rows, out]."""
+        from ..kernels import gemm
         groups, n, width = x.shape
         out = torch.empty((groups, n, self.weight.shape[1]), dtype=torch.float32, device=x.device)
         if n == 0:

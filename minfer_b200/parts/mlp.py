@@ -15,7 +15,6 @@ from typing import Dict, List, Optional
 import torch
 
 from ..kernels import api as K
-from ..kernels import gemm
 from ..weights.spec import MATRIX, VECTOR, Init, TensorSpec
 from .base import FeedForward, StepContext, settle_pending
 from .linear import Linear
@@ -81,6 +80,7 @@ class GatedMlp(FeedForward):
                 f"{prefix}{self.down_name}": self.down.weight}
 
     def forward_add(self, x: torch.Tensor, ctx: StepContext, residual: torch.Tensor) -> None:
+        from ..kernels import gemm
         act = torch.empty((x.shape[0], self.intermediate_size), dtype=ctx.act_dtype,
                           device=x.device)
         w = self.gate_up.weight
@@ -192,6 +192,7 @@ class DenseMlp(FeedForward):
         return out
 
     def forward_add(self, x: torch.Tensor, ctx: StepContext, residual: torch.Tensor) -> None:
+        from ..kernels import gemm
         act = torch.empty((x.shape[0], self.intermediate_size), dtype=ctx.act_dtype, device=x.device)
         if self.activation == "poly_norm":
             # a row's three sums come before any of its outputs: the activation is a kernel of
