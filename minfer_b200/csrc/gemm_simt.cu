@@ -110,7 +110,7 @@ gemm_simt_kernel(const TA* A, const TW* __restrict__ W, const float* __restrict_
 // in flight in registers while this one is multiplied.
 // Measured (us back to back, the tile that is chosen and the 64 x 64 x 16 kernel above in brackets):
 // 385 x 9,728 x 896 192 (64 x 64) [387], 385 x 896 x 4,864 216 (32 x 64) [480], 64 x 896 x 4,864 93 (32 x 64)
-// [469], 385 x 151,936 x 896 2,546 (128 x 128) [5,617], 1,600 x 8,448 x 2,048 1,080 (128 x 128) [2,505] = 51
+// [469] (these two with one CTA a tile; behind a norm 385 x 896 x 4,864 took 244 that way, 147 with four), 385 x 151,936 x 896 2,546 (128 x 128) [5,617], 1,600 x 8,448 x 2,048 1,080 (128 x 128) [2,505] = 51
 // TFLOP/s of the pipe's 74.  Plain multiply-adds instead of packed ones: 2 to 7 % slower.  AHEAD 2 (loads two tiles ahead) for the smallest tile, whose product of
 // a tile is shorter than a trip to memory: 64 x 896 x 4,864 129 -> 95; for 64 x 64 it lost (240 -> 280).
 __device__ __forceinline__ unsigned long long f32x2(float lo, float hi) {
