@@ -1781,7 +1781,9 @@ __global__ void __launch_bounds__(1024) norm_terms_kernel(NormTermsArgs a) {
     // The weights are read behind one sum over the block after another: asked for in L2 before the wait, so
     // that none of those reads is a trip to memory (a line of 128 bytes: 32 numbers): 8 rows of 2,048 in a
     // decode step 5.5 to 6.3 -> 4.0 to 5.2 us, two terms 9.7 -> 7.1
-    for (int i = threadIdx.x * 32; i < width; i += blockDim.x * 32) {
+    // Few rows only: with many, every CTA asks again for what is there already (two terms of 512, 2,000 rows
+    // 5.3 -> 14.1 us; of 2,048, 300 rows 4.8 -> 6.2).
+    for (int i = threadIdx.x * 32; gridDim.x <= 64 && i < width; i += blockDim.x * 32) {
         const float* weights[4] = {a.t1.scale, PAIR ? a.t2.scale : nullptr, a.out_w, a.next_w};
 #pragma unroll
         for (int k = 0; k < 4; ++k)
