@@ -808,6 +808,7 @@ extern "C" int mf_sink_attention_mma(const void* q, const void* k, const void* v
 // ------------------------------------------------------------------------------------------
 #define SD_WARPS 4
 #define SD_KEYS 32
+#define SD_MERGE 16              // splits that are merged in one trip
 
 struct SinkDecodeArgs {
     const __nv_bfloat16* q;   // [rows][n_heads][hd]
@@ -897,15 +898,16 @@ __global__ void __launch_bounds__(SD_WARPS * 32) sink_attention_decode_kernel(Si
     // In a step of one token a row the kernel before this one writes one position of the row, its own: a
     // tile that lies below it (and, in a ring, does not share its slot) is copied before the wait.  With the
     // merge in one trip and no splits beyond the longest sequence, us a layer at 8 rows of up to 1,300
-    // positions: mask of 8,192 positions 22.7 -> 11.5, window of 1,024 11.1 -> 9.2.
+    // positions: mask of 8,192 positions 22.7 -> 11.5, window of 1,024 11.1 -> 9.2.  (One place in the code that
+    // copies, in front of the wait or behind it: with two of them 512 CTAs of 3 tiles took 19.1 us instead of 16.6.)
     auto old_tile = [&](int vt) {
         const int key0 = real_tile(vt) * SD_KEYS;
         return a.old_keys_final != 0 && key0 + SD_KEYS - 1 < pos && (a.ring == 0 || key0 + a.ring > pos);
     };
     const bool early = tile <= tile_hi && old_tile(tile);
-    if (early) load_tile(real_tile(tile), 0);
-    pdl_wait();
-    if (tile <= tile_hi && !early) load_tile(real_tile(tile), 0);
+    if (!early) pdl_wait();
+    if (tile <= tile_hi) load_tile(real_tile(tile), 0);
+    if (early) pdl_wait();
 
     float m_r[2] = {-INFINITY, -INFINITY}, l_r[2] = {0.0f, 0.0f};
     float o[VDP / 8][4];
@@ -1081,13 +1083,13 @@ __global__ void sink_decode_combine_kernel(const float* partial,
     const size_t stride = (size_t)(vd + 2);
     const float* p = partial + rh * n_splits * stride;
     const float sink2 = (sink && sink_logit) ? sink_logit[rh % n_heads] * 1.4426950408889634f : 0.0f;
-    if (n_splits <= 16) {
+    if (n_splits <= SD_MERGE) {
         // the usual case: every maximum, sum and value a thread needs in one trip (the loops below make
         // three and more); the same operations in the same order
-        float mc[16], lc[16], oc[16];
+        float mc[SD_MERGE], lc[SD_MERGE], oc[SD_MERGE];
         const int d = threadIdx.x;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
+        for (int c = 0; c < SD_MERGE; ++c) {
             mc[c] = -INFINITY;
             if (c < n_splits) {
                 mc[c] = p[c * stride];
@@ -1097,10 +1099,10 @@ __global__ void sink_decode_combine_kernel(const float* partial,
         }
         float m = sink ? sink2 : -INFINITY;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) m = fmaxf(m, mc[c]);
+        for (int c = 0; c < SD_MERGE; ++c) m = fmaxf(m, mc[c]);
         float l = sink ? exp2f(sink2 - m) : 0.0f, acc = 0.0f;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
+        for (int c = 0; c < SD_MERGE; ++c) {
             if (mc[c] > -INFINITY) {
                 const float f = exp2f(mc[c] - m);
                 l = fmaf(lc[c], f, l);
@@ -1131,22 +1133,26 @@ __global__ void sink_decode_combine_kernel(const float* partial,
 // How the keys of single queries are cut: (tiles of 32 keys per CTA, splits), from the sizes
 // only.  `n_kv`: key/value heads times the blocks of 16 query heads on each.  `reach_keys`: the
 // most keys a query sees (its reach, or the longest sequence).
-extern "C" int mf_sink_decode_plan(int rows, int n_kv, int reach_keys, int* tiles_per_cta,
-                                   int* n_splits) {
+extern "C" int mf_sink_decode_plan_on(int rows, int n_kv, int reach_keys, int sms, int* tiles_per_cta,
+                                      int* n_splits) {
     const int n_tiles = reach_keys / SD_KEYS + 2;                  // the range need not start on a tile
-    int splits = (2 * mf_sm_count() + rows * n_kv - 1) / (rows * n_kv > 0 ? rows * n_kv : 1);
+    int splits = (2 * sms + rows * n_kv - 1) / (rows * n_kv > 0 ? rows * n_kv : 1);
     const int most = (n_tiles + SD_WARPS - 1) / SD_WARPS;
     // A warp with one tile needs one buffer and has its keys on the way before it waits; with 64 KB a CTA (head
     // size 128) three share an SM.  So a tile a warp while all CTAs are on the GPU at once: 8 sequences of up to
     // 1,536 positions, 4 key/value heads, 13 splits of one tile a warp instead of 7 of two with 128 KB a CTA
-    // and two rounds.
-    if (splits > most || (long long)rows * n_kv * most <= 3 * mf_sm_count()) splits = most;
+    // and two rounds.  But no more splits than the merge takes in one trip: 3 sequences of 8,000 positions, 2
+    // key/value heads 32 splits 23.9 us (head size 64: 15.8), 63 splits 28.6 (22.1).
+    if (splits > most || (most <= SD_MERGE && (long long)rows * n_kv * most <= 3 * sms)) splits = most;
     if (splits < 1) splits = 1;
     int tpc = (n_tiles + splits - 1) / splits;
     tpc = ((tpc + SD_WARPS - 1) / SD_WARPS) * SD_WARPS;
     *tiles_per_cta = tpc;
     *n_splits = (n_tiles + tpc - 1) / tpc;
     return 0;
+}
+extern "C" int mf_sink_decode_plan(int rows, int n_kv, int reach_keys, int* tiles_per_cta, int* n_splits) {
+    return mf_sink_decode_plan_on(rows, n_kv, reach_keys, mf_sm_count(), tiles_per_cta, n_splits);
 }
 
 template <int HDP, int VDP>

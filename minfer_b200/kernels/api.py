@@ -243,6 +243,7 @@ def _sig_attention_sink(lib: ctypes.CDLL) -> None:
 
 
     lib.mf_sink_decode_plan.argtypes = [c_int, c_int, c_int, c_void_p, c_void_p]
+    lib.mf_sink_decode_plan_on.argtypes = [c_int, c_int, c_int, c_int, c_void_p, c_void_p]
     lib.mf_sink_attention_decode.argtypes = ([c_void_p] * 6 + [c_int, c_int] + [c_void_p] * 4 +
                                              [c_int] * 8 + [c_float, c_int, c_void_p, c_float, c_int, c_int,
                                                             c_void_p])

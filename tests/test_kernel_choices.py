@@ -76,6 +76,9 @@ def test_which_float32_prompts_walk_their_keys_by_tiles(lens, tiled):
     (20, 4_000_000, 2), (20, 5_000_000, 0),         # 65,535 tiles of 64 columns end at 4,194,240
     (20, 9_000_000, -1),
 ])
-def test_tile_of_a_float32_product(m, n, tile):
-    """0: 128 x 128, 1: 64 x 64, 2: 32 x 64, -1: the general kernel."""
-    assert K._lib("gemm_simt").mf_gemm_f32_tile(m, n, SMS) == tile
+def test_cut_of_single_queries(rows, kv, reach, tiles, splits):
+    out = (ctypes.c_int * 2)()
+    K._lib("attention_sink").mf_sink_decode_plan_on(rows, kv, reach, SMS, ctypes.addressof(out),
+                                                    ctypes.addressof(out) + 4)
+    assert tuple(out) == (tiles, splits)
+    assert tiles * splits * 32 >= reach + 31                 # the reach need not start on a tile
