@@ -1,5 +1,7 @@
 """Which kernel a call takes: host functions of sizes, each with the sizes that were measured on either side
 of its line (148 SMs, no GPU)."""
+import ctypes
+
 import pytest
 
 from minfer_b200.kernels import api as K
@@ -75,6 +77,19 @@ def test_which_float32_prompts_walk_their_keys_by_tiles(lens, tiled):
     (700, 9001, 0), (2170, 2175, 0), (4096, 1152, 0), (1600, 8448, 0), (385, 151936, 0),
     (20, 4_000_000, 2), (20, 5_000_000, 0),         # 65,535 tiles of 64 columns end at 4,194,240
     (20, 9_000_000, -1),
+])
+def test_tile_of_a_float32_product(m, n, tile):
+    """0: 128 x 128, 1: 64 x 64, 2: 32 x 64, -1: the general kernel."""
+    assert K._lib("gemm_simt").mf_gemm_f32_tile(m, n, SMS) == tile
+
+
+@pytest.mark.parametrize("rows,kv,reach,tiles,splits", [
+    # (tiles a CTA, CTAs that share a row's keys); four tiles: a tile a warp
+    (8, 4, 1300, 4, 11), (8, 4, 1536, 4, 13),      # all CTAs on the GPU at once, merged in one trip
+    (3, 2, 1900, 4, 16), (3, 2, 2000, 4, 16),
+    (3, 2, 8000, 8, 32), (3, 2, 8192, 8, 33), (26, 1, 3000, 8, 12),    # more splits than one trip takes
+    (8, 8, 3000, 20, 5), (64, 4, 1300, 24, 2), (64, 8, 100, 8, 1),     # the rows alone fill the GPU
+    (1, 8, 100, 4, 2), (1, 1, 1, 4, 1),
 ])
 def test_cut_of_single_queries(rows, kv, reach, tiles, splits):
     out = (ctypes.c_int * 2)()
