@@ -26,14 +26,15 @@ __host__ __device__ constexpr int f32_stretch(int K) { return K < 2048 ? K : ((K
 #define BK 16
 
 // accumulate: 0  C = acc + bias        1  C = C + acc + bias  (C float32: residual stream)
-template <typename TA, typename TW, typename TC>
-__global__ void __launch_bounds__(256)
+template <typename TA, typename TW, typename TC, bool LONG>
+__global__ void __launch_bounds__(256, 4)
 gemm_simt_kernel(const TA* A, const TW* __restrict__ W, const float* __restrict__ bias,
                  TC* C, int M, int N, int K, long long lda, long long ldw,
                  long long ldc, int accumulate) {
     pdl_prologue();
     __shared__ float As[BK][BM + 4];
     __shared__ float Ws[BK][BN + 4];
+    __shared__ float4 done[LONG ? 4 * 256 : 1];      // every thread's sums of the stretches before this one
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;          // 16 x 16 threads, 4 x 4 outputs each
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
@@ -43,56 +44,71 @@ gemm_simt_kernel(const TA* A, const TW* __restrict__ W, const float* __restrict_
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
 
-    const int stretch = f32_stretch(K);
-    float done[4][4];                                // the stretches before this one
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        if (k0 > 0 && k0 % stretch == 0) {
+    // LONG (four stretches of k): the sums put away in shared memory, so that four CTAs share an SM as they do for
+    // one stretch: in registers, and in kernels of any K, 385 x 3,028 x 10,600 (bfloat16 x float32) took 4,030 us
+    // instead of 2,340, 64 x 896 x 4,864 497 instead of 465.  Now, with two tiles of k a round, 1,760 and 411.
+    const int stretch = LONG ? f32_stretch(K) : K;
+    for (int k0 = 0; k0 < K;) {
+        if (LONG && k0 > 0) {
+            float4* d = done + tid;
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    done[i][j] = k0 == stretch ? acc[i][j] : done[i][j] + acc[i][j];
-                    acc[i][j] = 0.0f;
+            for (int i = 0; i < 4; ++i) {
+                float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+                if (k0 > stretch) {
+                    const float4 o = d[i * 256];
+                    v.x = o.x + v.x; v.y = o.y + v.y; v.z = o.z + v.z; v.w = o.w + v.w;
                 }
-        }
-        // 64 rows x 16 k per operand = 1024 elements, 4 per thread; k fastest for coalescing
+                d[i * 256] = v;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int idx = tid + e * 256;
-            const int r = idx >> 4, kk = idx & 15;
-            const int k = k0 + kk;
-            float a = 0.0f, w = 0.0f;
-            if (k < K) {
-                if (m0 + r < M) a = to_f32(A[(size_t)(m0 + r) * lda + k]);
-                if (n0 + r < N) w = to_f32(W[(size_t)(n0 + r) * ldw + k]);
+                for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
             }
-            As[kk][r] = a;
-            Ws[kk][r] = w;
         }
-        __syncthreads();
+#pragma unroll 2
+        for (const int end = LONG ? min(k0 + stretch, K) : K; k0 < end; k0 += BK) {
+            // 64 rows x 16 k per operand = 1024 elements, 4 per thread; k fastest for coalescing
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float a[4], w[4];
+            for (int e = 0; e < 4; ++e) {
+                const int idx = tid + e * 256;
+                const int r = idx >> 4, kk = idx & 15;
+                const int k = k0 + kk;
+                float a = 0.0f, w = 0.0f;
+                if (k < K) {
+                    if (m0 + r < M) a = to_f32(A[(size_t)(m0 + r) * lda + k]);
+                    if (n0 + r < N) w = to_f32(W[(size_t)(n0 + r) * ldw + k]);
+                }
+                As[kk][r] = a;
+                Ws[kk][r] = w;
+            }
+            __syncthreads();
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
+            for (int kk = 0; kk < BK; ++kk) {
+                float a[4], w[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = Ws[kk][tx * 4 + j];
+                for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+                for (int j = 0; j < 4; ++j) w[j] = Ws[kk][tx * 4 + j];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+            }
+            __syncthreads();
         }
-        __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int m = m0 + ty * 4 + i;
         if (m >= M) continue;
+        if (LONG) {
+            const float4 o = done[i * 256 + tid];
+            acc[i][0] = o.x + acc[i][0]; acc[i][1] = o.y + acc[i][1];
+            acc[i][2] = o.z + acc[i][2]; acc[i][3] = o.w + acc[i][3];
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int n = n0 + tx * 4 + j;
             if (n >= N) continue;
-            float v = stretch < K ? done[i][j] + acc[i][j] : acc[i][j];
+            float v = acc[i][j];
             if (bias) v += bias[n];
             TC* c = C + (size_t)m * ldc + n;
             if (accumulate) v += to_f32(*c);
@@ -360,7 +376,11 @@ __device__ __forceinline__ void copy16_async(void* smem, const void* src, bool r
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-template <int RT>
+// LONG: four stretches of k, one behind the other; 8 x 896 x 4,864 29.4 us (29.1 as one chain).  The end of a stretch is
+// counted and stands behind the wait for a chunk's copies: with a remainder for every chunk, in kernels of any K, it took
+// 36.3 (8 x 896 x 896 7.9 instead of 6.6), with a loop around the stretches 36.8; a quarter of a chunk from each
+// stretch, as four independent chains, 29.6, but 8 x 5,228 x 15,960 325 instead of 245: 64-byte pieces of a row.
+template <int RT, bool LONG>
 __global__ void __launch_bounds__(F32Few<RT>::WARPS * 32)
 gemm_f32_few_kernel(const float* A, const float* W, const float* __restrict__ bias, float* C, int M, int N,
                     int K, long long lda, long long ldw, long long ldc, int accumulate) {
@@ -391,15 +411,9 @@ gemm_f32_few_kernel(const float* A, const float* W, const float* __restrict__ bi
     float acc[RT], done[RT];                                         // done: the stretches before this one
 #pragma unroll
     for (int i = 0; i < RT; ++i) acc[i] = 0.0f;
-    const int stretch = f32_stretch(K);
+    const int per = LONG ? f32_stretch(K) / T::KC : chunks;          // chunks of a stretch
+    int end = per;
     for (int c = 0; c < chunks; ++c) {
-        if (c > 0 && c * T::KC % stretch == 0) {
-#pragma unroll
-            for (int i = 0; i < RT; ++i) {
-                done[i] = c * T::KC == stretch ? acc[i] : done[i] + acc[i];
-                acc[i] = 0.0f;
-            }
-        }
         if (c + 1 < chunks) {
             fetch(c + 1);
             asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -407,6 +421,14 @@ gemm_f32_few_kernel(const float* A, const float* W, const float* __restrict__ bi
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
         __syncwarp();
+        if (LONG && c == end) {
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                done[i] = c == per ? acc[i] : done[i] + acc[i];
+                acc[i] = 0.0f;
+            }
+            end += per;
+        }
         const float (*st)[T::PITCH] = ring[warp][c % T::STAGES];
         const int ks = min(T::KC, K - c * T::KC);
 #pragma unroll 8
@@ -429,7 +451,7 @@ gemm_f32_few_kernel(const float* A, const float* W, const float* __restrict__ bi
     for (int i = 0; i < RT; ++i) {
         const int m = grp + 4 * i;
         if (m >= M) continue;
-        float v = stretch < K ? done[i] + acc[i] : acc[i];
+        float v = LONG ? done[i] + acc[i] : acc[i];
         if (bias != nullptr) v += bias[n];
         float* c = C + (size_t)m * ldc + n;
         if (accumulate) v += *c;
@@ -496,12 +518,16 @@ static bool launch_f32(const float* A, const float* W, const float* bias, float*
     if (((uintptr_t)A | (uintptr_t)W) & 15 || (K | lda | ldw) & 3) return false;
     if (M <= 16) {
         const int warps = (int)(((long long)N + 7) / 8);
-#define MF_FEW(RT)                                                                                      \
-    mf_launch(gemm_f32_few_kernel<RT>, dim3((warps + F32Few<RT>::WARPS - 1) / F32Few<RT>::WARPS),        \
-              dim3(F32Few<RT>::WARPS * 32), 0, stream, A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate)
-        if (M <= 4) MF_FEW(1);
-        else if (M <= 8) MF_FEW(2);
-        else MF_FEW(4);
+#define MF_FEW(RT)                                                                                       \
+    if (f32_stretch(K) < K)                                                                              \
+        mf_launch(gemm_f32_few_kernel<RT, true>, dim3((warps + F32Few<RT>::WARPS - 1) / F32Few<RT>::WARPS), \
+                  dim3(F32Few<RT>::WARPS * 32), 0, stream, A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate); \
+    else                                                                                                 \
+        mf_launch(gemm_f32_few_kernel<RT, false>, dim3((warps + F32Few<RT>::WARPS - 1) / F32Few<RT>::WARPS), \
+                  dim3(F32Few<RT>::WARPS * 32), 0, stream, A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate)
+        if (M <= 4) { MF_FEW(1); }
+        else if (M <= 8) { MF_FEW(2); }
+        else { MF_FEW(4); }
 #undef MF_FEW
         return true;
     }
@@ -528,10 +554,13 @@ extern "C" int mf_gemm_simt(const void* A, int a_dtype, const void* W, int w_dty
         return MF_LAUNCH_CHECK();
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return MF_ERR_UNSUPPORTED;
-#define MF_GEMM(TA, TW, TC)                                                                  \
-    mf_launch(gemm_simt_kernel<TA, TW, TC>, dim3(grid), dim3(256), 0, stream, (const TA*)A, (const TW*)W, bias,  \
-                                                           (TC*)C, M, N, K, lda, ldw, ldc,   \
-                                                           accumulate)
+#define MF_GEMM(TA, TW, TC)                                                                                   \
+    if (f32_stretch(K) < K)                                                                                   \
+        mf_launch(gemm_simt_kernel<TA, TW, TC, true>, dim3(grid), dim3(256), 0, stream, (const TA*)A, (const TW*)W, \
+                  bias, (TC*)C, M, N, K, lda, ldw, ldc, accumulate);                                           \
+    else                                                                                                      \
+        mf_launch(gemm_simt_kernel<TA, TW, TC, false>, dim3(grid), dim3(256), 0, stream, (const TA*)A, (const TW*)W, \
+                  bias, (TC*)C, M, N, K, lda, ldw, ldc, accumulate)
     typedef __nv_bfloat16 bf16;
     const int key = a_dtype * 4 + w_dtype * 2 + c_dtype;
     switch (key) {

@@ -36,3 +36,26 @@ def test_rows_have_the_same_bits_in_every_kernel(n, k):
     out = torch.empty(40, n, device="cuda")
     K.gemm_simt(odd_x[:, :k], odd_w[:, :k], bias, out, False)
     assert torch.equal(out, whole[False][:40])
+
+
+@pytest.mark.parametrize("k", [40, 2044, 2047, 2048, 2049, 2180, 4864])
+@pytest.mark.parametrize("m,n", [(3, 70), (100, 129)])
+def test_mixed_types_have_the_bits_of_float32(m, n, k):
+    """The general kernel, one stretch of k and four, its last round of two tiles of k whole or half: numbers that
+    both types hold give the sums of the float32 kernels."""
+    from minfer_b200.kernels import api as K
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    x = torch.randn(m, k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).bfloat16()
+    old = torch.randn(m, n, generator=g, device="cuda")
+    for accumulate in (False, True):
+        want = old.clone()
+        K.gemm_simt(x.float(), w.float(), None, want, accumulate)
+        for a, b in ((x, w), (x, w.float()), (x.float(), w)):
+            out = old.clone()
+            K.gemm_simt(a, b, None, out, accumulate)
+            assert torch.equal(out, want)
+    half = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+    K.gemm_simt(x, w.float(), None, half, False)
+    K.gemm_simt(x.float(), w.float(), None, want, False)
+    assert torch.equal(half, want.bfloat16())
