@@ -20,6 +20,11 @@
 // CTAs a tile it does not.
 __host__ __device__ constexpr int f32_stretch(int K) { return K < 2048 ? K : ((K + 511) / 512) * 128; }
 #define F32_STRETCHES 4
+// how gemm_f32_tile_kernel goes through k: K as one stretch; a cluster of four CTAs a tile, a stretch each;
+// one CTA a tile, the four stretches one after the other
+#define F32_WHOLE 0
+#define F32_SPLIT 1
+#define F32_WALK 2
 
 #define BM 64
 #define BN 64
@@ -125,10 +130,12 @@ gemm_simt_kernel(const TA* A, const TW* __restrict__ W, const float* __restrict_
 // k swizzled by its quarter so that the transposing stores do not conflict; the next tile's loads are
 // in flight in registers while this one is multiplied.
 // Measured (us back to back, the tile that is chosen and the 64 x 64 x 16 kernel above in brackets):
-// 385 x 9,728 x 896 192 (64 x 64) [387], 385 x 896 x 4,864 216 (32 x 64) [480], 64 x 896 x 4,864 93 (32 x 64)
-// [469] (these two with one CTA a tile; behind a norm 385 x 896 x 4,864 took 244 that way, 147 with four), 385 x 151,936 x 896 2,546 (128 x 128) [5,617], 1,600 x 8,448 x 2,048 1,080 (128 x 128) [2,505] = 51
-// TFLOP/s of the pipe's 74.  Plain multiply-adds instead of packed ones: 2 to 7 % slower.  AHEAD 2 (loads two tiles ahead) for the smallest tile, whose product of
-// a tile is shorter than a trip to memory: 64 x 896 x 4,864 129 -> 95; for 64 x 64 it lost (240 -> 280).
+// 385 x 9,728 x 896 192 (64 x 64) [387], 385 x 151,936 x 896 2,546 (128 x 128) [5,617]; of a K in stretches, with
+// K as one in front: 385 x 896 x 4,864 227 -> 129 (32 x 64, a cluster a tile), 64 x 896 x 4,864 93 -> 56 (the same),
+// 1,600 x 2,048 x 8,448 1,380 -> 1,212 (128 x 128, the same), 1,600 x 8,448 x 2,048 1,082 -> 1,095 (128 x 128, one CTA a
+// tile) = 51 TFLOP/s of the pipe's 74; as a cluster a tile that took 1,197, 634 x 6,420 x 2,080 481 instead of 390.
+// Plain multiply-adds instead of packed ones: 2 to 7 % slower.  AHEAD 2 (loads two tiles ahead) for the smallest tile,
+// whose product of a tile is shorter than a trip to memory: 64 x 896 x 4,864 129 -> 95; for 64 x 64 it lost (240 -> 280).
 __device__ __forceinline__ unsigned long long f32x2(float lo, float hi) {
     unsigned long long r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -136,6 +143,11 @@ __device__ __forceinline__ unsigned long long f32x2(float lo, float hi) {
 }
 __device__ __forceinline__ void fma_f32x2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+__device__ __forceinline__ float4 f32_sums(unsigned long long a, unsigned long long b) {
+    return make_float4(__uint_as_float((unsigned)a), __uint_as_float((unsigned)(a >> 32)),
+                       __uint_as_float((unsigned)b), __uint_as_float((unsigned)(b >> 32)));
 }
 
 // An operand's 16 bytes, never moved above the wait for the kernel before (as a load through a const
@@ -193,9 +205,10 @@ struct F32Tile {
     static constexpr int THREADS = 32 * WARPS_N * (BM_ / (4 * TM));
 };
 
-// SPLIT: a cluster of four CTAs has a tile, CTA r the stretch r of k; they add their sums in order of the
-// stretches through distributed shared memory, each a quarter of the tile's rows.
-template <int BM_, int BN_, int TM, int TN, int BKT, int AHEAD, bool SPLIT>
+// F32_SPLIT: a cluster of four CTAs has a tile, CTA r the stretch r of k; they add their sums in order of the
+// stretches through distributed shared memory, each a quarter of the tile's rows.  F32_WALK: a CTA has a tile and
+// puts every thread's sums away in shared memory behind a stretch.
+template <int BM_, int BN_, int TM, int TN, int BKT, int AHEAD, int FORM>
 __global__ void __launch_bounds__(F32Tile<BM_, BN_, TM, TN>::THREADS,
                                   (AHEAD == 1 ? 512 : 384) / F32Tile<BM_, BN_, TM, TN>::THREADS)
 gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ bias, float* C,
@@ -204,7 +217,9 @@ gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ b
     constexpr int THREADS = F32Tile<BM_, BN_, TM, TN>::THREADS;
     constexpr int WARPS_N = F32Tile<BM_, BN_, TM, TN>::WARPS_N;
     constexpr int FA = BM_ * (BKT / 4) / THREADS, FW = BN_ * (BKT / 4) / THREADS;
+    constexpr bool SPLIT = FORM == F32_SPLIT, WALK = FORM == F32_WALK;
     __shared__ __align__(16) float pool[2 * BKT * (BM_ + BN_)];
+    extern __shared__ __align__(16) float f32_done[];  // WALK: every thread's sums of the stretches before
     float (*As)[BKT][BM_] = reinterpret_cast<float (*)[BKT][BM_]>(pool);
     float (*Ws)[BKT][BN_] = reinterpret_cast<float (*)[BKT][BN_]>(pool + 2 * BKT * BM_);
     const int k_first = SPLIT ? (int)blockIdx.z * f32_stretch(K_all) : 0;
@@ -262,7 +277,22 @@ gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ b
     put(0, 0);
     if (AHEAD == 2) fetch(1, 1);
     __syncthreads();
-    for (int t = 0; t < tiles; t += AHEAD) {
+    const int per = WALK ? f32_stretch(K_all) / BKT : tiles;         // tiles of a stretch: an even number
+    for (int t = 0, end = per; t < tiles; t += AHEAD) {
+        if (WALK && t == end) {
+            float4* d = reinterpret_cast<float4*>(f32_done) + threadIdx.x;
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int h = 0; h < TN / 4; ++h) {
+                    float4 v = f32_sums(acc[i][h * 2], acc[i][h * 2 + 1]);
+                    float4& at = d[(i * (TN / 4) + h) * THREADS];
+                    if (t > per) { const float4 o = at; v.x = o.x + v.x; v.y = o.y + v.y; v.z = o.z + v.z; v.w = o.w + v.w; }
+                    at = v;
+                    acc[i][h * 2] = acc[i][h * 2 + 1] = 0ull;
+                }
+            end += per;
+        }
 #pragma unroll
         for (int u = 0; u < AHEAD; ++u) {
             if (t + u >= tiles) break;
@@ -282,11 +312,9 @@ gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ b
             if (h > 0) cluster_wait_all();                            // the group before has been read
 #pragma unroll
             for (int i = 0; i < TM; ++i) {
-                const unsigned long long p0 = acc[i][h * 2], p1 = acc[i][h * 2 + 1];
                 *reinterpret_cast<float4*>(pool + (ty + (i >> 2) * 16 + (i & 3)) * COLS +
                                            (warp % WARPS_N) * 32 + (lane & 7) * 4) =
-                    make_float4(__uint_as_float((unsigned)p0), __uint_as_float((unsigned)(p0 >> 32)),
-                                __uint_as_float((unsigned)p1), __uint_as_float((unsigned)(p1 >> 32)));
+                    f32_sums(acc[i][h * 2], acc[i][h * 2 + 1]);
             }
             cluster_wait_all();
             for (int idx = threadIdx.x; idx < MINE * QUADS; idx += THREADS) {
@@ -333,12 +361,11 @@ gemm_f32_tile_kernel(const float* A, const float* W, const float* __restrict__ b
             const int m = m0 + ty + (i >> 2) * 16 + (i & 3);
             if (m >= M) continue;
             float* c = C + (size_t)m * ldc + n;
-            float v[4];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const unsigned long long p = acc[i][h * 2 + j];
-                v[2 * j] = __uint_as_float((unsigned)p);
-                v[2 * j + 1] = __uint_as_float((unsigned)(p >> 32));
+            const float4 sum = f32_sums(acc[i][h * 2], acc[i][h * 2 + 1]);
+            float v[4] = {sum.x, sum.y, sum.z, sum.w};
+            if (WALK) {
+                const float4 o = reinterpret_cast<const float4*>(f32_done)[(i * (TN / 4) + h) * THREADS + threadIdx.x];
+                v[0] = o.x + v[0]; v[1] = o.y + v[1]; v[2] = o.z + v[2]; v[3] = o.w + v[3];
             }
             if (bias != nullptr) {
 #pragma unroll
@@ -460,14 +487,30 @@ gemm_f32_few_kernel(const float* A, const float* W, const float* __restrict__ bi
 }
 
 template <int BM_, int BN_, int TM, int TN, int BKT, int AHEAD>
-static void launch_f32_tile(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
-                            long long lda, long long ldw, long long ldc, int accumulate, cudaStream_t stream) {
-    const dim3 grid((M + BM_ - 1) / BM_, (N + BN_ - 1) / BN_, f32_stretch(K) < K ? F32_STRETCHES : 1);
+static int launch_f32_tile(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
+                            long long lda, long long ldw, long long ldc, int accumulate, int form,
+                            cudaStream_t stream) {
+    const dim3 grid((M + BM_ - 1) / BM_, (N + BN_ - 1) / BN_, form == F32_SPLIT ? F32_STRETCHES : 1);
     const dim3 block(F32Tile<BM_, BN_, TM, TN>::THREADS);
-    if (grid.z == 1) {
-        mf_launch(gemm_f32_tile_kernel<BM_, BN_, TM, TN, BKT, AHEAD, false>, grid, block, 0, stream, A, W, bias, C, M,
-                  N, K, lda, ldw, ldc, accumulate);
-        return;
+    if (form == F32_WHOLE) {
+        mf_launch(gemm_f32_tile_kernel<BM_, BN_, TM, TN, BKT, AHEAD, F32_WHOLE>, grid, block, 0, stream, A, W, bias, C,
+                  M, N, K, lda, ldw, ldc, accumulate);
+        return 0;
+    }
+    if (form == F32_WALK) {
+        constexpr int done = BM_ * BN_ * (int)sizeof(float);
+        static bool configured[64] = {false};
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MF_ERR_UNSUPPORTED;
+        if (!configured[dev]) {
+            cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<BM_, BN_, TM, TN, BKT, AHEAD, F32_WALK>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, done);
+            if (e != cudaSuccess) return (int)e;
+            configured[dev] = true;
+        }
+        mf_launch(gemm_f32_tile_kernel<BM_, BN_, TM, TN, BKT, AHEAD, F32_WALK>, grid, block, done, stream, A, W, bias,
+                  C, M, N, K, lda, ldw, ldc, accumulate);
+        return 0;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -482,39 +525,58 @@ static void launch_f32_tile(const float* A, const float* W, const float* bias, f
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = mf_pdl_enabled() ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<BM_, BN_, TM, TN, BKT, AHEAD, true>, A, W, bias, C, M, N, K, lda,
-                       ldw, ldc, accumulate);
+    cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<BM_, BN_, TM, TN, BKT, AHEAD, F32_SPLIT>, A, W, bias, C, M, N, K,
+                       lda, ldw, ldc, accumulate);
+    return 0;
 }
 
 // The tile of a float32 product of more than 16 rows (an index into `tiles`; -1: the general kernel, whose
-// grid takes more columns): the one whose fullest SM is done first.  `shared`: what a CTA takes of a full
-// SM.  `few`: what the product takes when its CTAs are few: launched while the kernel before still runs, they
-// pile up on the SMs that are free, as many as one takes (2, 4 and 3 of these tiles).  Both in units of the
-// 64 x 64 tile's share, 27 us a thousand k, fitted to 255 products of 17 to 4,096 rows behind a norm, each
-// timed with every tile: the choice is within 0.1 % of the best tile on average (13 % at worst), and within
-// 1.1 % (21 %) of 109 products back to back; 66 others 0.3 % (6 %) and 0.7 % (24 %).  us, 128 x 128 / 64 x 64 /
-// 32 x 64, norm and product: 200 x 4,096 x 2,048 373 / 224 / 136, 385 x 9,728 x 896 241 / 194 / 205,
-// 385 x 896 x 4,864 467 / 276 / 242, 1,600 x 8,448 x 2,048 1,086 / 1,243 / 1,471.
-static int f32_tile(int M, int N, int sms, int stretches) {
-    static const struct { int bm, bn; double few, shared; } tiles[] = {
-        {128, 128, 6.4, 3.3}, {64, 64, 3.9, 1.0}, {32, 64, 1.8, 0.58}};
-    int best = -1;
+// grid takes more columns) and how it goes through k: what lets the fullest SM be done first.  `shared`: what a
+// CTA takes of a full SM.  `few`: what the product takes when its CTAs are few: launched while the kernel before
+// still runs, they pile up on the SMs that are free, as many as one takes (2, 4 and 3 of these tiles).  Both in
+// units of the 64 x 64 tile's share, 27 us a thousand k, fitted to products behind a norm, each timed with every
+// tile; `cut` the same for a cluster of four CTAs a tile, fitted in the same way to 190 products of 17 to 4,096
+// rows and 2,048 to 18,944 k in both forms.
+//   K below 2,048, 255 products: the choice is within 0.1 % of the best tile on average (13 % at worst), and
+//   within 1.1 % (21 %) of 109 products back to back; 66 others 0.3 % (6 %) and 0.7 % (24 %).
+//   From 2,048 on, 190 products: 0.6 % (16 %) behind a norm, 0.9 % (19 %) back to back.  A cluster a tile
+//   whatever the size, by the numbers of the other form: 1.7 % (25 %) and 1.9 % (24 %); none is slower than
+//   with that by more than 1 %.
+// us, 128 x 128 / 64 x 64 / 32 x 64, norm and product: 385 x 9,728 x 896 241 / 194 / 205; clusters, then one CTA
+// a tile: 200 x 4,096 x 2,048 107 / 116 / 115, 376 / 223 / 135; 385 x 896 x 4,864 248 / 143 / 132,
+// 476 / 273 / 240; 1,600 x 8,448 x 2,048 1,202 / 1,274 / 1,570, 1,099 / 1,242 / 1,476.
+struct F32Cut { int tile, form; };
+static F32Cut f32_cut(int M, int N, int K, int sms) {
+    static const struct { int bm, bn; double few, shared, cut_few, cut_shared; } tiles[] = {
+        {128, 128, 6.4, 3.3, 5.92, 3.18}, {64, 64, 3.9, 1.0, 3.73, 0.921}, {32, 64, 1.8, 0.58, 1.65, 0.598}};
+    F32Cut best = {-1, F32_WHOLE};
     double least = 0.0;
+    const int stretch = f32_stretch(K);
     for (int i = 0; i < 3; ++i) {
         const long long nt = ((long long)N + tiles[i].bn - 1) / tiles[i].bn;
-        const long long mt = ((long long)M + tiles[i].bm - 1) / tiles[i].bm;
+        const long long ctas = ((long long)M + tiles[i].bm - 1) / tiles[i].bm * nt;
         if (nt > 65535) continue;                                    // the grid's second dimension
-        const double share = (double)((nt * mt * stretches + sms - 1) / sms) * tiles[i].shared;
-        const double cost = share > tiles[i].few ? share : tiles[i].few;
-        if (best < 0 || cost < least) { best = i; least = cost; }
+        const double whole = (double)((ctas + sms - 1) / sms) * tiles[i].shared;
+        const double cost = (whole > tiles[i].few ? whole : tiles[i].few) * K;
+        if (best.tile < 0 || cost < least) { best = {i, stretch < K ? F32_WALK : F32_WHOLE}; least = cost; }
+        if (stretch == K) continue;
+        // (49: adding the four parts, in k)
+        const double part = (double)((F32_STRETCHES * ctas + sms - 1) / sms) * tiles[i].cut_shared;
+        const double cut = (part > tiles[i].cut_few ? part : tiles[i].cut_few) * (stretch + 49);
+        if (cut < least) { best = {i, F32_SPLIT}; least = cut; }
     }
     return best;
 }
-extern "C" int mf_gemm_f32_tile(int M, int N, int sms) { return f32_tile(M, N, sms, 1); }
+// `form` receives 0 (K as one stretch), 1 (a cluster a tile) or 2 (one CTA a tile, four stretches)
+extern "C" int mf_gemm_f32_tile(int M, int N, int K, int sms, int* form) {
+    const F32Cut c = f32_cut(M, N, K, sms);
+    *form = c.form;
+    return c.tile;
+}
 
 // Float32 operands whose rows start on 16 bytes; false: the general kernel has to run.
 static bool launch_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
-                       long long lda, long long ldw, long long ldc, int accumulate, cudaStream_t stream) {
+                       long long lda, long long ldw, long long ldc, int accumulate, cudaStream_t stream, int* err) {
     if (((uintptr_t)A | (uintptr_t)W) & 15 || (K | lda | ldw) & 3) return false;
     if (M <= 16) {
         const int warps = (int)(((long long)N + 7) / 8);
@@ -531,14 +593,17 @@ static bool launch_f32(const float* A, const float* W, const float* bias, float*
 #undef MF_FEW
         return true;
     }
-    // (four CTAs a tile, each with a quarter of the work: the same comparison at four times the CTAs)
-    const int best = f32_tile(M, N, mf_sm_count(), f32_stretch(K) < K ? F32_STRETCHES : 1);
-    switch (best) {
-        case 0: launch_f32_tile<128, 128, 8, 8, 16, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;
-        case 1: launch_f32_tile<64, 64, 4, 8, 32, 1>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;
-        case 2: launch_f32_tile<32, 64, 4, 4, 32, 2>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, stream); break;
+    const F32Cut cut = f32_cut(M, N, K, mf_sm_count());
+#define MF_TILE(BM_, BN_, TM, TN, BKT, AHEAD)                                                              \
+    *err = launch_f32_tile<BM_, BN_, TM, TN, BKT, AHEAD>(A, W, bias, C, M, N, K, lda, ldw, ldc, accumulate, \
+                                                         cut.form, stream)
+    switch (cut.tile) {
+        case 0: MF_TILE(128, 128, 8, 8, 16, 1); break;
+        case 1: MF_TILE(64, 64, 4, 8, 32, 1); break;
+        case 2: MF_TILE(32, 64, 4, 4, 32, 2); break;
         default: return false;
     }
+#undef MF_TILE
     return true;
 }
 
@@ -549,9 +614,10 @@ extern "C" int mf_gemm_simt(const void* A, int a_dtype, const void* W, int w_dty
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return MF_ERR_ARGUMENT;
     if (accumulate && c_dtype != MF_DTYPE_F32) return MF_ERR_UNSUPPORTED;
+    int err = 0;
     if (a_dtype == MF_DTYPE_F32 && w_dtype == MF_DTYPE_F32 && c_dtype == MF_DTYPE_F32 &&
-        launch_f32((const float*)A, (const float*)W, bias, (float*)C, M, N, K, lda, ldw, ldc, accumulate, stream))
-        return MF_LAUNCH_CHECK();
+        launch_f32((const float*)A, (const float*)W, bias, (float*)C, M, N, K, lda, ldw, ldc, accumulate, stream, &err))
+        return err != 0 ? err : MF_LAUNCH_CHECK();
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return MF_ERR_UNSUPPORTED;
 #define MF_GEMM(TA, TW, TC)                                                                                   \

@@ -669,8 +669,10 @@ def float32_products(reps):
     """Float32 products behind a norm and alone, with the tile each size takes."""
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     names = {0: "128 x 128", 1: "64 x 64", 2: "32 x 64", -1: "general"}
-    for m, n, k in ((8, 896, 4864), (64, 896, 4864), (200, 4096, 2048), (385, 1152, 896), (385, 9728, 896),
-                    (385, 896, 4864), (385, 151936, 896), (1600, 8448, 2048), (4096, 9728, 896)):
+    forms = {0: "", 1: ", a cluster a tile", 2: ", four stretches a CTA"}
+    for m, n, k in ((8, 896, 896), (8, 896, 4864), (64, 896, 4864), (200, 4096, 2048), (385, 1152, 896), (385, 9728, 896),
+                    (385, 896, 4864), (385, 151936, 896), (512, 18944, 3584), (634, 6420, 2080), (1600, 2048, 8448),
+                    (1600, 8448, 2048), (4096, 9728, 896)):
         h, g = torch.randn(m, k, device="cuda"), torch.rand(k, device="cuda")
         x, w = torch.empty(m, k, device="cuda"), torch.randn(n, k, device="cuda")
         out = torch.empty(m, n, device="cuda")
@@ -679,9 +681,15 @@ def float32_products(reps):
             K.rmsnorm(h, g, 1e-5, x)
             K.gemm_simt(x, w, None, out)
         after, alone = _time(both, reps), _time(lambda: K.gemm_simt(x, w, None, out), reps)
-        tile = "few rows" if m <= 16 else names[K._lib("gemm_simt").mf_gemm_f32_tile(m, n, sms)]
+        tile, form = K.gemm_f32_cut(m, n, k, sms)
+        tile = "few rows" if m <= 16 else names[tile] + forms[form]
         print(f"float32 {m} x {n} x {k} ({tile}): norm and product {after:.1f} us, product alone {alone:.1f} us, "
               f"{2.0 * m * n * k / alone / 1e6:.1f} TFLOP/s")
+    for m, n, k in ((8, 896, 4864), (385, 3028, 10600), (1024, 2048, 2048)):        # the general kernel
+        x, w = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, k, device="cuda")
+        out = torch.empty(m, n, device="cuda")
+        us = _time(lambda: K.gemm_simt(x, w, None, out), reps)
+        print(f"bfloat16 x float32 {m} x {n} x {k}: {us:.1f} us, {2.0 * m * n * k / us / 1e6:.1f} TFLOP/s")
 
 
 def _rows(lens):

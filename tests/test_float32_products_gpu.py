@@ -59,3 +59,52 @@ def test_mixed_types_have_the_bits_of_float32(m, n, k):
     K.gemm_simt(x, w.float(), None, half, False)
     K.gemm_simt(x.float(), w.float(), None, want, False)
     assert torch.equal(half, want.bfloat16())
+
+
+@pytest.mark.parametrize("m,n,k,cut", [(485, 2173, 2180, (0, 1)), (390, 9001, 2052, (0, 2)), (700, 900, 2052, (1, 1)),
+                                       (1600, 1157, 2052, (1, 2)), (64, 899, 2052, (2, 1)), (41, 12001, 2052, (2, 2))])
+def test_every_tile_in_both_forms(m, n, k, cut):
+    """Rows, columns and the last stretch end inside a tile: bias and accumulation, the bits of up to 16 rows,
+    a guard around the output."""
+    from minfer_b200.kernels import api as K
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert K.gemm_f32_cut(m, n, k, 148) == cut
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    x = torch.randn(m, k, generator=g, device="cuda")
+    w = torch.randn(n, k, generator=g, device="cuda") * k ** -0.5
+    bias, old = torch.randn(n, generator=g, device="cuda"), torch.randn(m, n, generator=g, device="cuda")
+    want = x.double() @ w.double().t() + bias.double()
+    for accumulate in (False, True):
+        room = torch.full((m + 2, n + 3), 5.0, device="cuda")
+        out = room[1:m + 1, :n]
+        out.copy_(old)
+        K.gemm_simt(x, w, bias, out, accumulate)
+        whole = want + old.double() if accumulate else want
+        # as above, and one rounding of the largest value for each addition behind the products
+        assert float((out.double() - whole).abs().max()) < 2 ** -24 * (k / 4 + 133) * float(whole.abs().max())
+        assert float((room[0] - 5).abs().max()) == float((room[m + 1] - 5).abs().max()) == 0.0
+        assert float((room[:, n:] - 5).abs().max()) == 0.0
+        for lo in (0, m // 2, m - 9):
+            few = old[lo:lo + 9].clone()
+            K.gemm_simt(x[lo:lo + 9], w, bias, few, accumulate)
+            assert torch.equal(few, out[lo:lo + 9])
+
+
+@pytest.mark.parametrize("m,n,k", [(5, 896, 4864), (64, 896, 4864), (41, 12001, 2052), (390, 9001, 2052)])
+def test_products_of_a_long_k_wait_for_the_kernel_that_writes_their_input(m, n, k):
+    """Launched while a norm still writes the rows it reads: up to 16 rows, a cluster a tile, four stretches a CTA."""
+    from minfer_b200.kernels import api as K
+    g = torch.Generator(device="cuda").manual_seed(m)
+    h, w = torch.randn(m, k, generator=g, device="cuda"), torch.randn(n, k, generator=g, device="cuda")
+    scale = torch.rand(k, generator=g, device="cuda")
+    x, out = torch.empty(m, k, device="cuda"), torch.empty(m, n, device="cuda")
+    K.rmsnorm(h, scale, 1e-5, x)
+    torch.cuda.synchronize()
+    K.gemm_simt(x, w, None, out)
+    torch.cuda.synchronize()
+    want = out.clone()
+    for _ in range(20):
+        x.fill_(float("nan"))
+        K.rmsnorm(h, scale, 1e-5, x)
+        K.gemm_simt(x, w, None, out)
+        assert torch.equal(out, want)
