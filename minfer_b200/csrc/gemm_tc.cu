@@ -1619,16 +1619,17 @@ extern "C" long long mf_gemm_tc_workspace_floats(int M, int N, int K, int epi) {
 struct FewPlan { int row_tiles, warp_units, tok_stride, depth, cluster, groups; size_t smem; };
 static int g_few_mode = 1;                // 0 never, 1 where the rule says so, 2 also below FEW_MIN_BYTES (tests, measurement)
 extern "C" void mf_gemm_few_mode(int mode) { g_few_mode = mode; }
-static FewPlan few_plan(int M, int N, int K) {
+static FewPlan few_plan(int M, int N, int K, int sms) {
     FewPlan p = {0, 0, 0, 0, 0, 0, 0};
     if (g_few_mode == 0 || M < 1 || M > FEW_MAX_M || N < 1 || K < 1) return p;
     const long long bytes = (long long)N * K * 2;
     // (with two tiles of tokens an SM reads twice as much shared memory for a byte of weights: 16 tokens, 7B
     // q|k|v of 33 MB 11.4 -> 12.1 us, O of 26 MB 8.5 -> 10.3; 0.5B shape's layer 24.4 -> 20.9)
     if (bytes > (M <= 8 ? FEW_MAX_BYTES : FEW_MAX_BYTES / 4) || (bytes < FEW_MIN_BYTES && g_few_mode != 2)) return p;
-    const int units = (K + 63) / 64, tiles = (N + 7) / 8, sms = sm_count();
+    const int units = (K + 63) / 64, tiles = (N + 7) / 8;
     for (int cluster = 1; cluster <= 4; cluster *= 2) {
-        const int slots = cluster == 4 ? (sms - 16) / 4 : sms / cluster;       // clusters that fit at once
+        int slots = cluster == 4 ? (sms - 16) / 4 : sms / cluster;             // clusters that fit at once
+        if (slots < 1) slots = 1;
         const int rt = (tiles + slots - 1) / slots, wu = (units + cluster * FEW_WARPS - 1) / (cluster * FEW_WARPS);
         const int stride = 8 * (rt | 1);
         const size_t fixed = sizeof(float) * ((size_t)FEW_WARPS * M * stride + 16 + (size_t)M * rt +
@@ -1640,21 +1641,23 @@ static FewPlan few_plan(int M, int N, int K) {
             depth = d;
             if (d >= rt * wu) break;
         }
-        const int groups = (tiles + rt - 1) / rt;
         if (fixed + (size_t)FEW_WARPS * depth * 1024 > FEW_BUDGET) continue;
+        p.row_tiles = rt; p.warp_units = wu; p.tok_stride = stride; p.depth = depth; p.cluster = cluster;
+        p.groups = (tiles + rt - 1) / rt; p.smem = fixed + (size_t)FEW_WARPS * depth * 1024;
         // K is cut between CTAs only where one CTA's share of the tokens does not fit, or where the rows
         // alone leave a quarter of the SMs without work and K is long
-        const bool idle = groups * cluster * 4 < sms * 3 && wu > 4;
-        if (p.groups == 0 || !idle) {
-            p.row_tiles = rt; p.warp_units = wu; p.tok_stride = stride; p.depth = depth; p.cluster = cluster;
-            p.groups = groups; p.smem = fixed + (size_t)FEW_WARPS * depth * 1024;
-        }
-        if (!idle) break;
+        if (p.groups * cluster * 4 >= sms * 3 || wu <= 4) break;
     }
     return p;
 }
 // Column groups of a product of these sizes on gemm_few_kernel, 0: another kernel takes it.
-extern "C" int mf_gemm_few_groups(int M, int N, int K) { return few_plan(M, N, K).groups; }
+extern "C" int mf_gemm_few_groups(int M, int N, int K) { return few_plan(M, N, K, sm_count()).groups; }
+// The same on a GPU of `sms` SMs; `cluster` receives the number of CTAs that cut K between them.
+extern "C" int mf_gemm_few_plan(int M, int N, int K, int sms, int* cluster) {
+    const FewPlan p = few_plan(M, N, K, sms);
+    *cluster = p.cluster;
+    return p.groups;
+}
 
 template <int NT, int DEPTH>
 static int launch_few(const FewPlan& p, const FewArgs& f, const GemmArgs& a, cudaStream_t stream) {
@@ -1716,7 +1719,7 @@ static int pair_mode_on() {
 // the product in the ordinary way and runs the norm as a kernel).
 extern "C" int mf_gemm_tc_prep_parts(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
-    if (const int groups = few_plan(M, N, K).groups) return groups;
+    if (const int groups = few_plan(M, N, K, sm_count()).groups) return groups;
     int nt, splits;
     mf_gemm_tc_plan(M, N, K, EPI_ACCUM, &nt, &splits);
     const int kblocks = (K + TILE_K - 1) / TILE_K;
@@ -1753,7 +1756,7 @@ static int gemm_tc_impl(const void* x, long long ldx, const void* w, long long l
     int nt, splits;
     mf_gemm_tc_plan(M, N, K, epi, &nt, &splits);
     // (a caller that wants the K splits for its next kernel gets them from the kernel that splits)
-    const FewPlan few = deferred == nullptr ? few_plan(M, N, K) : FewPlan{0, 0, 0, 0, 0, 0, 0};
+    const FewPlan few = deferred == nullptr ? few_plan(M, N, K, sm_count()) : FewPlan{0, 0, 0, 0, 0, 0, 0};
     if (splits > 1 && workspace == nullptr && !prep && few.groups == 0) return MF_ERR_ARGUMENT;
     CUtensorMap mw, mx;
     if (few.groups == 0)

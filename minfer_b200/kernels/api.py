@@ -291,6 +291,7 @@ def _sig_gemm_tc(lib: ctypes.CDLL) -> None:
                                      c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p]
     lib.mf_gemm_tc_prep_parts.argtypes = [c_int, c_int, c_int]
     lib.mf_gemm_few_groups.argtypes = [c_int, c_int, c_int]
+    lib.mf_gemm_few_plan.argtypes = [c_int, c_int, c_int, c_int, c_void_p]
     lib.mf_gemm_few_mode.argtypes = [c_int]
     lib.mf_gemm_few_mode.restype = None
     lib.mf_wait_probe.argtypes = [c_void_p, ctypes.c_uint, c_ulonglong, c_void_p, c_void_p]
@@ -684,6 +685,13 @@ def gemm_few_groups(m: int, n: int, k: int) -> int:
     if got is None:
         got = _FEW[key] = int(_lib("gemm_tc").mf_gemm_few_groups(m, n, k))
     return got
+
+
+def gemm_few_plan(m: int, n: int, k: int, sms: int) -> tuple[int, int]:
+    """The column groups of ``gemm_few_groups`` on a GPU of ``sms`` SMs, and the CTAs that cut K between them."""
+    cluster = ctypes.c_int(0)
+    groups = int(_lib("gemm_tc").mf_gemm_few_plan(m, n, k, sms, ctypes.addressof(cluster)))
+    return groups, cluster.value
 
 
 def gemm_few_mode(mode: int) -> None:

@@ -107,3 +107,24 @@ def test_cut_of_single_queries(rows, kv, reach, tiles, splits):
                                                     ctypes.addressof(out) + 4)
     assert tuple(out) == (tiles, splits)
     assert tiles * splits * 32 >= reach + 31                 # the reach need not start on a tile
+
+
+@pytest.mark.parametrize("m,n,k,groups,cluster", [
+    # 512 KB to 64 MB of weights, 16 MB beyond 8 tokens
+    (1, 256, 1016, 0, 0), (1, 256, 1024, 32, 1), (8, 16384, 2048, 147, 1), (8, 16896, 2048, 0, 0),
+    (8, 9728, 896, 136, 1), (9, 9728, 896, 0, 0), (9, 9360, 896, 147, 1), (8, 3584, 3584, 112, 1), (9, 3584, 3584, 0, 0),
+    (16, 1152, 896, 144, 1), (17, 1152, 896, 0, 0),
+    # K cut between CTAs: the tokens of one do not fit, or few rows and a long K (the largest cluster where none
+    # fills the GPU)
+    (8, 896, 4864, 112, 1), (16, 896, 4864, 56, 2), (8, 2048, 8448, 128, 1), (1, 88, 4496, 11, 2), (8, 144, 8840, 18, 4),
+    (1, 72, 17632, 9, 4), (3, 40, 20000, 5, 4),
+])
+def test_products_for_a_handful_of_tokens(m, n, k, groups, cluster):
+    assert K.gemm_few_plan(m, n, k, SMS) == (groups, cluster)
+
+
+@pytest.mark.parametrize("sms", [1, 2, 3, 15, 16, 17, 19, 20, 148, 300])
+def test_the_cut_for_a_handful_of_tokens_on_any_number_of_sms(sms):
+    for m, n, k in ((1, 1152, 896), (16, 896, 4864), (3, 40, 20000), (8, 2048, 8448)):
+        groups, cluster = K.gemm_few_plan(m, n, k, sms)
+        assert (groups == 0) == (cluster == 0) and groups <= (n + 7) // 8
