@@ -777,7 +777,8 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 //     reproducible, and complete, so no next kernel has K splits to add.
 // Bound by latency: what is left after the wait is a trip for the tokens, the MMAs, the warps' sums and a
 // store.  Measured, us a layer's products in a chain (q|k|v, O, gate|up, down), tcgen05 tiles -> here, 1 / 8
-// tokens: 0.5B shape 23.3 -> 17.9 / 24.0 -> 18.0; width 2,048, feed-forward 8,448 39.2 -> 34.6 / 41.0 -> 37.2;
+// tokens: 0.5B shape 23.3 -> 17.9 / 24.0 -> 18.0; width 2,048, feed-forward 8,448 (gate|up,
+// 66 MB, stays on the tcgen05 tiles) 39.2 -> 34.6 / 41.0 -> 37.2;
 // 7B (q|k|v and O only) 86.4 -> 82.3 / 87.5 -> 82.8.  q|k|v of the 0.5B shape alone 5.8 -> 2.3.
 // Slower: the weights in registers instead of shared memory (27.4), 16 rows a tile (22.4), 8 warps (19.6),
 // two CTAs of 8 warps an SM (18.6), registers for two CTAs of 16 and the rest of the weights asked for in L2
@@ -1617,7 +1618,8 @@ extern "C" long long mf_gemm_tc_workspace_floats(int M, int N, int K, int epi) {
 
 // How gemm_few_kernel cuts a product, or groups 0: another kernel takes it.
 struct FewPlan { int row_tiles, warp_units, tok_stride, depth, cluster, groups; size_t smem; };
-static int g_few_mode = 1;                // 0 never, 1 where the rule says so, 2 also below FEW_MIN_BYTES (tests, measurement)
+static int g_few_mode = 1;                // 0 never, 1 where the rule says so, 2 also those
+                                          // below FEW_MIN_BYTES or of many rows and a short K (tests, measurement)
 extern "C" void mf_gemm_few_mode(int mode) { g_few_mode = mode; }
 static FewPlan few_plan(int M, int N, int K, int sms) {
     FewPlan p = {0, 0, 0, 0, 0, 0, 0};
@@ -1627,6 +1629,12 @@ static FewPlan few_plan(int M, int N, int K, int sms) {
     // q|k|v of 33 MB 11.4 -> 12.1 us, O of 26 MB 8.5 -> 10.3; 0.5B shape's layer 24.4 -> 20.9)
     if (bytes > (M <= 8 ? FEW_MAX_BYTES : FEW_MAX_BYTES / 4) || (bytes < FEW_MIN_BYTES && g_few_mode != 2)) return p;
     const int units = (K + 63) / 64, tiles = (N + 7) / 8;
+    // A row tile takes a CTA 0.2 us (0.4 with two tiles of tokens) to sum and store, whatever K is, and a short K
+    // leaves warps without work: many rows of a short K go to the tcgen05 tiles.  us there / here, one head (float32
+    // out) of 1 and of 9 tokens: 32,000 x 256 6.0 / 7.7 and 6.5 / 13.6, 16,000 x 192 4.6 / 4.8 and 4.8 / 5.9, 16,000 x
+    // 256 (K splits to add there) 6.7 / 4.9 and 7.9 / 6.0 - but gated 4.6 / 5.0 and 4.6 / 5.7; 32,000 x 1,024 13.6 / 12.1.
+    const long long each = (tiles + sms - 1) / sms;
+    if (g_few_mode != 2 && 5ll * K < (M <= 8 ? 6 : 25) * each * each) return p;
     for (int cluster = 1; cluster <= 4; cluster *= 2) {
         int slots = cluster == 4 ? (sms - 16) / 4 : sms / cluster;             // clusters that fit at once
         if (slots < 1) slots = 1;
@@ -1645,7 +1653,7 @@ static FewPlan few_plan(int M, int N, int K, int sms) {
         p.row_tiles = rt; p.warp_units = wu; p.tok_stride = stride; p.depth = depth; p.cluster = cluster;
         p.groups = (tiles + rt - 1) / rt; p.smem = fixed + (size_t)FEW_WARPS * depth * 1024;
         // K is cut between CTAs only where one CTA's share of the tokens does not fit, or where the rows
-        // alone leave a quarter of the SMs without work and K is long
+        // alone leave a quarter of the SMs without work and K is long (4 x 40 x 20,000 one CTA a row tile 9.8 us, four 5.0)
         if (p.groups * cluster * 4 >= sms * 3 || wu <= 4) break;
     }
     return p;

@@ -696,7 +696,7 @@ def gemm_few_plan(m: int, n: int, k: int, sms: int) -> tuple[int, int]:
 
 def gemm_few_mode(mode: int) -> None:
     """0: the kernel for a handful of tokens takes no product; 1: those its rule names (the default); 2: smaller
-    ones too."""
+    ones and those of many rows and a short K too."""
     _lib("gemm_tc").mf_gemm_few_mode(int(mode))
     _FEW.clear()
     _PREP_PARTS.clear()

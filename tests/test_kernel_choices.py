@@ -114,6 +114,9 @@ def test_cut_of_single_queries(rows, kv, reach, tiles, splits):
     (1, 256, 1016, 0, 0), (1, 256, 1024, 32, 1), (8, 16384, 2048, 147, 1), (8, 16896, 2048, 0, 0),
     (8, 9728, 896, 136, 1), (9, 9728, 896, 0, 0), (9, 9360, 896, 147, 1), (8, 3584, 3584, 112, 1), (9, 3584, 3584, 0, 0),
     (16, 1152, 896, 144, 1), (17, 1152, 896, 0, 0),
+    # many rows and a short K: heads of small models
+    (1, 8192, 64, 147, 1), (1, 16000, 64, 0, 0), (8, 16000, 192, 0, 0), (8, 16000, 256, 143, 1), (1, 32000, 768, 0, 0),
+    (1, 32000, 1024, 143, 1), (1, 152064, 128, 0, 0), (9, 8192, 192, 0, 0), (9, 8192, 256, 147, 1), (9, 16000, 512, 0, 0),
     # K cut between CTAs: the tokens of one do not fit, or few rows and a long K (the largest cluster where none
     # fills the GPU)
     (8, 896, 4864, 112, 1), (16, 896, 4864, 56, 2), (8, 2048, 8448, 128, 1), (1, 88, 4496, 11, 2), (8, 144, 8840, 18, 4),
