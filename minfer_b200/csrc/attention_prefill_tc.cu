@@ -224,7 +224,7 @@ template <int HD, bool PAGED, bool MOD>
 __global__ void __launch_bounds__(FA_THREADS, 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const FaArgs a) {
-    pdl_wait();
+    pdl_prologue();
     constexpr int NB = HD / 64;                         // 64-column blocks per row
     constexpr int BLOCK = 128 * 128;                    // bytes of a [128 rows][64 cols] block
     constexpr int T_BYTES = NB * BLOCK;                 // a [128 rows][HD] tile
@@ -318,9 +318,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     }
     fa_fence_before();
     __syncthreads();
-    // The next kernel may start from here on, not earlier: a product's CTA allocates tensor memory before it
-    // waits, and on an SM it shares with this one (head size 64) could leave none.
-    pdl_launch_dependents();
     fa_fence_after();
     const uint32_t tmem = *tmem_slot;
 
@@ -669,7 +666,11 @@ static int fa_cache_map(CUtensorMap* map, const void* ptr, long long rows, int h
 template <int HD, bool PAGED, bool MOD = false>
 static int fa_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FaArgs& a,
                      int n_seqs, int max_len, cudaStream_t stream) {
-    constexpr int smem = (HD / 64) * 16384 * 6 + 1024 + 256 + (MOD ? (FA_TAB_MAX + 2 * FA_TAB_PAD) * 4 : 0);
+    constexpr int used = (HD / 64) * 16384 * 6 + 1024 + 256 + (MOD ? (FA_TAB_MAX + 2 * FA_TAB_PAD) * 4 : 0);
+    // All columns are allocated behind the wait, the next kernel let on before it: no other CTA with tensor memory
+    // may share the SM (head size 64 uses 98 KB).  Let on only once they are allocated, a prompt of 64 tokens and
+    // the product behind it took 18.4 -> 21.1 us (28 heads of 128), 16.3 -> 19.1 (14 of 64); now 17.9 and 16.0.
+    constexpr int smem = used > MF_TMEM_SMEM_ALONE ? used : MF_TMEM_SMEM_ALONE;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, PAGED, MOD>,

@@ -108,6 +108,15 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// Shared memory (bytes) and tensor memory.  A kernel lets the next one start early, whose CTAs may allocate tensor
+// memory before they wait.  Were such a CTA on an SM beside one that has not allocated its own yet, it could take
+// columns that one waits for, and wait for it: neither would go on.  So every kernel with tensor memory asks for
+// MF_TMEM_SMEM at least, and one that lets the next kernel on before it has allocated most of the columns for
+// MF_TMEM_SMEM_ALONE: an SM (228 KB, 1 KB of them kept back for each CTA) has no room for the two.
+#define MF_TMEM_SMEM (96 * 1024)
+#define MF_TMEM_SMEM_ALONE (132 * 1024)
+static_assert(MF_TMEM_SMEM + MF_TMEM_SMEM_ALONE + 2 * 1024 > 228 * 1024, "both fit an SM");
+
 __device__ __forceinline__ void pdl_prologue() {
     pdl_launch_dependents();
     pdl_wait();

@@ -1144,6 +1144,7 @@ template <int NT, int STAGES>
 static int launch_grouped(const CUtensorMap& mw, const CUtensorMap& mx, const GemmArgs& a, int tiles,
                           cudaStream_t stream) {
     constexpr int smem = STAGES * (A_BYTES + NT * TILE_K * 2) + 1024 + 256 + NT * 4;
+    static_assert(smem >= MF_TMEM_SMEM, "see MF_TMEM_SMEM_ALONE");
     static bool configured[64] = {false};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MF_ERR_UNSUPPORTED;
@@ -1162,6 +1163,7 @@ template <int NT, int STAGES>
 static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const GemmArgs& a, int splits,
                   cudaStream_t stream) {
     constexpr int smem = STAGES * (A_BYTES + NT * TILE_K * 2) + 1024 + 256 + NT * 4;
+    static_assert(smem >= MF_TMEM_SMEM, "see MF_TMEM_SMEM_ALONE");
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<NT, STAGES>,
@@ -1179,6 +1181,7 @@ template <int NT, int STAGES>
 static int launch_cluster(const CUtensorMap& mw, const CUtensorMap& mx, const GemmArgs& a,
                           cudaStream_t stream) {
     constexpr int smem = STAGES * (A_BYTES + NT * TILE_K * 2) + TILE_N * NT * 4 + 1024 + 256 + NT * 4 + NT * 2;
+    static_assert(smem >= MF_TMEM_SMEM, "see MF_TMEM_SMEM_ALONE");
     static bool configured[64] = {false};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return MF_ERR_UNSUPPORTED;
@@ -1315,6 +1318,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
     const int kblocks = (a.K + TILE_K - 1) / TILE_K;
 
+    pdl_launch_dependents();                                  // (no other CTA with tensor memory fits beside this one)
     // The barriers, and the weights of the first stages, which no kernel of the step writes: before the wait
     // for the kernel before.
     if (tid == 0) {
@@ -1356,8 +1360,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();                                       // both CTAs have their tensor memory
-    // ... and only now the next kernel may come onto this SM, which may allocate before it waits
-    pdl_launch_dependents();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
@@ -1490,6 +1492,7 @@ static int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const GemmA
                        cudaStream_t stream) {
     constexpr int smem = STAGES * (A_BYTES + (DUAL ? 2 : 1) * (NT / 2) * TILE_K * 2) + 1024 + 256;
     static_assert(smem <= 227 * 1024, "the ring does not fit an SM's shared memory");
+    static_assert(smem >= MF_TMEM_SMEM_ALONE, "a kernel with tensor memory may share the SM");
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<NT, STAGES, DUAL>,
