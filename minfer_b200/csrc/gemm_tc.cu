@@ -1522,52 +1522,61 @@ static int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const GemmA
 static int sm_count() { return mf_sm_count(); }
 
 // How the CTA-pair kernel cuts a product: the token tile and whether a pair takes two token
-// tiles at once (DUAL).  A model of the kernel's time picks them; its figures are measured on
-// this kernel (2,048 to 8,192 tokens, K 1,792 to 18,944):
+// tiles at once (DUAL).  A model of the kernel's time picks them (ns; fitted to 535 products of 256 to
+// 8,192 tokens behind a norm, each timed with every tile in both forms):
 //   * operand bytes: every k-block a pair pulls 256 weight rows and its tokens' rows, 128 bytes
-//     each, through L2, and all pairs together get 11.8 TB/s (a 208-token tile takes 0.905 of a
-//     256-token one: the ratio of the bytes, not of the flops);
-//   * tensor cores: 23.4 TFLOP/s a pair with every pair at work (the clock under load);
-//   * rounds: the pairs walk the tiles in step, so the last round counts in full
-//     (14 weight tiles x 8 token tiles of 256 are 112 tiles for 74 pairs; 10 token tiles of 208
-//     are 140 tiles and two full rounds);
+//     each, through L2, and all pairs together get 11.8 TB/s;
+//   * tensor cores: 24.7 TFLOP/s a pair and 32 ns a k-block for the hand-over between the roles;
+//   * rounds: the pairs walk the tiles in step, so the last round counts in full, and each takes
+//     2 us beside its k-blocks; a tile's epilogue, 1.6 us for 256 tokens at least, hides behind the
+//     next tile's main loop only where that is as long;
 //   * what is not hidden: the last tile's epilogue, and with DUAL every tile's (both
 //     accumulators are in use, so none is free for the next tile's main loop).
-// DUAL therefore wins where the tiles make one or two rounds, the more the longer K is (the
-// down projection of a 2,048-token prompt: 181 against 217 us; the O projection: 44 against 50);
-// it is not considered beyond two rounds.  An element's sum does not depend
-// on the cut (k ascending, one accumulator), so the choice changes no bits.
+// DUAL is not considered beyond two rounds, and with 176 tokens not below 4,096 k: 1,300 x 4,608 x 3,584 51 us, 46 with
+// tiles of 192 (but 1,024 x 5,120 x 13,824 136, 147 with DUAL of 192; 3,000 x 2,048 x 5,632 85, 93 likewise).
+// The choice is within 1.7 % of the best one on average (24 % at worst).  Before (23.4 TFLOP/s, neither k-blocks nor
+// rounds with a time of their own) it was 3.0 %, and the tile of 176, offered by that model, lost 10 to 13 % where it
+// left more pairs idle in the same round: 515 x 3,584 x 3,584 24.9 -> 28.1 us (tile of 160), 700 x 3,072 x 2,048 20.6 -> 22.6.
+// Against that choice none of the 535, and none of 153 that are gated or complete a residual, is slower, and all of them
+// take 0.99 of the time: 1,024 x 11,264 x 2,048 61 -> 56 us, 515 x 7,168 x 5,120 55 -> 52 (norm and product).  An element's
+// sum does not depend on the cut (k ascending, one accumulator), so the choice changes no bits.
 struct PairPlan { int nt; int dual; };
 static int g_pair_dual = -1;              // 0 never, 1 where the model says so, 2 always
 // MINFER_B200_PAIR_DUAL or this call (tests compare the two forms bit for bit) sets the mode.
 extern "C" void mf_gemm_pair_dual_mode(int mode) { g_pair_dual = mode; }
-static PairPlan pair_plan(int M, int N, int K) {
+static int g_pair_tile = 0;               // > 0: the token tile, one of the candidates (tests, measurement)
+extern "C" void mf_gemm_pair_tile(int token_tile) { g_pair_tile = token_tile; }
+static PairPlan pair_plan(int M, int N, int K, int sms) {
     static const int candidates[] = {256, 224, 208, 192, 176, 160};
     if (g_pair_dual < 0) { const char* ev = getenv("MINFER_B200_PAIR_DUAL"); g_pair_dual = ev ? atoi(ev) : 1; }
     const int allow_dual = g_pair_dual;
-    const double pairs = sm_count() / 2, tiles_n = (N + 255) / 256, kb = (K + TILE_K - 1) / TILE_K;
-    const double l2_bytes_per_ns = 11800.0 * (pairs / 74.0), pair_flops_per_ns = 23400.0;
+    const double pairs = sms / 2, tiles_n = (N + 255) / 256, kb = (K + TILE_K - 1) / TILE_K;
+    const double l2_bytes_per_ns = 11800.0 * (pairs / 74.0), pair_flops_per_ns = 24700.0;
     PairPlan best = {256, 0};
     double best_cost = -1.0;
     for (int dual = allow_dual == 2 ? 1 : 0; dual <= (allow_dual ? 1 : 0); ++dual)
         for (int nt : candidates) {
+            if (g_pair_tile > 0 && nt != g_pair_tile) continue;
             const int step = (dual ? 2 : 1) * nt;
             const double tiles = (double)((M + step - 1) / step) * tiles_n;
             const double rounds = (double)(long long)((tiles + pairs - 1) / pairs);
             const double bytes = 128.0 * (256 + step), flops = 2.0 * 256 * step * TILE_K;
             const double l2 = tiles * kb * bytes / l2_bytes_per_ns;
-            const double tc = rounds * kb * flops / pair_flops_per_ns;
-            const double epilogue = (dual ? rounds * 11600.0 : 4000.0) * nt / 256.0;
-            double cost = (l2 > tc ? l2 : tc) + epilogue;
-            if (dual && rounds > 2 && allow_dual != 2) continue;   // measured for one and two rounds only
+            const double tc = rounds * kb * (flops / pair_flops_per_ns + 32.0);
+            const double hidden = dual ? 0.0 : rounds * 1550.0 * nt / 256.0;         // epilogues behind main loops
+            const double epilogue = (dual ? rounds * 18800.0 : 8000.0) * nt / 256.0;
+            double cost = l2 > tc ? l2 : tc;
+            cost = (hidden > cost ? hidden : cost) + epilogue + rounds * 2050.0;
+            if (dual && allow_dual != 2 && (rounds > 2 || (nt == 176 && kb < 64))) continue;
             if (best_cost < 0 || cost < best_cost) { best = {nt, dual}; best_cost = cost; }
         }
     return best;
 }
 
-// The cut of the CTA-pair kernel for these sizes (it runs products of 256 tokens and more).
-extern "C" int mf_gemm_pair_plan(int M, int N, int K, int* token_tile, int* dual) {
-    const PairPlan pp = pair_plan(M, N, K);
+// The cut of the CTA-pair kernel for these sizes (it runs products of 256 tokens and more) on a GPU of `sms` SMs
+// (0: this one).
+extern "C" int mf_gemm_pair_plan(int M, int N, int K, int sms, int* token_tile, int* dual) {
+    const PairPlan pp = pair_plan(M, N, K, sms > 0 ? sms : sm_count());
     *token_tile = pp.nt;
     *dual = pp.dual;
     return 0;
@@ -1788,7 +1797,7 @@ static int gemm_tc_impl(const void* x, long long ldx, const void* w, long long l
     }
     if (pair_mode_on() && M >= 256 && splits == 1) {
         if (a.row_ssq != nullptr) return MF_ERR_UNSUPPORTED;     // the CTA-pair kernel applies no row scale
-        const PairPlan pp = pair_plan(M, N, K);
+        const PairPlan pp = pair_plan(M, N, K, sm_count());
         const int pnt = pp.nt, dual = pp.dual;
         if (int e = make_map(&mx, x, M, K, ldx, pnt / 2)) return e;
         if (dual)

@@ -272,9 +272,11 @@ def _sig_gemm_tc(lib: ctypes.CDLL) -> None:
     lib.mf_gemm_tc_workspace_floats.argtypes = [c_int, c_int, c_int, c_int]
     lib.mf_gemm_tc_workspace_floats.restype = c_longlong
     lib.mf_gemm_tc_plan.argtypes = [c_int, c_int, c_int, c_int, c_void_p, c_void_p]
-    lib.mf_gemm_pair_plan.argtypes = [c_int, c_int, c_int, c_void_p, c_void_p]
+    lib.mf_gemm_pair_plan.argtypes = [c_int, c_int, c_int, c_int, c_void_p, c_void_p]
     lib.mf_gemm_pair_dual_mode.argtypes = [c_int]
     lib.mf_gemm_pair_dual_mode.restype = None
+    lib.mf_gemm_pair_tile.argtypes = [c_int]
+    lib.mf_gemm_pair_tile.restype = None
     lib.mf_gemm_pair_group_m.argtypes = [c_int]
     lib.mf_gemm_pair_group_m.restype = None
     lib.mf_gemm_tc_fused.argtypes = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p,
@@ -654,11 +656,11 @@ def gemm_tc_plan(m: int, n: int, k: int, epi: int = EPI_STORE) -> tuple[int, int
     return _gemm_tc_shape(m, n, k, epi)[:2]
 
 
-def gemm_pair_plan(m: int, n: int, k: int) -> tuple[int, bool]:
+def gemm_pair_plan(m: int, n: int, k: int, sms: int = 0) -> tuple[int, bool]:
     """(token tile, two token tiles a pair at once) of the CTA-pair kernel, which runs products
-    of 256 tokens and more."""
+    of 256 tokens and more; ``sms``: on a GPU of that many SMs instead of this one."""
     nt, dual = ctypes.c_int(0), ctypes.c_int(0)
-    _lib("gemm_tc").mf_gemm_pair_plan(m, n, k, ctypes.addressof(nt), ctypes.addressof(dual))
+    _lib("gemm_tc").mf_gemm_pair_plan(m, n, k, sms, ctypes.addressof(nt), ctypes.addressof(dual))
     return nt.value, bool(dual.value)
 
 
@@ -666,6 +668,14 @@ def gemm_pair_dual_mode(mode: int) -> None:
     """0: a pair never takes two token tiles at once; 1: where the kernel's cost model says so
     (the default); 2: always.  The result's bits are the same in every mode."""
     _lib("gemm_tc").mf_gemm_pair_dual_mode(int(mode))
+
+
+def gemm_pair_tile(token_tile: int) -> None:
+    """The CTA-pair kernel's token tile: 256, 224, 208, 192, 176 or 160 (0: where its cost model says so, the default).
+    The result's bits are the same with every tile."""
+    if token_tile not in (0, 160, 176, 192, 208, 224, 256):
+        raise KernelError(f"gemm: the CTA-pair kernel has no token tile of {token_tile}")
+    _lib("gemm_tc").mf_gemm_pair_tile(int(token_tile))
 
 
 def gemm_pair_group_m(group_m: int) -> None:

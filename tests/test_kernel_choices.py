@@ -131,3 +131,18 @@ def test_the_cut_for_a_handful_of_tokens_on_any_number_of_sms(sms):
     for m, n, k in ((1, 1152, 896), (16, 896, 4864), (3, 40, 20000), (8, 2048, 8448)):
         groups, cluster = K.gemm_few_plan(m, n, k, sms)
         assert (groups == 0) == (cluster == 0) and groups <= (n + 7) // 8
+
+
+@pytest.mark.parametrize("m,n,k,tile,dual", [
+    # the largest tile that leaves no pair idle in the last round ...
+    (2048, 37888, 3584, 256, False), (20011, 3584, 18944, 256, False), (1024, 11264, 2048, 208, False),
+    (515, 27648, 5120, 176, False), (515, 5120, 13824, 176, False),
+    # ... but no larger one that makes fewer tiles of a single round
+    (515, 3584, 3584, 160, False), (700, 3072, 2048, 160, False), (1000, 2048, 5632, 160, False),
+    (515, 7168, 5120, 160, False),
+    # two token tiles a pair: long K, one or two rounds
+    (2048, 3584, 18944, 208, True), (2048, 3584, 3584, 208, True), (1024, 5120, 13824, 176, True),
+    (3000, 2048, 5632, 176, True), (1300, 4608, 3584, 192, False),
+])
+def test_tile_of_a_product_of_a_prompt(m, n, k, tile, dual):
+    assert K.gemm_pair_plan(m, n, k, SMS) == (tile, dual)

@@ -438,6 +438,42 @@ def test_gemm_tensor_core_against_float64(m, n, k):
     assert torch.equal(again, out)
 
 
+@pytest.mark.parametrize("tile", [256, 224, 208, 192, 176, 160])
+@pytest.mark.parametrize("form", [0, 2])
+def test_gemm_pair_kernel_at_every_token_tile(tile, form):
+    """Each token tile, one of them a pair (0) and two (2): full tiles, a last one of one token, of one more than half
+    a tile, of all but one; ragged rows and k; every epilogue against float64, the same bits with every tile."""
+    from minfer_b200.kernels import api as K
+    st = status()
+    for m in (2 * tile + 1, 3 * tile + tile // 2 + 1, 5 * tile - 1):
+        n, k = 364, 456
+        g = torch.Generator().manual_seed(m)
+        x, w = (torch.randn(m, k, generator=g) * 0.5).bfloat16().cuda(), (torch.randn(n, k, generator=g) * 0.5).bfloat16().cuda()
+        bias, start = torch.randn(n, generator=g).cuda(), torch.randn(m, n, generator=g).cuda()
+        want, results = x.double() @ w.double().t(), []
+        try:
+            for force, dual in ((tile, form), (256, 0)):
+                K.gemm_pair_tile(force)
+                K.gemm_pair_dual_mode(dual)
+                assert K.gemm_pair_plan(m, n, k) == (force, dual == 2)
+                out, acc = torch.zeros(m, n, device="cuda"), start.clone()
+                act = torch.zeros(m, n // 2, dtype=torch.bfloat16, device="cuda")
+                K.gemm_tc(x, w, bias, out, K.EPI_STORE, st)
+                K.gemm_tc(x, w, None, acc, K.EPI_ACCUM, st)
+                K.gemm_tc(x, w, None, act, K.EPI_SWIGLU, st)
+                results.append((out, acc, act))
+        finally:
+            K.gemm_pair_tile(0)
+            K.gemm_pair_dual_mode(1)
+        out, acc, act = results[0]
+        close(out, want + bias.double(), torch.float32)
+        close(acc, start.double() + want, torch.float32)
+        close(act, torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2], torch.bfloat16)
+        for a, b in zip(*results):
+            assert torch.equal(a, b)
+    assert int(st) == 0
+
+
 @pytest.mark.parametrize("m,n,k", [(300, 640, 328), (2048, 512, 200), (777, 1000, 520),
                                    (256, 256, 64), (1300, 768, 1024), (3000, 300, 136)])
 def test_gemm_pair_kernel_two_token_tiles_at_once(m, n, k):
