@@ -567,8 +567,10 @@ static F32Cut f32_cut(int M, int N, int K, int sms) {
     }
     return best;
 }
-// `form` receives 0 (K as one stretch), 1 (a cluster a tile) or 2 (one CTA a tile, four stretches)
-extern "C" int mf_gemm_f32_tile(int M, int N, int K, int sms, int* form) {
+// The tile below 2,048 k.
+extern "C" int mf_gemm_f32_tile(int M, int N, int sms) { return f32_cut(M, N, 1024, sms).tile; }
+// The tile, and in `form` 0 (K as one stretch), 1 (a cluster a tile) or 2 (one CTA a tile, four stretches).
+extern "C" int mf_gemm_f32_cut(int M, int N, int K, int sms, int* form) {
     const F32Cut c = f32_cut(M, N, K, sms);
     *form = c.form;
     return c.tile;

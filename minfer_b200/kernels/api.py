@@ -216,7 +216,8 @@ def _sig_gemm_simt(lib: ctypes.CDLL) -> None:
     lib.mf_gemm_simt.argtypes = [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,
                                  c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int,
                                  c_void_p]
-    lib.mf_gemm_f32_tile.argtypes = [c_int] * 4 + [c_void_p]
+    lib.mf_gemm_f32_tile.argtypes = [c_int] * 3
+    lib.mf_gemm_f32_cut.argtypes = [c_int] * 4 + [c_void_p]
 
 
 def _sig_attention(lib: ctypes.CDLL) -> None:
@@ -621,7 +622,7 @@ def gemm_f32_cut(m: int, n: int, k: int, sms: int) -> tuple[int, int]:
     2: 32 x 64, -1: the general kernel) and how it goes through k (0: one stretch; of 2,048 k and more four,
     1: a cluster of CTAs a tile, 2: one CTA a tile, one after the other)."""
     form = ctypes.c_int(0)
-    tile = int(_lib("gemm_simt").mf_gemm_f32_tile(m, n, k, sms, ctypes.addressof(form)))
+    tile = int(_lib("gemm_simt").mf_gemm_f32_cut(m, n, k, sms, ctypes.addressof(form)))
     return tile, form.value
 
 
