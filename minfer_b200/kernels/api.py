@@ -652,8 +652,9 @@ _PLANS: dict = {}
 
 
 def gemm_tc_plan(m: int, n: int, k: int, epi: int = EPI_STORE) -> tuple[int, int]:
-    """(token tile, K splits) the kernel uses for these sizes (a function of the sizes only:
-    asked once per shape)."""
+    """(token tile, K splits) of the one-CTA tcgen05 kernel for these sizes (a function of the sizes only: asked
+    once per shape).  Products that ``gemm_few_groups`` names, and whole ones of 256 tokens and more
+    (``gemm_pair_plan``), run on other kernels."""
     return _gemm_tc_shape(m, n, k, epi)[:2]
 
 

@@ -61,7 +61,10 @@ def _gemm(m, n, k, epi, reps):
         K.gemm_tc(x, ws[state["i"] % n_w], None, out, epi, st)
         state["i"] += 1
     us = _time(run, reps)
-    print(f"gemm_tc m={m} n={n} k={k} epi={epi} plan={K.gemm_tc_plan(m, n, k, epi)}: {us:.1f} us, "
+    few, cluster = K.gemm_few_plan(m, n, k, torch.cuda.get_device_properties(0).multi_processor_count)
+    kernel = (f"{few} row groups x {cluster} CTAs, mma.sync" if few else f"pairs, tile {K.gemm_pair_plan(m, n, k)}"
+              if m >= 256 else f"plan={K.gemm_tc_plan(m, n, k, epi)}")
+    print(f"gemm_tc m={m} n={n} k={k} epi={epi} {kernel}: {us:.1f} us, "
           f"{2.0 * m * n * k / us / 1e6:.1f} TFLOP/s, {n * k * 2 / us / 1e3:.1f} GB/s of weights")
 
 
@@ -762,6 +765,50 @@ def gemm_m65_to_255(reps):
               f"{2.0 * 16 * rows * 1408 * 2048 / us / 1e6:.1f} TFLOP/s")
 
 
+def gemm_few_tokens(reps):
+    """Products of up to 16 tokens on either side of the lines between gemm_few_kernel and the tcgen05 kernels, each
+    on both: a head (float32 out), gate and up with their activation, a product that completes the residual and
+    prepares the next norm (or leaves that to a kernel).  Weights of 300 MB in turn."""
+    st = torch.zeros(1, dtype=torch.int32, device="cuda")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    pool = (torch.randn(200 << 20, device="cuda") * 0.02).bfloat16()
+    sizes = [(m, n, k) for n, k in ((1152, 896), (896, 4864), (2048, 2048), (2048, 8448), (3584, 3584)) for m in (1, 8, 9, 16)]
+    sizes += [(8, 9728, 896), (9, 9728, 896), (8, 16384, 2048), (8, 16896, 2048), (1, 40, 20000), (8, 144, 8840)]
+    sizes += [(m, n, k) for n, k in ((8192, 64), (8192, 192), (8192, 256), (16000, 192), (16000, 256), (32000, 512), (32000, 1024))
+              for m in (1, 9)]
+    for m, n, k in sizes:
+        nw = max(2, min(64, (300 << 20) // (n * k * 2)))
+        ws = [pool[i * n * k:(i + 1) * n * k].view(n, k) for i in range(nw)]
+        x = torch.randn(m, k, device="cuda").bfloat16()
+        out, act = torch.empty(m, n, device="cuda"), torch.empty(m, n // 2, dtype=torch.bfloat16, device="cuda")
+        h, g, xp = torch.zeros(m, n, device="cuda"), torch.ones(n, device="cuda"), torch.empty_like(out, dtype=torch.bfloat16)
+        turn, us = [0], {}
+
+        def weights():
+            turn[0] += 1
+            return ws[turn[0] % nw]
+
+        def residual():
+            parts = K.gemm_tc_prep_parts(m, n, k)
+            if parts:
+                K.gemm_tc_fused(x, weights(), None, h, K.EPI_ACCUM, st, prep_x=xp, prep_weight=g,
+                                prep_ssq=torch.empty(parts, m, device="cuda"))
+                return
+            part = K.gemm_tc_partial_sums(x, weights(), st)
+            if part is None:
+                K.gemm_tc(x, weights(), None, h, K.EPI_ACCUM, st)
+            K.add_rmsnorm(h, part, 0 if part is None else part.shape[0], None, g, 1e-6, xp)
+        for mode in (0, 2):
+            K.gemm_few_mode(mode)
+            us[mode] = [_time(f, reps) for f in (
+                lambda: K.gemm_tc(x, weights(), None, out, K.EPI_STORE, st),
+                lambda: K.gemm_tc(x, weights(), None, act, K.EPI_SWIGLU, st), residual)]
+        K.gemm_few_mode(1)
+        few = K.gemm_few_plan(m, n, k, sms)
+        print(f"{m} x {n} x {k} ({f'{few[0]} row groups x {few[1]} CTAs' if few[0] else 'tcgen05'}), tcgen05 / mma.sync: "
+              + ", ".join(f"{what} {a:.1f} / {b:.1f}" for what, a, b in zip(("head", "gated", "residual"), us[0], us[2])))
+
+
 CASES = {f.__name__: f for f in (gemm_decode, gemm_decode_split, gemm_decode_m64, gemm_decode_split_m64, gemm_prefill, gemm_prefill_down,
                                  gemm_decode_cluster, gemm_decode_cluster_o, gemm_decode_cluster_m64,
                                  attention_decode, attention_decode_b8, attention_decode_long, attention_prefill,
@@ -773,7 +820,8 @@ CASES = {f.__name__: f for f in (gemm_decode, gemm_decode_split, gemm_decode_m64
                                  zanelorn_step_prefill, zanelorn_step_decode,
                                  pikavik_step_prefill, pikavik_step_decode,
                                  pazatar_step_prefill, pazatar_step_decode,
-                                 float32_products, float32_prompt_attention, scans_of_row_mixes, gemm_m65_to_255)}
+                                 float32_products, float32_prompt_attention, scans_of_row_mixes, gemm_m65_to_255,
+                                 gemm_few_tokens)}
 
 
 def main(argv=None) -> int:

@@ -399,6 +399,15 @@ def test_unsupported_sizes_are_refused_not_miscomputed():
         Attention(hidden_size=40, n_heads=2, n_kv_heads=1, head_dim=20, scale=1.0)
 
 
+@pytest.fixture
+def no_few():
+    """Up to 16 tokens take the tcgen05 kernels too, which larger weights always do."""
+    from minfer_b200.kernels import api as K
+    K.gemm_few_mode(0)
+    yield
+    K.gemm_few_mode(1)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 128, 64), (8, 256, 128), (5, 130, 72), (16, 389, 328),
                                    (33, 640, 200), (64, 512, 1024), (100, 384, 512),
                                    (300, 640, 3584), (8, 3584, 3584), (700, 1000, 264),
@@ -406,10 +415,24 @@ def test_unsupported_sizes_are_refused_not_miscomputed():
                                    (14208, 256, 72), (64, 896, 896), (8, 1152, 896),
                                    (40, 896, 4864)])
 def test_gemm_tensor_core_against_float64(m, n, k):
-    """The tcgen05 kernels at every token tile (16..128 for one CTA; 160, 192, 208, 224 and 256
-    for the CTA pair: the last four sizes each pick another one), with and without K splits,
-    ragged edges in all three dimensions, every epilogue.  The last three are small weights,
-    which are cut along K until a CTA has two k-blocks (7 splits; 16 with a short last one)."""
+    """Products on the tensor cores at every token tile of one CTA (16..128), on the CTA pair and, of few tokens and
+    weights of 512 KB and more, on mma.sync, with and without K splits, ragged edges in all three dimensions, every
+    epilogue.  (64, 896, 896) and (40, 896, 4864) are small weights, which are cut along K until a CTA has two k-blocks
+    (7 splits; 16 with a short last one)."""
+    _product_against_float64(m, n, k)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 3584, 3584), (8, 3584, 3584), (16, 1000, 3592), (8, 1152, 896), (12, 896, 4864),
+                                   (16, 512, 18944), (3, 12000, 2056)])
+def test_gemm_tensor_core_of_up_to_16_tokens_against_float64(m, n, k, no_few):
+    """The 16-token tile of gemm_tc_kernel, its ring of six stages refilled many times (the gated epilogue, which
+    cannot be split, walks all of K), K splits of two k-blocks to 19."""
+    from minfer_b200.kernels import api as K
+    assert K.gemm_few_groups(m, n, k) == 0 and K.gemm_tc_plan(m, n, k)[0] == 16
+    _product_against_float64(m, n, k)
+
+
+def _product_against_float64(m, n, k):
     from minfer_b200.kernels import api as K
     g = torch.Generator().manual_seed(m + n + k)
     x = (torch.randn(m, k, generator=g) * 0.5).bfloat16().cuda()
@@ -890,9 +913,24 @@ def _norm_ref(h, g, eps):
 @pytest.mark.parametrize("n,k", [(3584, 3584), (896, 4864), (200, 1024), (64, 128), (384, 264)])
 def test_product_that_completes_the_residual_and_prepares_the_next_norm(m, n, k):
     """EPI_ACCUM with the next norm folded in (few tokens: K split over a cluster of CTAs that add
-    their tiles through distributed shared memory; many tokens: refused, the norm stays a
-    kernel): the residual, x' = bfloat16(h * g) and the sums of squares against float64; then a
+    their tiles through distributed shared memory, or up to 16 tokens on mma.sync; many tokens: refused, the norm
+    stays a kernel): the residual, x' = bfloat16(h * g) and the sums of squares against float64; then a
     product that reads x' with the row scale against norm-then-product in float64."""
+    _product_that_prepares_the_next_norm(m, n, k)
+
+
+@pytest.mark.parametrize("m", [1, 8, 16])
+@pytest.mark.parametrize("n,k", [(3584, 3584), (896, 4864), (2048, 8448), (1000, 18944)])
+def test_product_of_up_to_16_tokens_that_prepares_the_next_norm_on_tcgen05(m, n, k, no_few):
+    """The 16-token tile of gemm_tc_cluster_kernel, 7 to 37 k-blocks a CTA through a ring of five stages."""
+    from minfer_b200.kernels import api as K
+    assert K.gemm_few_groups(m, n, k) == 0
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert K.gemm_tc_prep_parts(m, n, k) == (n + 127) // 128
+    _product_that_prepares_the_next_norm(m, n, k)
+
+
+def _product_that_prepares_the_next_norm(m, n, k):
     from minfer_b200.kernels import api as K
     g0 = torch.Generator().manual_seed(m + n + k)
     x = (torch.randn(m, k, generator=g0) * 0.5).bfloat16().cuda()
