@@ -788,6 +788,13 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 #define FEW_THREADS (32 * FEW_WARPS)
 #define FEW_MAX_M 16
 #define FEW_BUDGET (200 * 1024)       // shared memory of a CTA (112 KB: fewer products at 8 tokens fit, 0.6 us a layer more)
+// Beyond 8 tokens a next product of 16 MB and more runs on the tcgen05 tiles.  Its CTAs (112 KB) stay off the SMs
+// until this kernel's have gone: two of those that came early shared an SM, and their weights its way to memory.  With
+// that and no more than 4 units a warp in flight a layer of width 2,048, feed-forward 5,632 takes 32.9 us instead of
+// 35.7 for 9 tokens (tcgen05 tiles alone 34.8), 32.7 instead of 34.7 for 12; feed-forward 8,448 37.6 and 37.5 instead of
+// 39.5 and 39.3; width 1,536, feed-forward 8,960, 9 tokens 32.2 instead of 35.7; 0.5B shape 22.5 instead of 22.7.  Up to 8
+// tokens neither made a difference.
+#define FEW_ALONE (118 * 1024)
 #define FEW_MIN_BYTES (512ll << 10)    // of weights: below, a product is a launch whichever kernel runs it
 #define FEW_MAX_BYTES (64ll << 20)     // of weights: beyond, the TMA ring streams as fast as memory gives
 
@@ -1657,13 +1664,14 @@ static FewPlan few_plan(int M, int N, int K, int sms) {
         const int depths[] = {2, 4, 8};
         int depth = 0;
         for (int d : depths) {
-            if (depth > 0 && fixed + (size_t)FEW_WARPS * d * 1024 > FEW_BUDGET) break;
+            if (depth > 0 && (fixed + (size_t)FEW_WARPS * d * 1024 > FEW_BUDGET || (M > 8 && d > 4))) break;
             depth = d;
             if (d >= rt * wu) break;
         }
         if (fixed + (size_t)FEW_WARPS * depth * 1024 > FEW_BUDGET) continue;
         p.row_tiles = rt; p.warp_units = wu; p.tok_stride = stride; p.depth = depth; p.cluster = cluster;
         p.groups = (tiles + rt - 1) / rt; p.smem = fixed + (size_t)FEW_WARPS * depth * 1024;
+        if (M > 8 && p.smem < FEW_ALONE) p.smem = FEW_ALONE;
         // K is cut between CTAs only where one CTA's share of the tokens does not fit, or where the rows
         // alone leave a quarter of the SMs without work and K is long (4 x 40 x 20,000 one CTA a row tile 9.8 us, four 5.0)
         if (p.groups * cluster * 4 >= sms * 3 || wu <= 4) break;
