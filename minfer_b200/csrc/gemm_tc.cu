@@ -4,8 +4,9 @@
 // memory by TMA (128-byte swizzle), an mbarrier ring between the TMA thread, the MMA
 // thread and the epilogue warps.  The reference multiplies with scalar SIMT kernels that
 // re-read the weights for every token (src/cuda_kernels.cu:32-93, grid.y = tokens); here a
-// weight tile is read once per step and the same kernel serves whole prompts (256-token
-// tiles) and decoding (16..64-token tiles that stream the weights at memory speed).
+// weight tile is read once per step: CTA pairs for whole prompts (160..256-token tiles), one CTA for
+// decoding (16..64-token tiles that stream the weights at memory speed).  Up to 16 tokens and weights
+// that fit the chip's shared memory take mma.sync instead (gemm_few_kernel, below).
 //
 // Roles of the operands are swapped against the usual convention: the WEIGHT tile
 // [128 rows of W][64 k] is the MMA's M side, the token tile [NT tokens][64 k] its N side,

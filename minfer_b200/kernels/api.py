@@ -729,7 +729,7 @@ def _gemm_tc_shape(m: int, n: int, k: int, epi: int) -> tuple[int, int, int]:
 
 def gemm_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
             epi: int, status: torch.Tensor) -> None:
-    """out (+)= x @ w^T + bias on tcgen05.  EPI_SWIGLU: w's rows alternate gate, up and out is
+    """out (+)= x @ w^T + bias on the tensor cores.  EPI_SWIGLU: w's rows alternate gate, up and out is
     [M, N/2] bfloat16 = silu(gate) * up."""
     m, k = x.shape
     n = w.shape[0]
@@ -753,7 +753,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out:
 
 def gemm_tc_xielu(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act_p: float, act_n: float,
                   status: torch.Tensor, row_scale: Optional["RowScale"] = None, act_l: float = 0.5) -> None:
-    """out = f(x @ w^T) on tcgen05, f(z) = act_p z^2 + act_l z (z > 0), act_n (exp(z) - 1 - z) + act_l z
+    """out = f(x @ w^T) on the tensor cores, f(z) = act_p z^2 + act_l z (z > 0), act_n (exp(z) - 1 - z) + act_l z
     (z <= 0), applied to the float32 sums in the product's epilogue: the xIELU activation (act_p =
     softplus(a0), act_n = 1/2 + softplus(a1), act_l = 1/2) or the square of relu (1, 0, 0).
     ``row_scale`` as in ``gemm_tc_fused``."""
@@ -780,7 +780,7 @@ GATE_CODES = {"silu": 0, "gelu_tanh": 1, "clamped_swish": 2}
 
 def gemm_tc_gated(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, activation: str, p0: float,
                   p1: float, status: torch.Tensor) -> None:
-    """out [M, N/2] (bfloat16) = act(gate, up) over the interleaved gate, up rows of ``w`` on tcgen05,
+    """out [M, N/2] (bfloat16) = act(gate, up) over the interleaved gate, up rows of ``w`` on the tensor cores,
     the activation applied to the float32 sums in the product's epilogue: "silu", "gelu_tanh", or
     "clamped_swish" with its limit ``p0`` and the factor ``p1`` inside the sigmoid."""
     m, k = x.shape
