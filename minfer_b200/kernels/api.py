@@ -687,11 +687,14 @@ def gemm_pair_group_m(group_m: int) -> None:
 
 
 _FEW: dict = {}
+FEW_MAX_TOKENS = 16
 
 
 def gemm_few_groups(m: int, n: int, k: int) -> int:
     """Column groups that the kernel for a handful of tokens cuts a product of these sizes into, 0 where another
     kernel takes it (a function of the sizes only).  It completes its sums: there are no K splits to add."""
+    if m > FEW_MAX_TOKENS:                    # (prompts: nothing is kept for their many lengths)
+        return 0
     key = (m, n, k)
     got = _FEW.get(key)
     if got is None:

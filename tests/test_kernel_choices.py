@@ -138,6 +138,13 @@ def test_products_for_a_handful_of_tokens(m, n, k, groups, cluster):
     assert K.gemm_few_plan(m, n, k, SMS) == (groups, cluster)
 
 
+def test_nothing_is_kept_for_the_lengths_of_prompts():
+    before = dict(K._FEW)
+    for m in range(17, 300):
+        assert K.gemm_few_groups(m, 1152, 896) == 0 and K.gemm_few_plan(m, 1152, 896, SMS) == (0, 0)
+    assert K._FEW == before
+
+
 @pytest.mark.parametrize("sms", [1, 2, 3, 15, 16, 17, 19, 20, 148, 300])
 def test_the_cut_for_a_handful_of_tokens_on_any_number_of_sms(sms):
     for m, n, k in ((1, 1152, 896), (16, 896, 4864), (3, 40, 20000), (8, 2048, 8448)):
